@@ -27,11 +27,12 @@
 // far smaller), and g = (d + 2) 2^-24 + 1e-5 (the error of the canonical FP32
 // chain against the real distance, and the rounding of the comparison
 // itself).  The scan resolves the sequential rule on bit masks (certain
-// occluders, undecided pairs) and computes the canonical FP32 distance only
-// for undecided pairs between a kept t and a still live p.  A node whose scan
-// reaches the end of the tile with fewer than range kept and more candidates
-// left is finished by the FP32 warp prune (kcna_prune_resume, kcna_graph.cu),
-// which continues from the kept list.
+// occluders, undecided pairs).  A node whose scan meets an undecided pair
+// between a kept t and a still live p hands its two masks to
+// prune_resolve_kernel, which computes the canonical FP32 distances of such
+// pairs.  A node whose scan reaches the end of the tile with fewer than range
+// kept and more candidates left is finished by the FP32 warp prune
+// (prune_resume_kernel, kcna_graph.cu), which continues from the kept list.
 //
 // The screen pays where the rule's margin is wide against the FP8 error: on
 // the 960-dimensional C4 rows with tau = 10, every pair of the first 50
@@ -52,7 +53,8 @@
 //                accumulators;
 //   warps 2-9    mask builders: TMEM lane quarter (warp % 4) x column half;
 //                64 pair decisions per thread into two bit planes;
-//   warp 10      scan: the kept list, undecided pairs resolved in FP32.
+//   warp 10      scan: the kept list of a node without undecided pairs, the
+//                masks of the others to memory for prune_resolve_kernel.
 #include <cuda_fp8.h>
 
 #include <algorithm>
@@ -98,7 +100,7 @@ struct FShared {
 };
 
 struct F8Args {
-    uint32_t n_items;         // nodes (or list entries) to prune
+    uint32_t item0, n_items;  // nodes (or list entries) [item0, n_items) to prune
     const uint32_t *nodes;    // list of nodes (null: item k is node k)
     const uint64_t *keys;     // candidate keys, row r = item (list) or node, `stride` apart
     uint64_t stride;
@@ -117,6 +119,9 @@ struct F8Args {
     uint32_t W;
     uint32_t *resume;         // items left to the FP32 prune
     uint32_t *resume_cnt;
+    uint32_t *masks;          // deferred items: 2 MWD PC words each (certain, undecided)
+    uint32_t *defer;          // their item numbers
+    uint32_t *defer_cnt;
     unsigned long long *comps;
     unsigned long long *exact; // undecided pairs recomputed in FP32
     int *err;
@@ -138,11 +143,6 @@ __device__ __forceinline__ void mma_e4m3(uint32_t tmem_d, uint64_t adesc, uint64
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void cp_wait1() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
 __device__ __forceinline__ void cp_wait0() { asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory"); }
-
-// Canonical FP32 distance of rows a and b (one FMA chain over the dimensions in order).
-__device__ __noinline__ float exact_l2(const float *__restrict__ X, uint32_t ld, uint32_t a, uint32_t b) {
-    return rows_l2(RowsF32{X, (int)ld}, a, b);
-}
 
 __global__ void __launch_bounds__(F8_THREADS, 1) prune_fp8_kernel(F8Args a) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
@@ -208,8 +208,8 @@ __global__ void __launch_bounds__(F8_THREADS, 1) prune_fp8_kernel(F8Args a) {
             }
         };
         uint32_t kk = 0;
-        request(blockIdx.x, 0u);
-        for (uint32_t k = blockIdx.x; k < a.n_items; k += gridDim.x, ++kk) {
+        request(a.item0 + blockIdx.x, 0u);
+        for (uint32_t k = a.item0 + blockIdx.x; k < a.n_items; k += gridDim.x, ++kk) {
             const int sl = (int)(kk & 1u);
             if (!mbar_wait(&S.keys_full[sl], (kk >> 1) & 1u)) { ok = false; break; }
             pending = -1;
@@ -275,7 +275,7 @@ __global__ void __launch_bounds__(F8_THREADS, 1) prune_fp8_kernel(F8Args a) {
         uint32_t gsl = 0;
         int pend = -1;
         uint32_t kk = 0;
-        for (uint32_t k = blockIdx.x; k < a.n_items; k += gridDim.x, ++kk) {
+        for (uint32_t k = a.item0 + blockIdx.x; k < a.n_items; k += gridDim.x, ++kk) {
             const int sl = (int)(kk & 1u);
             if (!mbar_wait(&S.ids_ready[sl], (kk >> 1) & 1u) || S.abort_flag) { ok = false; break; }
             const FMeta &M = S.meta[sl];
@@ -316,7 +316,7 @@ __global__ void __launch_bounds__(F8_THREADS, 1) prune_fp8_kernel(F8Args a) {
         if (lane == 0) {
             const uint32_t idesc = idesc_e4m3(PC, PC);
             uint32_t gsl = 0, kk = 0;
-            for (uint32_t k = blockIdx.x; k < a.n_items && ok; k += gridDim.x, ++kk) {
+            for (uint32_t k = a.item0 + blockIdx.x; k < a.n_items && ok; k += gridDim.x, ++kk) {
                 const int b = (int)(kk % NACC);
                 if (S.abort_flag) { ok = false; break; }
                 if (kk >= (uint32_t)NACC && !mbar_wait(&S.acc_empty[b], ((kk / NACC) - 1) & 1u)) { ok = false; break; }
@@ -351,7 +351,7 @@ __global__ void __launch_bounds__(F8_THREADS, 1) prune_fp8_kernel(F8Args a) {
         const int qt = warp & 3, h = (warp - 2) >> 2; // TMEM lane quarter, column half
         const int t = 32 * qt + lane;
         uint32_t kk = 0;
-        for (uint32_t k = blockIdx.x; k < a.n_items; k += gridDim.x, ++kk) {
+        for (uint32_t k = a.item0 + blockIdx.x; k < a.n_items; k += gridDim.x, ++kk) {
             const int sl = (int)(kk & 1u), b = (int)(kk % NACC);
             bool mine = mbar_wait(&S.meta_full[sl], (kk >> 1) & 1u) && !S.abort_flag;
             mine = mine && mbar_wait(&S.acc_full[b], (kk / NACC) & 1u);
@@ -394,9 +394,9 @@ __global__ void __launch_bounds__(F8_THREADS, 1) prune_fp8_kernel(F8Args a) {
         if (!ok) S.abort_flag = 1;
     } else {
         // ----------------------------------------------------------------- scan
-        unsigned long long cc = 0, ex = 0;
+        unsigned long long cc = 0;
         uint32_t kk = 0;
-        for (uint32_t k = blockIdx.x; k < a.n_items; k += gridDim.x, ++kk) {
+        for (uint32_t k = a.item0 + blockIdx.x; k < a.n_items; k += gridDim.x, ++kk) {
             const int sl = (int)(kk & 1u);
             const bool mine = mbar_wait(&S.mask_full[sl], (kk >> 1) & 1u) && !S.abort_flag;
             if (!__all_sync(KCNA_FULL, mine)) { ok = false; break; }
@@ -407,16 +407,16 @@ __global__ void __launch_bounds__(F8_THREADS, 1) prune_fp8_kernel(F8Args a) {
             uint32_t *gi = a.g_ids + (uint64_t)M.q * a.W;
             float *gd = a.g_dist + (uint64_t)M.q * a.W;
             int nk = 0;
-            bool exhausted = false;
+            bool exhausted = false, undecided = false;
+            unsigned long long cn = 0;
             if (nc > 0) {
                 uint32_t dead = lane < MWD ? M.dead[lane] : 0xFFFFFFFFu;
                 int t = 0;
                 for (;;) {
-                    const uint32_t tid_ = kcna_key_id(keys[t]);
                     if (lane == 0) {
-                        gi[nk] = tid_;
+                        gi[nk] = kcna_key_id(keys[t]);
                         gd[nk] = kcna_key_dist(keys[t]);
-                        cc += (unsigned long long)nk;
+                        cn += (unsigned long long)nk;
                     }
                     ++nk;
                     if (nk >= a.range) break;
@@ -427,23 +427,9 @@ __global__ void __launch_bounds__(F8_THREADS, 1) prune_fp8_kernel(F8Args a) {
                         o = cm[lane * PC + t] & above;
                         u = am[lane * PC + t] & above & ~dead;
                     }
-                    // undecided pairs with a live candidate: the canonical FP32 distance
-#pragma unroll 1
-                    for (int w = tw; w < MWD; ++w) {
-                        const uint32_t bits = __shfl_sync(KCNA_FULL, u, w);
-                        if (!bits) continue;
-                        const bool mine = (bits >> lane) & 1u; // lane l takes candidate 32 w + l
-                        bool hit = false;
-                        if (mine) {
-                            const int p = 32 * w + lane;
-                            const float djk = exact_l2(a.X, a.ld, tid_, kcna_key_id(keys[p]));
-                            hit = djk < M.th[p]; // src/kgraph.cpp:2859 (RNG: :1840)
-                            ++ex;
-                        }
-                        const uint32_t hw = __ballot_sync(KCNA_FULL, hit);
-                        if (lane == w) o |= hw;
-                    }
-                    cc += (unsigned long long)nk * __popc(o & ~dead); // dropped at the nk-th kept
+                    undecided = __any_sync(KCNA_FULL, u != 0u);
+                    if (undecided) break;
+                    cn += (unsigned long long)nk * __popc(o & ~dead); // dropped at the nk-th kept
                     dead |= o;
                     const uint32_t alive = ~dead & above;
                     const unsigned bal = __ballot_sync(KCNA_FULL, lane < MWD && alive != 0u);
@@ -455,32 +441,195 @@ __global__ void __launch_bounds__(F8_THREADS, 1) prune_fp8_kernel(F8Args a) {
                     t = 32 * L + __ffs(__shfl_sync(KCNA_FULL, alive, L)) - 1;
                 }
             }
-            const bool resume = exhausted && nk < a.range && M.ntot > (uint32_t)nc;
-            __syncwarp();
-            if (!resume)
-                for (int j = nk + lane; j < (int)a.W; j += 32) {
-                    gi[j] = KCNA_NONE;
-                    gd[j] = 0.f;
+            if (undecided) { // prune_resolve_kernel writes this node's row
+                uint32_t slot = 0;
+                if (lane == 0) {
+                    slot = atomicAdd(a.defer_cnt, 1u); // at most one per item of this launch
+                    a.defer[slot] = k;
                 }
-            if (lane == 0) {
-                a.g_deg[M.q] = (uint32_t)nk;
-                if (resume) a.resume[atomicAdd(a.resume_cnt, 1u)] = k;
+                slot = __shfl_sync(KCNA_FULL, slot, 0);
+                uint4 *dst = reinterpret_cast<uint4 *>(a.masks + (uint64_t)slot * 2 * MWD * PC);
+                const uint4 *c4 = reinterpret_cast<const uint4 *>(cm), *a4 = reinterpret_cast<const uint4 *>(am);
+                for (int i = lane; i < MWD * PC / 4; i += 32) {
+                    dst[i] = c4[i];
+                    dst[MWD * PC / 4 + i] = a4[i];
+                }
+            } else {
+                cc += cn;
+                const bool resume = exhausted && nk < a.range && M.ntot > (uint32_t)nc;
+                if (!resume)
+                    for (int j = nk + lane; j < (int)a.W; j += 32) {
+                        gi[j] = KCNA_NONE;
+                        gd[j] = 0.f;
+                    }
+                if (lane == 0) {
+                    a.g_deg[M.q] = (uint32_t)nk;
+                    if (resume) a.resume[atomicAdd(a.resume_cnt, 1u)] = k;
+                }
             }
             __syncwarp();
             if (lane == 0) mbar_arrive(&S.node_empty[sl]);
         }
         cc = kcna_warp_sum(cc);
-        ex = kcna_warp_sum(ex);
-        if (lane == 0) {
-            if (cc) atomicAdd(a.comps, cc);
-            if (ex) atomicAdd(a.exact, ex);
-        }
+        if (lane == 0 && cc) atomicAdd(a.comps, cc);
         if (!ok) S.abort_flag = 1;
     }
     fence_before();
     __syncthreads();
     if (warp == 1) tmem_free(tmem, NACC * PC);
     if (!ok) kcna_set_err(a.err, KCNA_DERR_SPIN);
+}
+
+// Scan of the items whose masks hold undecided pairs of live candidates: the
+// same sequential rule, with the canonical FP32 distance of every undecided
+// pair it meets.  Warp per item.  Bound by latency: a chain over 960
+// dimensions is 4 cycles a dimension whatever the other lanes do, and its rows
+// come from L2, so what counts is how many pairs run at once.  They are taken
+// 32 at a time, one per lane: when the scan keeps a t with undecided pairs, the
+// list is filled up with those of the next live candidates as if they were
+// kept too, and the answers go back into the masks (an answer for a candidate
+// that turns out dropped is never read).  40,009 rows of 960 (512 clusters,
+// tau = 10: 288 undecided pairs a node): 213 ms a prune when the tile kernel's
+// scan warp resolved them, one kept neighbour at a time and one warp per SM;
+// 21 ms now, 16 of them here (5.8 TB/s of rows from L2).  Two blocks an SM:
+// three (80 registers) take 17 ms, four (64) 26, with fewer loads in flight.
+constexpr int RW_WARPS = 8;
+struct ResolveShared {
+    uint32_t cm[MWD * PC], am[MWD * PC];
+    uint32_t id[PC];
+    float th[PC], pd[PC];
+    uint16_t pair[32]; // t | p << 8
+};
+
+__global__ void __launch_bounds__(RW_WARPS * 32, 2) prune_resolve_kernel(F8Args a) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    ResolveShared &S = reinterpret_cast<ResolveShared *>(smem_raw)[warp];
+    const uint32_t n = *a.defer_cnt;
+    unsigned long long cc = 0, ex = 0;
+    for (uint32_t i = blockIdx.x * RW_WARPS + warp; i < n; i += gridDim.x * RW_WARPS) {
+        const uint32_t k = a.defer[i];
+        const uint32_t q = a.nodes ? a.nodes[k] : k;
+        const uint64_t *keys = a.keys + (uint64_t)k * a.stride;
+        const int cnt = (int)a.cnt[k];
+        {
+            const uint4 *src = reinterpret_cast<const uint4 *>(a.masks + (uint64_t)i * 2 * MWD * PC);
+            uint4 *c4 = reinterpret_cast<uint4 *>(S.cm), *a4 = reinterpret_cast<uint4 *>(S.am);
+            for (int j = lane; j < MWD * PC / 4; j += 32) {
+                c4[j] = src[j];
+                a4[j] = src[MWD * PC / 4 + j];
+            }
+        }
+        // the candidates, as the tile kernel's metadata warp lays them out
+        const int first = cnt > 0 && kcna_key_id(keys[0]) == q ? 1 : 0;
+        const int ntot = first < cnt ? max(min(cnt, a.maxc), first + 1) - first : 0;
+        const int nc = min(ntot, PC);
+        uint32_t dead = 0xFFFFFFFFu;
+#pragma unroll
+        for (int w = 0; w < MWD; ++w) {
+            const int c = 32 * w + lane;
+            uint32_t id = 0u;
+            float pd = 0.f;
+            bool gone = true;
+            if (c < nc) {
+                const uint64_t key = keys[first + c];
+                id = kcna_key_id(key);
+                pd = kcna_key_dist(key);
+                gone = c > 0 && (id >= a.n_oracle || id == kcna_key_id(keys[first + c - 1]));
+            }
+            S.id[c] = id;
+            S.pd[c] = pd;
+            S.th[c] = __fsub_rn(pd, a.t3); // src/kgraph.cpp:2859 (tau = 0: RNG's d(q,p), :1840)
+            const uint32_t dm = __ballot_sync(KCNA_FULL, gone);
+            if (lane == w) dead = dm;
+        }
+        __syncwarp();
+        uint32_t *gi = a.g_ids + (uint64_t)q * a.W;
+        float *gd = a.g_dist + (uint64_t)q * a.W;
+        auto above_of = [&](int t) { // lane w: candidates of word w after t
+            const int tw = t >> 5;
+            return lane > tw ? 0xFFFFFFFFu : lane < tw ? 0u : ~((2u << (t & 31)) - 1u);
+        };
+        int nk = 0, t = 0;
+        bool exhausted = false;
+        for (;;) {
+            if (lane == 0) {
+                gi[nk] = S.id[t];
+                gd[nk] = S.pd[t];
+                cc += (unsigned long long)nk;
+            }
+            ++nk;
+            if (nk >= a.range) break;
+            const uint32_t above = above_of(t);
+            // undecided pairs of t (and, to fill the lanes, of the candidates after it)
+            while (__any_sync(KCNA_FULL, lane < MWD && (S.am[(lane & (MWD - 1)) * PC + t] & above & ~dead) != 0u)) {
+                int np = 0, tt = t;
+                uint32_t sdead = dead;
+                for (;;) {
+                    const uint32_t ab = above_of(tt);
+                    uint32_t u = lane < MWD ? S.am[lane * PC + tt] & ab & ~sdead : 0u;
+                    const int c = __popc(u);
+                    int at = c; // inclusive sum over the MWD words
+#pragma unroll
+                    for (int o = 1; o < MWD; o <<= 1) {
+                        const int x = __shfl_up_sync(KCNA_FULL, at, o);
+                        if (lane >= o) at += x;
+                    }
+                    const int tot = __shfl_sync(KCNA_FULL, at, MWD - 1);
+                    at += np - c;
+                    while (u && at < 32) {
+                        S.pair[at++] = (uint16_t)(tt | ((32 * lane + __ffs(u) - 1) << 8));
+                        u &= u - 1u;
+                    }
+                    np += tot;
+                    if (np >= 32) break;
+                    if (lane < MWD) sdead |= S.cm[lane * PC + tt] & ab;
+                    const uint32_t alive = lane < MWD ? ~sdead & ab : 0u;
+                    const unsigned bal = __ballot_sync(KCNA_FULL, alive != 0u);
+                    if (!bal) break;
+                    const int L = __ffs(bal) - 1;
+                    tt = 32 * L + __ffs(__shfl_sync(KCNA_FULL, alive, L)) - 1;
+                }
+                __syncwarp();
+                if (lane < np) {
+                    const int t_ = S.pair[lane] & 0xFF, p_ = S.pair[lane] >> 8;
+                    const bool hit = rows_l2(RowsF32{a.X, (int)a.ld}, S.id[t_], S.id[p_]) < S.th[p_];
+                    ++ex;
+                    atomicAnd(&S.am[(p_ >> 5) * PC + t_], ~(1u << (p_ & 31)));
+                    if (hit) atomicOr(&S.cm[(p_ >> 5) * PC + t_], 1u << (p_ & 31));
+                }
+                __syncwarp();
+            }
+            const uint32_t o = lane < MWD ? S.cm[lane * PC + t] & above : 0u;
+            cc += (unsigned long long)nk * __popc(o & ~dead); // dropped at the nk-th kept
+            dead |= o;
+            const uint32_t alive = ~dead & above;
+            const unsigned bal = __ballot_sync(KCNA_FULL, lane < MWD && alive != 0u);
+            if (!bal) {
+                exhausted = true;
+                break;
+            }
+            const int L = __ffs(bal) - 1;
+            t = 32 * L + __ffs(__shfl_sync(KCNA_FULL, alive, L)) - 1;
+        }
+        const bool resume = exhausted && nk < a.range && ntot > nc;
+        if (!resume)
+            for (int j = nk + lane; j < (int)a.W; j += 32) {
+                gi[j] = KCNA_NONE;
+                gd[j] = 0.f;
+            }
+        if (lane == 0) {
+            a.g_deg[q] = (uint32_t)nk;
+            if (resume) a.resume[atomicAdd(a.resume_cnt, 1u)] = k;
+        }
+        __syncwarp();
+    }
+    cc = kcna_warp_sum(cc);
+    ex = kcna_warp_sum(ex);
+    if (lane == 0) {
+        if (cc) atomicAdd(a.comps, cc);
+        if (ex) atomicAdd(a.exact, ex);
+    }
 }
 
 size_t prune_fp8_smem() { return 1024 + (size_t)NS * SLAB + sizeof(FShared); }
@@ -545,7 +694,6 @@ kcna_status kcna_prune_fp8_launch(kcna_ctx *c, const uint64_t *keys, uint64_t st
                                   unsigned long long *exact) {
     if (n_items == 0) return KCNA_OK;
     F8Args a;
-    a.n_items = n_items;
     a.nodes = nodes;
     a.keys = keys;
     a.stride = stride;
@@ -573,8 +721,41 @@ kcna_status kcna_prune_fp8_launch(kcna_ctx *c, const uint64_t *keys, uint64_t st
     KCNA_TRY(kcna_cuda_check(c, cudaFuncSetAttribute(prune_fp8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                      (int)sm),
                              "prune_fp8 smem attr"));
-    const uint32_t grid = (uint32_t)std::min<uint64_t>(n_items, (uint64_t)std::max(c->num_sms, 1));
-    prune_fp8_kernel<<<grid, F8_THREADS, sm, c->stream>>>(a);
-    KCNA_LAUNCHED(c);
-    return kcna_cuda_check(c, cudaGetLastError(), "prune_fp8_kernel");
+    const size_t rsm = RW_WARPS * sizeof(ResolveShared);
+    KCNA_TRY(kcna_cuda_check(c, cudaFuncSetAttribute(prune_resolve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                     (int)std::max<size_t>(rsm, 48 * 1024)),
+                             "prune_resolve smem attr"));
+    int per_sm = 0;
+    KCNA_TRY(kcna_cuda_check(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, prune_resolve_kernel,
+                                                                              RW_WARPS * 32, rsm),
+                             "prune_resolve occupancy"));
+    // items in runs of at most DEFER_RUN, so that the deferred items' masks
+    // (4 KiB each, any item can be one) stay within 128 MiB; a device too full
+    // for that takes shorter runs
+    constexpr uint32_t DEFER_RUN = 32768, DEFER_MIN = 1024, MASK_U32 = 2 * MWD * PC;
+    uint32_t run = std::min(n_items, DEFER_RUN);
+    uint32_t *buf = nullptr;
+    kcna_status s;
+    while ((s = kcna_alloc(c, &buf, (size_t)run * (MASK_U32 + 1) + 1, "undecided masks")) == KCNA_E_OOM && run > DEFER_MIN)
+        run = std::max(run / 2, DEFER_MIN);
+    if (s != KCNA_OK) return s;
+    c->err.clear();
+    a.masks = buf;
+    a.defer = buf + (size_t)run * MASK_U32;
+    a.defer_cnt = a.defer + run;
+    const uint32_t sms = (uint32_t)std::max(c->num_sms, 1);
+    for (uint32_t i0 = 0; i0 < n_items && s == KCNA_OK; i0 += run) {
+        a.item0 = i0;
+        a.n_items = std::min(n_items, i0 + run);
+        const uint32_t grid = std::min(a.n_items - i0, sms);
+        s = kcna_cuda_check(c, cudaMemsetAsync(a.defer_cnt, 0, 4, c->stream), "memset");
+        if (s != KCNA_OK) break;
+        prune_fp8_kernel<<<grid, F8_THREADS, sm, c->stream>>>(a);
+        KCNA_LAUNCHED(c);
+        prune_resolve_kernel<<<sms * (uint32_t)std::max(per_sm, 1), RW_WARPS * 32, rsm, c->stream>>>(a);
+        KCNA_LAUNCHED(c);
+        s = kcna_cuda_check(c, cudaGetLastError(), "prune_fp8_kernel");
+    }
+    kcna_release(c, buf); // back to the context's cache: later users run behind these kernels on its stream
+    return s;
 }
