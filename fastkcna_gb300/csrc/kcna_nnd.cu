@@ -6,13 +6,13 @@
 // statistics / stop rule (:1365-1426).
 //
 // GPU form of one iteration:
-//   join    one block per node n: gather the node's new list A and old list B,
-//           compute every pair of A x A (i < j) and A x B with the canonical
-//           FMA-chain distance in register tiles (rows staged through shared
-//           memory in 32-float chunks), and emit each pair to both endpoints'
-//           candidate buffers when it is within that endpoint's radius.
-//           Candidates of one target from one block are written as one
-//           contiguous run after a single atomicAdd.
+//   join    one warp per node n (one block for the few nodes with more than 64
+//           rows): gather the node's new list A and old list B, compute every
+//           pair of A x A (i < j) and A x B with the canonical FMA-chain
+//           distance in register tiles (rows staged through shared memory),
+//           and emit each pair to both endpoints' candidate buffers when it is
+//           within that endpoint's radius.  Candidates of one target from one
+//           node are written as one contiguous run after a single atomicAdd.
 //   merge   one block per node: sort the candidate buffer, drop duplicates,
 //           merge with the sorted pool by rank, keep the best `limit`; new
 //           entries carry flag=new (the reference's InsertIntoPool
@@ -31,6 +31,7 @@
 
 #include "kcna_internal.h"
 #include "kcna_join.cuh"
+#include "kcna_pairs.cuh"
 #include "kcna_sort.cuh"
 
 namespace {
@@ -252,8 +253,11 @@ __device__ void join_tiles(const JoinArgs &a, const R &rows, uint32_t node, cons
     }
 }
 
+// Join of the nodes queued by join_warp_kernel (more rows than a warp's region
+// holds): block per node, persistent over the queue.
 template <class R>
-__global__ void __launch_bounds__(JT, 3) join_kernel(JoinArgs a, R rows) {
+__global__ void __launch_bounds__(JT, 3) join_kernel(JoinArgs a, R rows, const uint32_t *__restrict__ big_list,
+                                                     const uint32_t *__restrict__ big_cnt) {
     extern __shared__ __align__(16) unsigned char smem[];
     float *s_As = reinterpret_cast<float *>(smem);                // 128 x JKP
     float *s_Bs = s_As + 128 * JKP;                               // JCOLS x JKP
@@ -262,36 +266,196 @@ __global__ void __launch_bounds__(JT, 3) join_kernel(JoinArgs a, R rows) {
     uint32_t *s_A = reinterpret_cast<uint32_t *>(s_radA + a.capA); // capA
     uint32_t *s_B = s_A + a.capA;                                 // capB
     __shared__ unsigned s_emit;
-    const uint32_t node = blockIdx.x;
-    // new list: forward new then a random subset (<= R) of reverse new
-    uint32_t fn = min(a.fwd_new_cnt[node], a.fwd_new_cap);
-    for (uint32_t i = threadIdx.x; i < fn; i += blockDim.x) s_A[i] = a.fwd_new[(uint64_t)node * a.fwd_new_cap + i];
-    uint32_t fo = min(a.fwd_old_cnt[node], a.fwd_old_cap);
-    for (uint32_t i = threadIdx.x; i < fo; i += blockDim.x) s_B[i] = a.fwd_old[(uint64_t)node * a.fwd_old_cap + i];
-    __syncthreads();
-    uint32_t rn = 0, ro = 0;
-    if (a.iter > 0) {
-        rn = take_reverse(a.rnew + (uint64_t)node * a.RB, a.rnew_cnt[node], a.R, s_A + fn);
-        ro = take_reverse(a.rold + (uint64_t)node * a.RB, a.rold_cnt[node], a.R, s_B + fo);
+    const uint32_t n_big = *big_cnt;
+    for (uint32_t bi = blockIdx.x; bi < n_big; bi += gridDim.x) {
+        const uint32_t node = big_list[bi];
+        __syncthreads(); // the previous node's lists and tiles are read
+        // new list: forward new then a random subset (<= R) of reverse new
+        uint32_t fn = min(a.fwd_new_cnt[node], a.fwd_new_cap);
+        for (uint32_t i = threadIdx.x; i < fn; i += blockDim.x) s_A[i] = a.fwd_new[(uint64_t)node * a.fwd_new_cap + i];
+        uint32_t fo = min(a.fwd_old_cnt[node], a.fwd_old_cap);
+        for (uint32_t i = threadIdx.x; i < fo; i += blockDim.x) s_B[i] = a.fwd_old[(uint64_t)node * a.fwd_old_cap + i];
         __syncthreads();
+        uint32_t rn = 0, ro = 0;
+        if (a.iter > 0) {
+            rn = take_reverse(a.rnew + (uint64_t)node * a.RB, a.rnew_cnt[node], a.R, s_A + fn);
+            ro = take_reverse(a.rold + (uint64_t)node * a.RB, a.rold_cnt[node], a.R, s_B + fo);
+            __syncthreads();
+        }
+        // at most 128 rows per tile; the forward list alone is <= S + R < 128 in practice
+        const int na = (int)min(fn + rn, 128u), nb = (int)(fo + ro);
+        for (int i = threadIdx.x; i < na; i += blockDim.x) s_radA[i] = __ldg(a.radius + s_A[i]);
+        if (threadIdx.x == 0) {
+            atomicAdd(a.counters + 0, (unsigned long long)((uint64_t)na * (na - 1) / 2 + (uint64_t)na * nb));
+            atomicAdd(a.counters + 5, (unsigned long long)(na + nb));
+            s_emit = 0;
+        }
+        __syncthreads();
+        if (na <= 32)
+            join_tiles<1>(a, rows, node, s_A, na, s_B, nb, s_As, s_Bs, s_D, s_radA, &s_emit);
+        else if (na <= 64)
+            join_tiles<2>(a, rows, node, s_A, na, s_B, nb, s_As, s_Bs, s_D, s_radA, &s_emit);
+        else
+            join_tiles<4>(a, rows, node, s_A, na, s_B, nb, s_As, s_Bs, s_D, s_radA, &s_emit);
+        if (threadIdx.x == 0 && s_emit) atomicAdd(a.counters + 6, (unsigned long long)s_emit);
     }
-    // at most 128 rows per tile; the forward list alone is <= S + R < 128 in practice
-    const int na = (int)min(fn + rn, 128u), nb = (int)(fo + ro);
-    for (int i = threadIdx.x; i < na; i += blockDim.x) s_radA[i] = __ldg(a.radius + s_A[i]);
-    __syncthreads();
-    if (na == 0) return;
-    if (threadIdx.x == 0) {
-        atomicAdd(a.counters + 0, (unsigned long long)((uint64_t)na * (na - 1) / 2 + (uint64_t)na * nb));
-        atomicAdd(a.counters + 5, (unsigned long long)(na + nb));
-        s_emit = 0;
+}
+
+// Warp per node, persistent: the same join for nodes of at most JW_ROWS rows
+// and PT_MAXT micro-tiles (kcna_pairs.cuh); larger nodes are queued for
+// join_kernel.  The micro-tiles are those of the upper triangle of A x A and of
+// A x B.  The distances go to a matrix over the rows' region (both triangles
+// of A x A), and the warp then takes the targets one by one: a count pass (two
+// ballots a target, kept by lane target % 32), one atomicAdd per target with
+// all of them in flight together, a write pass.
+// 18.7 KB a warp: twelve warps an SM, three per scheduler, which hides the
+// gathers behind the other warps' arithmetic.  Below the line of 64 rows lie
+// 99 % of the nodes of every workload here; a region of 96 rows would hold
+// eight warps.
+constexpr int JW_WARPS = 4, JW_ROWS = 64;
+struct JoinWarp {
+    float x[(JW_ROWS + PT_SPARE) * PT_P]; // rows, then the distance matrix: row i at i * (n | 1)
+    uint32_t id[JW_ROWS];
+    float rad[JW_ROWS];
+};
+static_assert(JW_ROWS * (JW_ROWS + 1) <= (JW_ROWS + PT_SPARE) * PT_P, "the distance matrix fits the rows' region");
+
+template <int R, class RowsT>
+__device__ __forceinline__ void join_warp_tiles(const RowsT &rows, JoinWarp &S, int na, int n, int T) {
+    const int lane = kcna_lane(), nb = n - na, GA = (na + 3) >> 2, GB = (nb + 3) >> 2;
+    const int TA = GA * (GA + 1) / 2;
+    PairTile t[R];
+    bool on[R];
+    float acc[R][16];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        int k = lane + 32 * r;
+        on[r] = k < T;
+        t[r] = PairTile{0, 0, 0, 0};
+        if (on[r]) {
+            if (k < TA) {
+                int g = 0;
+                while (k >= GA - g) k -= GA - g++;
+                t[r] = PairTile{g, GA, g + k, GA};
+            } else {
+                k -= TA;
+                t[r] = PairTile{k / GB, GA, na + k % GB, GB};
+            }
+        }
     }
-    if (na <= 32)
-        join_tiles<1>(a, rows, node, s_A, na, s_B, nb, s_As, s_Bs, s_D, s_radA, &s_emit);
-    else if (na <= 64)
-        join_tiles<2>(a, rows, node, s_A, na, s_B, nb, s_As, s_Bs, s_D, s_radA, &s_emit);
-    else
-        join_tiles<4>(a, rows, node, s_A, na, s_B, nb, s_As, s_Bs, s_D, s_radA, &s_emit);
-    if (threadIdx.x == 0 && s_emit) atomicAdd(a.counters + 6, (unsigned long long)s_emit);
+    pairs_distances<R>(rows, S.id, n, S.x, t, on, acc);
+    const int dp = n | 1;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        if (!on[r]) continue;
+        const bool inA = t[r].b0 < na;
+#pragma unroll
+        for (int x = 0; x < 4; ++x)
+#pragma unroll
+            for (int y = 0; y < 4; ++y) {
+                const int i = t[r].a0 + x * t[r].as, j = t[r].b0 + y * t[r].bs;
+                if (i >= na || j >= (inA ? na : n)) continue;
+                S.x[i * dp + j] = acc[r][4 * x + y];
+                if (inA) S.x[j * dp + i] = acc[r][4 * x + y];
+            }
+    }
+    __syncwarp();
+}
+
+template <class RowsT>
+__global__ void __launch_bounds__(JW_WARPS * 32, 3) join_warp_kernel(JoinArgs a, RowsT rows, uint32_t *big_list,
+                                                                    uint32_t *big_cnt) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int lane = kcna_lane();
+    JoinWarp &S = reinterpret_cast<JoinWarp *>(smem)[threadIdx.x >> 5];
+    unsigned long long pairs = 0, nrows = 0, emitted = 0;
+    for (uint32_t node = blockIdx.x * JW_WARPS + (threadIdx.x >> 5); node < a.N; node += gridDim.x * JW_WARPS) {
+        // new list A: forward new then a random subset (<= R) of reverse new; old list B likewise
+        const uint32_t fn = min(a.fwd_new_cnt[node], a.fwd_new_cap), fo = min(a.fwd_old_cnt[node], a.fwd_old_cap);
+        uint32_t rn = 0, ro = 0;
+        if (a.iter > 0) {
+            rn = min(a.rnew_cnt[node], a.R);
+            ro = min(a.rold_cnt[node], a.R);
+        }
+        if (fn + rn == 0) continue;
+        const uint32_t all = fn + rn + fo + ro;
+        const int na = (int)(fn + rn), n = (int)all, nb = n - na;
+        const int GA = (na + 3) >> 2, T = GA * (GA + 1) / 2 + GA * ((nb + 3) >> 2);
+        if (all > (uint32_t)JW_ROWS || T > PT_MAXT) {
+            if (lane == 0) big_list[atomicAdd(big_cnt, 1u)] = node;
+            continue;
+        }
+        for (int i = lane; i < n; i += 32) {
+            const uint32_t u = (uint32_t)i, v = u - (uint32_t)na;
+            const uint32_t id = u < fn            ? a.fwd_new[(uint64_t)node * a.fwd_new_cap + u]
+                                : u < (uint32_t)na ? a.rnew[(uint64_t)node * a.RB + (u - fn)]
+                                : v < fo           ? a.fwd_old[(uint64_t)node * a.fwd_old_cap + v]
+                                                   : a.rold[(uint64_t)node * a.RB + (v - fo)];
+            S.id[i] = id;
+            S.rad[i] = __ldg(a.radius + id);
+        }
+        __syncwarp();
+        if (T <= 32)
+            join_warp_tiles<1>(rows, S, na, n, T);
+        else if (T <= 64)
+            join_warp_tiles<2>(rows, S, na, n, T);
+        else
+            join_warp_tiles<PT_MAXR>(rows, S, na, n, T);
+        pairs += (unsigned long long)((uint64_t)na * (na - 1) / 2 + (uint64_t)na * nb);
+        nrows += (unsigned long long)n;
+        const int dp = n | 1;
+        // whether partner p (a row of the set) enters target t's buffer, and at which distance
+        auto emits = [&](int t, int p, float &dd) {
+            if (t < na ? p >= n || p == t : p >= na) return false;
+            dd = t < na ? S.x[t * dp + p] : S.x[p * dp + t];
+            return S.id[p] != S.id[t] && dd <= S.rad[t];
+        };
+        uint32_t m0[2] = {0u, 0u}, m1[2] = {0u, 0u}, base[2] = {0u, 0u}; // of targets lane and lane + 32
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            for (int t = 32 * h; t < min(n, 32 * h + 32); ++t) {
+                float dd;
+                const uint32_t b0 = __ballot_sync(KCNA_FULL, emits(t, lane, dd));
+                const uint32_t b1 = n > 32 ? __ballot_sync(KCNA_FULL, emits(t, lane + 32, dd)) : 0u;
+                if (lane == (t & 31)) {
+                    m0[h] = b0;
+                    m1[h] = b1;
+                }
+            }
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const uint32_t cnt = __popc(m0[h]) + __popc(m1[h]);
+            if (cnt) base[h] = atomicAdd(a.cand_cnt + S.id[32 * h + lane], cnt);
+            emitted += cnt;
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            for (int t = 32 * h; t < min(n, 32 * h + 32); ++t) {
+                const uint32_t b0 = __shfl_sync(KCNA_FULL, m0[h], t & 31), b1 = __shfl_sync(KCNA_FULL, m1[h], t & 31);
+                const uint32_t at = __shfl_sync(KCNA_FULL, base[h], t & 31);
+                const uint64_t s0 = (uint64_t)S.id[t] * a.CB;
+#pragma unroll
+                for (int v = 0; v < 2; ++v) {
+                    const uint32_t b = v ? b1 : b0;
+                    if (!((b >> lane) & 1u)) continue;
+                    const int p = lane + 32 * v;
+                    const uint32_t pos = at + (v ? __popc(b0) : 0) + __popc(b & kcna_lanemask_lt());
+                    const float dd = t < na ? S.x[t * dp + p] : S.x[p * dp + t];
+                    if (pos < a.CB)
+                        kcna_cand_put(a.cand, s0 + pos, kcna_key(dd, S.id[p], (uint32_t)(KCNA_FLAG_NEW | KCNA_FLAG_ISNEW)),
+                                      node);
+                }
+            }
+        }
+        __syncwarp(); // the next node reuses the region
+    }
+    emitted = kcna_warp_sum(emitted);
+    if (lane == 0) {
+        atomicAdd(a.counters + 0, pairs);
+        atomicAdd(a.counters + 5, nrows);
+        atomicAdd(a.counters + 6, emitted);
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -1115,6 +1279,7 @@ kcna_status kcna_nnd_join(kcna_ctx *c, const kcna_params *p, int iter, uint64_t 
     // found (src/kgraph.cpp:1104,1116): cleared for every node, then set by the
     // merge for the joiners whose candidates it inserts below K
     KCNA_TRY(kcna_cuda_check(c, cudaMemsetAsync(c->found, 0, c->n, c->stream), "memset"));
+    KCNA_TRY(kcna_cuda_check(c, cudaMemsetAsync(c->big_cnt, 0, 4, c->stream), "memset"));
     KCNA_TRY(kcna_phase_begin(c));
     if ((c->gram_exact || c->bf16_screen) && kcna_join_tc_fits(a)) {
         KCNA_TRY(kcna_join_tc_launch(c, a));
@@ -1137,12 +1302,29 @@ kcna_status kcna_nnd_join(kcna_ctx *c, const kcna_params *p, int iter, uint64_t 
             KCNA_TRY(kcna_cuda_check(c, cudaGetLastError(), "rescore_kernel"));
         }
     } else {
+        // warp per node; the nodes it queues (merge's queue, idle here) go to the block kernel
+        auto launch = [&](auto rows) -> kcna_status {
+            auto warp_kern = join_warp_kernel<decltype(rows)>;
+            const size_t wsm = JW_WARPS * sizeof(JoinWarp);
+            int per_sm = 0;
+            KCNA_TRY(kcna_cuda_check(c, cudaFuncSetAttribute(warp_kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                             (int)wsm),
+                                     "join smem attr"));
+            KCNA_TRY(kcna_cuda_check(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, warp_kern, JW_WARPS * 32,
+                                                                                     wsm),
+                                     "join occupancy"));
+            const uint32_t sms = (uint32_t)std::max(c->num_sms, 1);
+            const uint32_t grid = std::min(kcna_div_up(c->n, JW_WARPS), sms * (uint32_t)std::max(per_sm, 1));
+            warp_kern<<<grid, JW_WARPS * 32, wsm, c->stream>>>(a, rows, c->big_list, c->big_cnt);
+            KCNA_LAUNCHED(c);
+            join_kernel<<<std::min(c->n, sms * 3), JT, sm, c->stream>>>(a, rows, c->big_list, c->big_cnt);
+            KCNA_LAUNCHED(c);
+            return kcna_cuda_check(c, cudaGetLastError(), "join_kernel");
+        };
         if (c->bf16_exact)
-            join_kernel<<<c->n, JT, sm, c->stream>>>(a, RowsB16{c->Xh, (int)c->ld});
+            KCNA_TRY(launch(RowsB16{c->Xh, (int)c->ld}));
         else
-            join_kernel<<<c->n, JT, sm, c->stream>>>(a, RowsF32{c->X, (int)c->ld});
-        KCNA_LAUNCHED(c);
-        KCNA_TRY(kcna_cuda_check(c, cudaGetLastError(), "join_kernel"));
+            KCNA_TRY(launch(RowsF32{c->X, (int)c->ld}));
     }
     KCNA_TRY(kcna_phase_end(c, KCNA_PHASE_JOIN));
     unsigned long long h[8] = {};
