@@ -18,6 +18,7 @@
 #include <set>
 
 #include "kcna_internal.h"
+#include "kcna_pairs.cuh"
 #include "kcna_sort.cuh"
 
 namespace {
@@ -983,172 +984,182 @@ __global__ void count_new_edges_kernel(const uint8_t *__restrict__ g_isnew, cons
     if (lane == 0) nnew[q] = (uint16_t)n;
 }
 
-// P2K join, tiled: one block per node q.  Rows = pushers u of q (rnn(q), up to
-// 128 per tile), columns = q's graph neighbours w (up to 64), staged through
-// shared memory in 32-float chunks; each thread keeps RI x 8 canonical FMA
-// accumulators.  Pair (u, w) is skipped when u == w or both are old
-// (src/kgraph.cpp:2639-2641); survivors within u's radius become candidates of
-// u, written as one run per (q, u) after one atomicAdd.
-constexpr int PJT = 256, PJC = 64, PJK = 32, PJP = PJK + 4;
+// P2K join, warp per node q, persistent.  Rows = q's graph neighbours w (up to
+// 64 at a time, those flagged new first) and pushers u of q (rnn(q), those
+// flagged new first, as many as the region holds); the pairs as 4 x 4
+// micro-tiles (kcna_pairs.cuh).  Pair (u, w) is skipped when u == w or both are
+// old (src/kgraph.cpp:2639-2641), so new pushers meet all neighbours, old
+// pushers only the new ones, and rows without a partner are not read.
+// Survivors within u's radius become candidates of u, one run per (q, u) after
+// one atomicAdd.  A node has about 10 pushers and 26 neighbours (C2): the block
+// per node that this replaces computed a 32 x 64 tile for those 260 pairs, and
+// its rounds on 150,001 x 128 rows took 2.6 ms each (P2K_MS here).
+// 23 KB a warp: nine warps an SM.
+constexpr int PJ_WARPS = 3, PJ_ROWS = 80, PJ_COLS = 64, PJ_U = 32;
+struct P2kWarp {
+    float x[(PJ_ROWS + PT_SPARE) * PT_P]; // rows, then the distance matrix: pusher i at i * (PJ_COLS + 1)
+    uint32_t id[PJ_ROWS];                 // neighbours, then pushers
+    float rad[PJ_U];
+};
+static_assert(PJ_U * (PJ_COLS + 1) <= (PJ_ROWS + PT_SPARE) * PT_P, "the distance matrix fits the rows' region");
+static_assert((PJ_U / 4) * (PJ_COLS / 4) <= PT_MAXT, "a tile's micro-tiles fit the lanes");
 
-template <int RI, class R>
-__device__ void p2k_tile(const R &rows, int ld, uint32_t N, const uint32_t *s_u, const uint8_t *s_unew,
-                         int nu, const uint32_t *s_w, const uint8_t *s_wnew, int nw, const float *__restrict__ radius,
-                         uint64_t *__restrict__ cand, uint32_t *__restrict__ cand_cnt, uint32_t CB, float *s_As,
-                         float *s_Bs, float *s_D, unsigned long long *s_cc) {
-    const int tid = threadIdx.x, tx = tid & 7, ty = tid >> 3;
-    float acc[RI][8];
+// rows [0, nw): neighbours, the first nwN new; [nw, nw + nu): pushers, the first nuN new
+template <int R, class RowsT>
+__device__ __forceinline__ void p2k_warp_tiles(const RowsT &rows, P2kWarp &S, int nw, int nwN, int nu, int nuN, int T) {
+    const int lane = kcna_lane(), nuO = nu - nuN;
+    const int GN = (nuN + 3) >> 2, GO = (nuO + 3) >> 2, GW = (nw + 3) >> 2, GWN = (nwN + 3) >> 2;
+    PairTile t[R];
+    bool on[R];
+    float acc[R][16];
 #pragma unroll
-    for (int i = 0; i < RI; ++i)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
-    for (int k0 = 0; k0 < ld; k0 += PJK) {
-        for (int idx = tid; idx < 32 * RI * (PJK / 4); idx += PJT) {
-            int r = idx >> 3, c = (idx & 7) * 4;
-            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (r < nu && k0 + c < ld) v = rows.ld4(s_u[r], (k0 + c) >> 2);
-            *reinterpret_cast<float4 *>(s_As + r * PJP + c) = v;
-        }
-        for (int idx = tid; idx < PJC * (PJK / 4); idx += PJT) {
-            int r = idx >> 3, c = (idx & 7) * 4;
-            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (r < nw && k0 + c < ld) v = rows.ld4(s_w[r], (k0 + c) >> 2);
-            *reinterpret_cast<float4 *>(s_Bs + r * PJP + c) = v;
-        }
-        __syncthreads();
-        const int kend = min(PJK, ld - k0);
-        for (int k = 0; k < kend; k += 4) {
-            float4 ra[RI], cb[8];
-#pragma unroll
-            for (int i = 0; i < RI; ++i) ra[i] = *reinterpret_cast<const float4 *>(s_As + (ty + 32 * i) * PJP + k);
-#pragma unroll
-            for (int j = 0; j < 8; ++j) cb[j] = *reinterpret_cast<const float4 *>(s_Bs + (tx + 8 * j) * PJP + k);
-#pragma unroll
-            for (int i = 0; i < RI; ++i)
-#pragma unroll
-                for (int j = 0; j < 8; ++j) acc[i][j] = kcna_acc4(acc[i][j], ra[i], cb[j]);
-        }
-        __syncthreads();
-    }
-#pragma unroll
-    for (int i = 0; i < RI; ++i)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) s_D[(ty + 32 * i) * (PJC + 1) + tx + 8 * j] = acc[i][j];
-    __syncthreads();
-    const int warp = tid >> 5, lane = tid & 31;
-    unsigned long long cc = 0;
-    for (int i = warp; i < nu; i += PJT / 32) {
-        const uint32_t u = s_u[i];
-        const bool unew = s_unew[i] != 0;
-        const float rad = __ldg(radius + u);
-        bool ok[2];
-        uint64_t keys[2];
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int j = lane + 32 * h;
-            ok[h] = false;
-            if (j < nw && s_w[j] != u && (unew || s_wnew[j])) {
-                ++cc;
-                float dd = s_D[i * (PJC + 1) + j];
-                if (dd <= rad) {
-                    ok[h] = true;
-                    keys[h] = kcna_key(dd, s_w[j], (uint32_t)(KCNA_FLAG_NEW | KCNA_FLAG_ISNEW));
-                }
+    for (int r = 0; r < R; ++r) {
+        int k = lane + 32 * r;
+        on[r] = k < T;
+        t[r] = PairTile{0, 0, 0, 0};
+        if (on[r]) {
+            if (k < GN * GW) {
+                t[r] = PairTile{nw + k / GW, GN, k % GW, GW};
+            } else {
+                k -= GN * GW;
+                t[r] = PairTile{nw + nuN + k / GWN, GO, k % GWN, GWN};
             }
         }
-        unsigned m0 = __ballot_sync(KCNA_FULL, ok[0]), m1 = __ballot_sync(KCNA_FULL, ok[1]);
-        int cnt = __popc(m0) + __popc(m1);
-        if (!cnt) continue;
-        uint32_t base = 0;
-        if (lane == 0) base = atomicAdd(cand_cnt + u, (uint32_t)cnt);
-        base = __shfl_sync(KCNA_FULL, base, 0);
-        const uint64_t s0 = (uint64_t)u * CB; // whole slots, joiner 0 (no credit)
-        if (ok[0]) {
-            uint32_t p = base + __popc(m0 & kcna_lanemask_lt());
-            if (p < CB) kcna_cand_put(cand, s0 + p, keys[0], 0u);
-        }
-        if (ok[1]) {
-            uint32_t p = base + __popc(m0) + __popc(m1 & kcna_lanemask_lt());
-            if (p < CB) kcna_cand_put(cand, s0 + p, keys[1], 0u);
+    }
+    pairs_distances<R>(rows, S.id, nw + nu, S.x, t, on, acc);
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        if (!on[r]) continue;
+        const bool neu = t[r].a0 < nw + nuN;
+        const int iend = neu ? nuN : nu, jend = neu ? nw : nwN;
+#pragma unroll
+        for (int x = 0; x < 4; ++x)
+#pragma unroll
+            for (int y = 0; y < 4; ++y) {
+                const int i = t[r].a0 + x * t[r].as - nw, j = t[r].b0 + y * t[r].bs;
+                if (i < iend && j < jend) S.x[i * (PJ_COLS + 1) + j] = acc[r][4 * x + y];
+            }
+    }
+    __syncwarp();
+}
+
+template <class RowsT>
+__global__ void __launch_bounds__(PJ_WARPS * 32, 3) p2k_warp_kernel(RowsT rows, uint32_t N,
+                                                                   const uint64_t *__restrict__ off,
+                                                                   const uint32_t *__restrict__ rnn,
+                                                                   const uint32_t *__restrict__ g_ids,
+                                                                   const uint32_t *__restrict__ g_deg,
+                                                                   const uint8_t *__restrict__ g_isnew, uint32_t W,
+                                                                   const float *__restrict__ radius,
+                                                                   uint64_t *__restrict__ cand,
+                                                                   uint32_t *__restrict__ cand_cnt, uint32_t CB,
+                                                                   unsigned long long *comps) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int lane = kcna_lane();
+    P2kWarp &S = reinterpret_cast<P2kWarp *>(smem)[threadIdx.x >> 5];
+    unsigned long long cc = 0;
+    for (uint32_t q = blockIdx.x * PJ_WARPS + (threadIdx.x >> 5); q < N; q += gridDim.x * PJ_WARPS) {
+        const uint64_t r0 = off[q], r1 = off[q + 1];
+        if (r0 == r1) continue;
+        const int deg = (int)min(g_deg[q], W);
+        for (int c0 = 0; c0 < deg; c0 += PJ_COLS) { // graph rows wider than 64: column chunks
+            const int nwAll = min(PJ_COLS, deg - c0);
+            uint32_t w[2];
+            unsigned mN[2], mO[2];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int j = lane + 32 * h;
+                const bool in = j < nwAll;
+                const uint64_t at = (uint64_t)q * W + c0 + j;
+                w[h] = in ? g_ids[at] : KCNA_NONE;
+                const bool f = in && g_isnew[at];
+                mN[h] = __ballot_sync(KCNA_FULL, f);
+                mO[h] = __ballot_sync(KCNA_FULL, in && !f);
+            }
+            const int nwN = __popc(mN[0]) + __popc(mN[1]);
+            __syncwarp(); // the previous chunk's ids are read
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const unsigned lt = kcna_lanemask_lt();
+                if ((mN[h] >> lane) & 1u) S.id[(h ? __popc(mN[0]) : 0) + __popc(mN[h] & lt)] = w[h];
+                if ((mO[h] >> lane) & 1u) S.id[nwN + (h ? __popc(mO[0]) : 0) + __popc(mO[h] & lt)] = w[h];
+            }
+            const int cap_u = min(PJ_U, PJ_ROWS - nwAll);
+            for (uint64_t t0 = r0; t0 < r1; t0 += cap_u) {
+                const bool in = lane < cap_u && t0 + lane < r1;
+                const uint32_t v = in ? rnn[t0 + lane] : 0u;
+                const uint32_t u = (v & 0x7FFFFFFFu) < N ? (v & 0x7FFFFFFFu) : 0u;
+                const unsigned uN = __ballot_sync(KCNA_FULL, in && (v >> 31));
+                const unsigned uO = nwN ? __ballot_sync(KCNA_FULL, in && !(v >> 31)) : 0u;
+                const int nuN = __popc(uN), nu = nuN + __popc(uO);
+                if (nu == 0) continue;
+                const int nw = nuN ? nwAll : nwN; // neighbours somebody meets
+                int pos = -1;
+                if ((uN >> lane) & 1u) pos = __popc(uN & kcna_lanemask_lt());
+                if ((uO >> lane) & 1u) pos = nuN + __popc(uO & kcna_lanemask_lt());
+                // with old pushers only, the pushers take the place of the old neighbours' ids; these
+                // are not needed again: the next pushers' chunk has them loaded anew below
+                uint32_t keep = KCNA_NONE; // this lane's old-neighbour id, put back after the chunk
+                const bool spare = nw < nwAll;
+                __syncwarp();
+                const int kpos = nw + lane;
+                if (spare && lane < nu && kpos < nwAll) keep = S.id[kpos];
+                __syncwarp();
+                if (pos >= 0) {
+                    S.id[nw + pos] = u;
+                    S.rad[pos] = __ldg(radius + u);
+                }
+                __syncwarp();
+                const int T = ((nuN + 3) >> 2) * ((nw + 3) >> 2) + ((nu - nuN + 3) >> 2) * ((nwN + 3) >> 2);
+                if (T <= 32)
+                    p2k_warp_tiles<1>(rows, S, nw, nwN, nu, nuN, T);
+                else if (T <= 64)
+                    p2k_warp_tiles<2>(rows, S, nw, nwN, nu, nuN, T);
+                else
+                    p2k_warp_tiles<PT_MAXR>(rows, S, nw, nwN, nu, nuN, T);
+                // count pass (lane i keeps pusher i's ballots), reservations together, write pass
+                uint32_t m0 = 0u, m1 = 0u, base = 0u;
+                auto meets = [&](int i, int j, uint32_t uid, bool &ok) {
+                    ok = false;
+                    if (j >= (i < nuN ? nw : nwN) || S.id[j] == uid) return;
+                    ++cc;
+                    ok = S.x[i * (PJ_COLS + 1) + j] <= S.rad[i];
+                };
+                for (int i = 0; i < nu; ++i) {
+                    const uint32_t uid = S.id[nw + i];
+                    bool o0, o1 = false;
+                    meets(i, lane, uid, o0);
+                    meets(i, lane + 32, uid, o1);
+                    const uint32_t b0 = __ballot_sync(KCNA_FULL, o0), b1 = __ballot_sync(KCNA_FULL, o1);
+                    if (lane == i) {
+                        m0 = b0;
+                        m1 = b1;
+                    }
+                }
+                const uint32_t cnt = __popc(m0) + __popc(m1);
+                if (cnt) base = atomicAdd(cand_cnt + S.id[nw + lane], cnt);
+                for (int i = 0; i < nu; ++i) {
+                    const uint32_t b0 = __shfl_sync(KCNA_FULL, m0, i), b1 = __shfl_sync(KCNA_FULL, m1, i);
+                    const uint32_t at = __shfl_sync(KCNA_FULL, base, i);
+                    const uint64_t s0 = (uint64_t)S.id[nw + i] * CB; // whole slots, joiner 0 (no credit)
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const uint32_t b = h ? b1 : b0;
+                        if (!((b >> lane) & 1u)) continue;
+                        const int j = lane + 32 * h;
+                        const uint32_t p = at + (h ? __popc(b0) : 0) + __popc(b & kcna_lanemask_lt());
+                        if (p < CB)
+                            kcna_cand_put(cand, s0 + p, kcna_key(S.x[i * (PJ_COLS + 1) + j], S.id[j],
+                                                                 (uint32_t)(KCNA_FLAG_NEW | KCNA_FLAG_ISNEW)), 0u);
+                    }
+                }
+                __syncwarp();
+                if (keep != KCNA_NONE) S.id[kpos] = keep;
+            }
         }
     }
     cc = kcna_warp_sum(cc);
-    if (lane == 0 && cc) atomicAdd(s_cc, cc);
-    __syncthreads();
-}
-
-template <int RMAX>
-constexpr size_t p2k_smem_bytes() {
-    return (size_t)(RMAX * PJP + PJC * PJP + RMAX * (PJC + 1)) * sizeof(float);
-}
-
-// RMAX = 32: nodes with at most 32 pushers (almost all), 22 KB of shared memory
-// so eight blocks fit per SM; RMAX = 128: the other nodes, in row tiles of 128.
-template <int RMAX, class R>
-__global__ void __launch_bounds__(PJT) p2k_join_kernel(R rows, int ld, uint32_t N,
-                                                       const uint64_t *__restrict__ off,
-                                                       const uint32_t *__restrict__ rnn,
-                                                       const uint32_t *__restrict__ g_ids,
-                                                       const uint32_t *__restrict__ g_deg,
-                                                       const uint8_t *__restrict__ g_isnew, uint32_t W,
-                                                       const float *__restrict__ radius, uint64_t *__restrict__ cand,
-                                                       uint32_t *__restrict__ cand_cnt, uint32_t CB,
-                                                       unsigned long long *comps) {
-    extern __shared__ __align__(16) unsigned char smem[];
-    float *s_As = reinterpret_cast<float *>(smem); // RMAX x PJP
-    float *s_Bs = s_As + RMAX * PJP;               // PJC x PJP
-    float *s_D = s_Bs + PJC * PJP;                 // RMAX x (PJC+1)
-    __shared__ uint32_t s_u[RMAX], s_w[PJC];
-    __shared__ uint8_t s_unew[RMAX], s_wnew[PJC];
-    __shared__ unsigned long long s_cc;
-    __shared__ int s_n;
-    const uint32_t q = blockIdx.x;
-    const uint64_t r0 = off[q], r1 = off[q + 1];
-    const int deg = (int)min(g_deg[q], W);
-    if (r0 == r1 || deg == 0) return;
-    if ((RMAX == 32) != (r1 - r0 <= 32)) return; // each node is handled by one of the two instances
-    if (threadIdx.x == 0) s_cc = 0;
-    for (int c0 = 0; c0 < deg; c0 += PJC) { // graph rows wider than 64: column chunks
-        const int nw = min(PJC, deg - c0);
-        __syncthreads();
-        int wn = 0;
-        for (int j = threadIdx.x; j < nw; j += PJT) {
-            s_w[j] = g_ids[(uint64_t)q * W + c0 + j];
-            s_wnew[j] = g_isnew[(uint64_t)q * W + c0 + j];
-            wn |= s_wnew[j];
-        }
-        // a pair of an old pusher and an old neighbour is skipped
-        // (src/kgraph.cpp:2639-2641): without a new neighbour in this chunk only
-        // the new pushers enter the tile, and a tile without pushers is skipped
-        const bool any_wnew = __syncthreads_or(wn) != 0;
-        for (uint64_t t0 = r0; t0 < r1; t0 += RMAX) {
-            const int nraw = (int)min((uint64_t)RMAX, r1 - t0);
-            __syncthreads();
-            if (threadIdx.x == 0) s_n = 0;
-            __syncthreads();
-            for (int i = threadIdx.x; i < nraw; i += PJT) {
-                const uint32_t v = rnn[t0 + i];
-                if (!any_wnew && !(v & 0x80000000u)) continue;
-                const uint32_t u = v & 0x7FFFFFFFu;
-                const int k = atomicAdd(&s_n, 1);
-                s_u[k] = u < N ? u : 0;
-                s_unew[k] = (v & 0x80000000u) ? 1 : 0;
-            }
-            __syncthreads();
-            const int nu = s_n;
-            if (nu == 0) continue;
-            if (RMAX == 32 || nu <= 32)
-                p2k_tile<1>(rows, ld, N, s_u, s_unew, nu, s_w, s_wnew, nw, radius, cand, cand_cnt, CB, s_As, s_Bs, s_D,
-                            &s_cc);
-            else if (nu <= 64)
-                p2k_tile<RMAX >= 64 ? 2 : 1>(rows, ld, N, s_u, s_unew, nu, s_w, s_wnew, nw, radius, cand, cand_cnt, CB,
-                                             s_As, s_Bs, s_D, &s_cc);
-            else
-                p2k_tile<RMAX >= 128 ? 4 : 1>(rows, ld, N, s_u, s_unew, nu, s_w, s_wnew, nw, radius, cand, cand_cnt, CB,
-                                              s_As, s_Bs, s_D, &s_cc);
-        }
-    }
-    if (threadIdx.x == 0 && s_cc) atomicAdd(comps, s_cc);
+    if (lane == 0 && cc) atomicAdd(comps, cc);
 }
 
 PruneRule make_rule(const kcna_params *p, int kind) {
@@ -1707,16 +1718,22 @@ kcna_status kcna_bridge_view(kcna_ctx *c, const kcna_params *p, uint32_t maxl, i
         count_new_edges_kernel<<<wblocks, 256, 0, c->stream>>>(c->g_isnew, c->g_deg, N, c->W, nnew);
         KCNA_LAUNCHED(c);
     }
-    if ((s = kcna_cuda_check(c, cudaFuncSetAttribute(p2k_join_kernel<128, RowsF32>,
-                                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                     (int)p2k_smem_bytes<128>()),
-                             "p2k smem attr")) != KCNA_OK)
-        return cleanup(), s;
-    if ((s = kcna_cuda_check(c, cudaFuncSetAttribute(p2k_join_kernel<128, RowsB16>,
-                                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                     (int)p2k_smem_bytes<128>()),
-                             "p2k smem attr")) != KCNA_OK)
-        return cleanup(), s;
+    // FP32 join (or the exact BF16 copy outside the Gram tiles' range): warp per node
+    auto join_fp32 = [&](auto rows) -> kcna_status {
+        auto kern = p2k_warp_kernel<decltype(rows)>;
+        const size_t sm = PJ_WARPS * sizeof(P2kWarp);
+        int per_sm = 0;
+        KCNA_TRY(kcna_cuda_check(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm),
+                                 "p2k smem attr"));
+        KCNA_TRY(kcna_cuda_check(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, PJ_WARPS * 32, sm),
+                                 "p2k occupancy"));
+        const uint32_t grid = std::min(kcna_div_up(N, PJ_WARPS),
+                                       (uint32_t)std::max(c->num_sms, 1) * (uint32_t)std::max(per_sm, 1));
+        kern<<<grid, PJ_WARPS * 32, sm, c->stream>>>(rows, N, off, rnn, c->g_ids, c->g_deg, c->g_isnew, c->W, c->radius,
+                                                     c->cand, c->cand_cnt, c->CB, c->counters + 21);
+        KCNA_LAUNCHED(c);
+        return kcna_cuda_check(c, cudaGetLastError(), "p2k_warp_kernel");
+    };
     // the reference loops until a thin round; 100 rounds bound it here
     for (int round = 0; round < 100; ++round) {
         // capped round: count, then the uncapped remainder when the round is thin
@@ -1763,24 +1780,10 @@ kcna_status kcna_bridge_view(kcna_ctx *c, const kcna_params *p, uint32_t maxl, i
         cudaMemsetAsync(c->counters + 21, 0, 8, c->stream);
         if (tc) {
             if ((s = kcna_p2k_tc_launch(c, off, rnn, nnew, pnew, c->counters + 21)) != KCNA_OK) return cleanup(), s;
-        } else if (c->bf16_exact) {
-            const RowsB16 rows{c->Xh, (int)c->ld};
-            p2k_join_kernel<32><<<N, PJT, p2k_smem_bytes<32>(), c->stream>>>(
-                rows, (int)c->ld, N, off, rnn, c->g_ids, c->g_deg, c->g_isnew, c->W, c->radius, c->cand, c->cand_cnt,
-                c->CB, c->counters + 21);
-            p2k_join_kernel<128><<<N, PJT, p2k_smem_bytes<128>(), c->stream>>>(
-                rows, (int)c->ld, N, off, rnn, c->g_ids, c->g_deg, c->g_isnew, c->W, c->radius, c->cand, c->cand_cnt,
-                c->CB, c->counters + 21);
         } else {
-            const RowsF32 rows{c->X, (int)c->ld};
-            p2k_join_kernel<32><<<N, PJT, p2k_smem_bytes<32>(), c->stream>>>(
-                rows, (int)c->ld, N, off, rnn, c->g_ids, c->g_deg, c->g_isnew, c->W, c->radius, c->cand, c->cand_cnt,
-                c->CB, c->counters + 21);
-            p2k_join_kernel<128><<<N, PJT, p2k_smem_bytes<128>(), c->stream>>>(
-                rows, (int)c->ld, N, off, rnn, c->g_ids, c->g_deg, c->g_isnew, c->W, c->radius, c->cand, c->cand_cnt,
-                c->CB, c->counters + 21);
+            s = c->bf16_exact ? join_fp32(RowsB16{c->Xh, (int)c->ld}) : join_fp32(RowsF32{c->X, (int)c->ld});
+            if (s != KCNA_OK) return cleanup(), s;
         }
-        if (!tc) c->launches += 2; // the FP32 pair
         unsigned long long h = 0;
         cudaMemcpyAsync(&h, c->counters + 21, 8, cudaMemcpyDeviceToHost, c->stream);
         if ((s = kcna_phase_end(c, KCNA_PHASE_P2K)) != KCNA_OK) return cleanup(), s;
