@@ -991,18 +991,19 @@ __global__ void count_new_edges_kernel(const uint8_t *__restrict__ g_isnew, cons
 // old (src/kgraph.cpp:2639-2641), so new pushers meet all neighbours, old
 // pushers only the new ones, and rows without a partner are not read.
 // Survivors within u's radius become candidates of u, one run per (q, u) after
-// one atomicAdd.  A node has about 10 pushers and 26 neighbours (C2): the block
-// per node that this replaces computed a 32 x 64 tile for those 260 pairs, and
-// its rounds on 150,001 x 128 rows took 2.6 ms each (P2K_MS here).
-// 23 KB a warp: nine warps an SM.
-constexpr int PJ_WARPS = 3, PJ_ROWS = 80, PJ_COLS = 64, PJ_U = 32;
+// one atomicAdd.  A node has about 10 pushers and 26 neighbours (C2): a block
+// per node with a 32 x 64 tile for those 260 pairs took 2.6 ms a round on
+// 150,001 x 128 rows (1.1 ms here).  What is left is the latency of a node's
+// loads, so its ids come while the node before it is computed, and the radii
+// while its rows do.  13.7 KB a warp: sixteen warps an SM.
+constexpr int PJ_WARPS = 16, PJ_ROWS = 80, PJ_COLS = 64, PJ_U = 24;
 struct P2kWarp {
-    float x[(PJ_ROWS + PT_SPARE) * PT_P]; // rows, then the distance matrix: pusher i at i * (PJ_COLS + 1)
-    uint32_t id[PJ_ROWS];                 // neighbours, then pushers
+    float x[pairs_region(PJ_ROWS)]; // rows, then the distance matrix: pusher i at i * (PJ_COLS + 1)
+    uint32_t id[PJ_ROWS];           // neighbours, then pushers
     float rad[PJ_U];
 };
-static_assert(PJ_U * (PJ_COLS + 1) <= (PJ_ROWS + PT_SPARE) * PT_P, "the distance matrix fits the rows' region");
-static_assert((PJ_U / 4) * (PJ_COLS / 4) <= PT_MAXT, "a tile's micro-tiles fit the lanes");
+static_assert(PJ_U * (PJ_COLS + 1) <= pairs_region(PJ_ROWS), "the distance matrix fits the rows' region");
+static_assert((PJ_U / 4) * (PJ_COLS / 4) <= 32 * PT_MAXR, "a tile's micro-tiles fit the lanes");
 
 // rows [0, nw): neighbours, the first nwN new; [nw, nw + nu): pushers, the first nuN new
 template <int R, class RowsT>
@@ -1026,7 +1027,7 @@ __device__ __forceinline__ void p2k_warp_tiles(const RowsT &rows, P2kWarp &S, in
             }
         }
     }
-    pairs_distances<R>(rows, S.id, nw + nu, S.x, t, on, acc);
+    pairs_distances<32, R>(rows, S.id, nw + nu, S.x, t, on, acc);
 #pragma unroll
     for (int r = 0; r < R; ++r) {
         if (!on[r]) continue;
@@ -1040,11 +1041,18 @@ __device__ __forceinline__ void p2k_warp_tiles(const RowsT &rows, P2kWarp &S, in
                 if (i < iend && j < jend) S.x[i * (PJ_COLS + 1) + j] = acc[r][4 * x + y];
             }
     }
-    __syncwarp();
 }
 
+// One unit of work: neighbours [c0, c0 + 64) of q against pushers [t0, t0 +
+// cap): each lane's neighbours (two), their flags, and its pusher.
+struct P2kUnit {
+    uint32_t q, w[2], v;
+    int nw, cap;
+    bool f[2], in;
+};
+
 template <class RowsT>
-__global__ void __launch_bounds__(PJ_WARPS * 32, 3) p2k_warp_kernel(RowsT rows, uint32_t N,
+__global__ void __launch_bounds__(PJ_WARPS * 32, 1) p2k_warp_kernel(RowsT rows, uint32_t N,
                                                                    const uint64_t *__restrict__ off,
                                                                    const uint32_t *__restrict__ rnn,
                                                                    const uint32_t *__restrict__ g_ids,
@@ -1058,105 +1066,141 @@ __global__ void __launch_bounds__(PJ_WARPS * 32, 3) p2k_warp_kernel(RowsT rows, 
     const int lane = kcna_lane();
     P2kWarp &S = reinterpret_cast<P2kWarp *>(smem)[threadIdx.x >> 5];
     unsigned long long cc = 0;
-    for (uint32_t q = blockIdx.x * PJ_WARPS + (threadIdx.x >> 5); q < N; q += gridDim.x * PJ_WARPS) {
-        const uint64_t r0 = off[q], r1 = off[q + 1];
-        if (r0 == r1) continue;
-        const int deg = (int)min(g_deg[q], W);
-        for (int c0 = 0; c0 < deg; c0 += PJ_COLS) { // graph rows wider than 64: column chunks
-            const int nwAll = min(PJ_COLS, deg - c0);
-            uint32_t w[2];
-            unsigned mN[2], mO[2];
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int j = lane + 32 * h;
-                const bool in = j < nwAll;
-                const uint64_t at = (uint64_t)q * W + c0 + j;
-                w[h] = in ? g_ids[at] : KCNA_NONE;
-                const bool f = in && g_isnew[at];
-                mN[h] = __ballot_sync(KCNA_FULL, f);
-                mO[h] = __ballot_sync(KCNA_FULL, in && !f);
+    // this warp's share of the pushes, [p0, p1): equal shares, so that a hub's
+    // pushers are split among warps (with nodes dealt out instead, the warps with
+    // the hubs ran four times as long as the rest on 40,009 x 960 rows)
+    const uint64_t total = off[N], G = (uint64_t)gridDim.x * PJ_WARPS, gw = blockIdx.x * PJ_WARPS + (threadIdx.x >> 5);
+    const uint64_t share = (total + G - 1) / G, p0 = min(total, gw * share), p1 = min(total, p0 + share);
+    if (p0 == p1) return;
+    // the last node whose pushers begin at or before p0
+    uint32_t q0 = 0;
+    for (uint32_t hi = N; hi - q0 > 1;) {
+        const uint32_t mid = q0 + (hi - q0) / 2;
+        if (off[mid] <= p0)
+            q0 = mid;
+        else
+            hi = mid;
+    }
+    // pushers' range and degree of 32 nodes from `at`, one per lane
+    uint64_t m0 = 0, m1 = 0;
+    int md = 0;
+    // the walk: node `at` (its place j among the 32), its pushers [t0, r1) and neighbours [c0, deg) to come
+    uint64_t at = q0, r0 = 0, r1 = 0, t0 = 0;
+    int j = -1, deg = 0, c0 = 0;
+    auto next = [&](P2kUnit &u) -> bool { // loads only: nothing is waited for
+        while (c0 >= deg || t0 >= r1) {
+            if (c0 < deg && (c0 += PJ_COLS) < deg) { // the next neighbours, all pushers again
+                t0 = r0;
+                break;
             }
-            const int nwN = __popc(mN[0]) + __popc(mN[1]);
-            __syncwarp(); // the previous chunk's ids are read
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const unsigned lt = kcna_lanemask_lt();
-                if ((mN[h] >> lane) & 1u) S.id[(h ? __popc(mN[0]) : 0) + __popc(mN[h] & lt)] = w[h];
-                if ((mO[h] >> lane) & 1u) S.id[nwN + (h ? __popc(mO[0]) : 0) + __popc(mO[h] & lt)] = w[h];
+            if (j >= 0) ++at;
+            if (at >= N) return false;
+            j = (j + 1) & 31;
+            if (j == 0) {
+                const uint64_t q = at + lane;
+                m0 = q < N ? max(off[q], p0) : p1;
+                m1 = q < N ? min(off[q + 1], p1) : p1;
+                md = q < N ? (int)min(g_deg[q], W) : 0;
             }
-            const int cap_u = min(PJ_U, PJ_ROWS - nwAll);
-            for (uint64_t t0 = r0; t0 < r1; t0 += cap_u) {
-                const bool in = lane < cap_u && t0 + lane < r1;
-                const uint32_t v = in ? rnn[t0 + lane] : 0u;
-                const uint32_t u = (v & 0x7FFFFFFFu) < N ? (v & 0x7FFFFFFFu) : 0u;
-                const unsigned uN = __ballot_sync(KCNA_FULL, in && (v >> 31));
-                const unsigned uO = nwN ? __ballot_sync(KCNA_FULL, in && !(v >> 31)) : 0u;
-                const int nuN = __popc(uN), nu = nuN + __popc(uO);
-                if (nu == 0) continue;
-                const int nw = nuN ? nwAll : nwN; // neighbours somebody meets
-                int pos = -1;
-                if ((uN >> lane) & 1u) pos = __popc(uN & kcna_lanemask_lt());
-                if ((uO >> lane) & 1u) pos = nuN + __popc(uO & kcna_lanemask_lt());
-                // with old pushers only, the pushers take the place of the old neighbours' ids; these
-                // are not needed again: the next pushers' chunk has them loaded anew below
-                uint32_t keep = KCNA_NONE; // this lane's old-neighbour id, put back after the chunk
-                const bool spare = nw < nwAll;
-                __syncwarp();
-                const int kpos = nw + lane;
-                if (spare && lane < nu && kpos < nwAll) keep = S.id[kpos];
-                __syncwarp();
-                if (pos >= 0) {
-                    S.id[nw + pos] = u;
-                    S.rad[pos] = __ldg(radius + u);
-                }
-                __syncwarp();
-                const int T = ((nuN + 3) >> 2) * ((nw + 3) >> 2) + ((nu - nuN + 3) >> 2) * ((nwN + 3) >> 2);
-                if (T <= 32)
-                    p2k_warp_tiles<1>(rows, S, nw, nwN, nu, nuN, T);
-                else if (T <= 64)
-                    p2k_warp_tiles<2>(rows, S, nw, nwN, nu, nuN, T);
-                else
-                    p2k_warp_tiles<PT_MAXR>(rows, S, nw, nwN, nu, nuN, T);
-                // count pass (lane i keeps pusher i's ballots), reservations together, write pass
-                uint32_t m0 = 0u, m1 = 0u, base = 0u;
-                auto meets = [&](int i, int j, uint32_t uid, bool &ok) {
-                    ok = false;
-                    if (j >= (i < nuN ? nw : nwN) || S.id[j] == uid) return;
-                    ++cc;
-                    ok = S.x[i * (PJ_COLS + 1) + j] <= S.rad[i];
-                };
-                for (int i = 0; i < nu; ++i) {
-                    const uint32_t uid = S.id[nw + i];
-                    bool o0, o1 = false;
-                    meets(i, lane, uid, o0);
-                    meets(i, lane + 32, uid, o1);
-                    const uint32_t b0 = __ballot_sync(KCNA_FULL, o0), b1 = __ballot_sync(KCNA_FULL, o1);
-                    if (lane == i) {
-                        m0 = b0;
-                        m1 = b1;
-                    }
-                }
-                const uint32_t cnt = __popc(m0) + __popc(m1);
-                if (cnt) base = atomicAdd(cand_cnt + S.id[nw + lane], cnt);
-                for (int i = 0; i < nu; ++i) {
-                    const uint32_t b0 = __shfl_sync(KCNA_FULL, m0, i), b1 = __shfl_sync(KCNA_FULL, m1, i);
-                    const uint32_t at = __shfl_sync(KCNA_FULL, base, i);
-                    const uint64_t s0 = (uint64_t)S.id[nw + i] * CB; // whole slots, joiner 0 (no credit)
+            r0 = t0 = __shfl_sync(KCNA_FULL, m0, j);
+            r1 = __shfl_sync(KCNA_FULL, m1, j);
+            deg = __shfl_sync(KCNA_FULL, md, j);
+            c0 = 0;
+            if (t0 >= p1) return false; // the next warp's
+            if (t0 >= r1) c0 = deg;     // no pushers: the next node
+        }
+        u.q = (uint32_t)at;
+        u.nw = min(PJ_COLS, deg - c0);
+        u.cap = min(PJ_U, PJ_ROWS - u.nw);
 #pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        const uint32_t b = h ? b1 : b0;
-                        if (!((b >> lane) & 1u)) continue;
-                        const int j = lane + 32 * h;
-                        const uint32_t p = at + (h ? __popc(b0) : 0) + __popc(b & kcna_lanemask_lt());
-                        if (p < CB)
-                            kcna_cand_put(cand, s0 + p, kcna_key(S.x[i * (PJ_COLS + 1) + j], S.id[j],
-                                                                 (uint32_t)(KCNA_FLAG_NEW | KCNA_FLAG_ISNEW)), 0u);
-                    }
-                }
-                __syncwarp();
-                if (keep != KCNA_NONE) S.id[kpos] = keep;
+        for (int h = 0; h < 2; ++h) {
+            const int k = lane + 32 * h;
+            const uint64_t e = at * W + c0 + k;
+            u.w[h] = k < u.nw ? __ldg(g_ids + e) : KCNA_NONE;
+            u.f[h] = k < u.nw && __ldg(g_isnew + e);
+        }
+        u.in = lane < u.cap && t0 + lane < r1;
+        u.v = u.in ? __ldg(rnn + t0 + lane) : 0u;
+        t0 += u.cap;
+        return true;
+    };
+    P2kUnit c, nx;
+    bool have = next(c);
+    while (have) {
+        // new ones first, neighbours then pushers
+        const unsigned lt = kcna_lanemask_lt();
+        const unsigned n0 = __ballot_sync(KCNA_FULL, c.f[0]), n1 = __ballot_sync(KCNA_FULL, c.f[1]);
+        const int nwN = __popc(n0) + __popc(n1);
+        const unsigned uN = __ballot_sync(KCNA_FULL, c.in && (c.v >> 31));
+        const unsigned uO = nwN ? __ballot_sync(KCNA_FULL, c.in && !(c.v >> 31)) : 0u;
+        const int nuN = __popc(uN), nu = nuN + __popc(uO);
+        const int nw = nuN ? c.nw : nwN; // neighbours somebody meets
+        const uint32_t u = (c.v & 0x7FFFFFFFu) < N ? (c.v & 0x7FFFFFFFu) : 0u;
+        if (nu == 0 || nw == 0) {
+            have = next(c);
+            continue;
+        }
+        int pos = -1;
+        if ((uN >> lane) & 1u) pos = __popc(uN & lt);
+        if ((uO >> lane) & 1u) pos = nuN + __popc(uO & lt);
+        if (c.f[0]) S.id[__popc(n0 & lt)] = c.w[0];
+        if (c.f[1]) S.id[__popc(n0) + __popc(n1 & lt)] = c.w[1];
+        if (nuN) { // old neighbours: lanes below this one that hold a neighbour not flagged new
+            if (lane < c.nw && !c.f[0]) S.id[nwN + __popc(~n0 & lt)] = c.w[0];
+            if (lane + 32 < c.nw && !c.f[1]) S.id[nwN + __popc(~n0) + __popc(~n1 & lt)] = c.w[1];
+        }
+        float rad = 0.f;
+        if (pos >= 0) {
+            S.id[nw + pos] = u;
+            rad = __ldg(radius + u); // consumed after the distances
+        }
+        __syncwarp();
+        const bool more = next(nx);
+        const int T = ((nuN + 3) >> 2) * ((nw + 3) >> 2) + ((nu - nuN + 3) >> 2) * ((nwN + 3) >> 2);
+        if (T <= 32)
+            p2k_warp_tiles<1>(rows, S, nw, nwN, nu, nuN, T);
+        else if (T <= 64)
+            p2k_warp_tiles<2>(rows, S, nw, nwN, nu, nuN, T);
+        else
+            p2k_warp_tiles<PT_MAXR>(rows, S, nw, nwN, nu, nuN, T);
+        if (pos >= 0) S.rad[pos] = rad;
+        __syncwarp();
+        // count pass (lane i keeps pusher i's ballots), reservations together, write pass
+        uint32_t b0 = 0u, b1 = 0u, base = 0u;
+        auto meets = [&](int i, int k, uint32_t uid) {
+            if (k >= (i < nuN ? nw : nwN) || S.id[k] == uid) return false;
+            ++cc;
+            return S.x[i * (PJ_COLS + 1) + k] <= S.rad[i];
+        };
+        for (int i = 0; i < nu; ++i) {
+            const uint32_t uid = S.id[nw + i];
+            const uint32_t x0 = __ballot_sync(KCNA_FULL, meets(i, lane, uid));
+            const uint32_t x1 = nw > 32 ? __ballot_sync(KCNA_FULL, meets(i, lane + 32, uid)) : 0u;
+            if (lane == i) {
+                b0 = x0;
+                b1 = x1;
             }
         }
+        const uint32_t cnt = __popc(b0) + __popc(b1);
+        if (cnt) base = atomicAdd(cand_cnt + S.id[nw + lane], cnt);
+        for (int i = 0; i < nu; ++i) {
+            const uint32_t x0 = __shfl_sync(KCNA_FULL, b0, i), x1 = __shfl_sync(KCNA_FULL, b1, i);
+            const uint32_t to = __shfl_sync(KCNA_FULL, base, i);
+            const uint64_t s0 = (uint64_t)S.id[nw + i] * CB; // whole slots, joiner 0 (no credit)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const uint32_t x = h ? x1 : x0;
+                const int k = lane + 32 * h;
+                const uint32_t p = to + (h ? __popc(x0) : 0) + __popc(x & lt);
+                if (((x >> lane) & 1u) && p < CB)
+                    kcna_cand_put(cand, s0 + p,
+                                  kcna_key(S.x[i * (PJ_COLS + 1) + k], S.id[k], (uint32_t)(KCNA_FLAG_NEW | KCNA_FLAG_ISNEW)),
+                                  0u);
+            }
+        }
+        __syncwarp(); // the next unit reuses the region
+        have = more;
+        c = nx;
     }
     cc = kcna_warp_sum(cc);
     if (lane == 0 && cc) atomicAdd(comps, cc);

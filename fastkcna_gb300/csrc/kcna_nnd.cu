@@ -6,8 +6,7 @@
 // statistics / stop rule (:1365-1426).
 //
 // GPU form of one iteration:
-//   join    one warp per node n (one block for the few nodes with more than 64
-//           rows): gather the node's new list A and old list B, compute every
+//   join    one warp per node n (a block for a node of more than 64 rows): gather the node's new list A and old list B, compute every
 //           pair of A x A (i < j) and A x B with the canonical FMA-chain
 //           distance in register tiles (rows staged through shared memory),
 //           and emit each pair to both endpoints' candidate buffers when it is
@@ -253,11 +252,11 @@ __device__ void join_tiles(const JoinArgs &a, const R &rows, uint32_t node, cons
     }
 }
 
-// Join of the nodes queued by join_warp_kernel (more rows than a warp's region
-// holds): block per node, persistent over the queue.
+// Join of the nodes with more rows than join_set_kernel's regions hold: block
+// per node, persistent over the queue (from the end of `list` down).
 template <class R>
-__global__ void __launch_bounds__(JT, 3) join_kernel(JoinArgs a, R rows, const uint32_t *__restrict__ big_list,
-                                                     const uint32_t *__restrict__ big_cnt) {
+__global__ void __launch_bounds__(JT, 3) join_kernel(JoinArgs a, R rows, const uint32_t *__restrict__ list,
+                                                     const uint32_t *__restrict__ cnt) {
     extern __shared__ __align__(16) unsigned char smem[];
     float *s_As = reinterpret_cast<float *>(smem);                // 128 x JKP
     float *s_Bs = s_As + 128 * JKP;                               // JCOLS x JKP
@@ -266,9 +265,9 @@ __global__ void __launch_bounds__(JT, 3) join_kernel(JoinArgs a, R rows, const u
     uint32_t *s_A = reinterpret_cast<uint32_t *>(s_radA + a.capA); // capA
     uint32_t *s_B = s_A + a.capA;                                 // capB
     __shared__ unsigned s_emit;
-    const uint32_t n_big = *big_cnt;
+    const uint32_t n_big = cnt[1];
     for (uint32_t bi = blockIdx.x; bi < n_big; bi += gridDim.x) {
-        const uint32_t node = big_list[bi];
+        const uint32_t node = list[a.N - 1 - bi];
         __syncthreads(); // the previous node's lists and tiles are read
         // new list: forward new then a random subset (<= R) of reverse new
         uint32_t fn = min(a.fwd_new_cnt[node], a.fwd_new_cap);
@@ -301,35 +300,79 @@ __global__ void __launch_bounds__(JT, 3) join_kernel(JoinArgs a, R rows, const u
     }
 }
 
-// Warp per node, persistent: the same join for nodes of at most JW_ROWS rows
-// and PT_MAXT micro-tiles (kcna_pairs.cuh); larger nodes are queued for
-// join_kernel.  The micro-tiles are those of the upper triangle of A x A and of
-// A x B.  The distances go to a matrix over the rows' region (both triangles
-// of A x A), and the warp then takes the targets one by one: a count pass (two
-// ballots a target, kept by lane target % 32), one atomicAdd per target with
-// all of them in flight together, a write pass.
-// 18.7 KB a warp: twelve warps an SM, three per scheduler, which hides the
-// gathers behind the other warps' arithmetic.  Below the line of 64 rows lie
-// 99 % of the nodes of every workload here; a region of 96 rows would hold
-// eight warps.
-constexpr int JW_WARPS = 4, JW_ROWS = 64;
-struct JoinWarp {
-    float x[(JW_ROWS + PT_SPARE) * PT_P]; // rows, then the distance matrix: row i at i * (n | 1)
-    uint32_t id[JW_ROWS];
-    float rad[JW_ROWS];
+// The same join for nodes of at most ROWS rows: NT threads per node (a warp for
+// up to 64 rows, a block of four warps for up to 160), persistent.  The pairs
+// are the 4 x 4 micro-tiles (kcna_pairs.cuh) of the upper triangle of A x A and
+// of A x B.  The distances go to a matrix over the rows' region (both triangles
+// of A x A), and each warp then takes its targets (target % warps): a count
+// pass (ballots over the target's partners, kept by lane i of the i-th target),
+// one atomicAdd per target with all of them in flight together, a write pass.
+// A node's list lengths come with those of 31 others, its ids while the node
+// before it is computed, its radii while its rows are.
+// First the warp version walks all nodes and queues larger ones in `list`:
+// those for the block version from the front (cnt[0]), those for join_kernel
+// from the end (cnt[1]).  150,001 x 128 rows (28 rows a node): 20 ms a
+// build against 47 for a block of 256 threads per node.
+// 11.5 KB a warp: sixteen warps an SM, as many as the registers allow.
+template <int NT, int ROWS>
+struct JoinSet {
+    float x[pairs_region(ROWS)]; // rows, then the distance matrix: row i at i * (n | 1)
+    uint32_t id[2][ROWS];        // this node's ids and the next one's
+    float rad[ROWS];
 };
-static_assert(JW_ROWS * (JW_ROWS + 1) <= (JW_ROWS + PT_SPARE) * PT_P, "the distance matrix fits the rows' region");
+constexpr int JW_ROWS = 64, JM_ROWS = 160, JM_NT = 128;
+using JoinWarp = JoinSet<32, JW_ROWS>;
+using JoinMid = JoinSet<JM_NT, JM_ROWS>;
 
-template <int R, class RowsT>
-__device__ __forceinline__ void join_warp_tiles(const RowsT &rows, JoinWarp &S, int na, int n, int T) {
-    const int lane = kcna_lane(), nb = n - na, GA = (na + 3) >> 2, GB = (nb + 3) >> 2;
+// sizes of one node's lists
+struct JoinLists {
+    uint32_t fn, rn, fo, ro;
+    __device__ int na() const { return (int)(fn + rn); }
+    __device__ int n() const { return (int)(fn + rn + fo + ro); }
+    __device__ int tiles() const {
+        const int ga = (na() + 3) >> 2;
+        return ga * (ga + 1) / 2 + ga * ((int)(fo + ro + 3) >> 2);
+    }
+    template <int NT, int ROWS> __device__ bool fits() const {
+        return n() <= ROWS && tiles() <= NT * PT_MAXR && na() * (n() | 1) <= pairs_region(ROWS);
+    }
+};
+__device__ __forceinline__ JoinLists join_lists(const JoinArgs &a, uint32_t node) {
+    JoinLists l;
+    l.fn = min(a.fwd_new_cnt[node], a.fwd_new_cap);
+    l.fo = min(a.fwd_old_cnt[node], a.fwd_old_cap);
+    l.rn = a.iter > 0 ? min(a.rnew_cnt[node], a.R) : 0u; // the random subsets select_reverse_kernel left first
+    l.ro = a.iter > 0 ? min(a.rold_cnt[node], a.R) : 0u;
+    return l;
+}
+// ids of the node's set (A then B) by cp.async, one group
+template <int NT>
+__device__ __forceinline__ void join_load_ids(const JoinArgs &a, uint32_t node, const JoinLists &l, uint32_t *s_id) {
+    const uint32_t na = l.fn + l.rn, n = na + l.fo + l.ro;
+    for (uint32_t u = pairs_lane<NT>(); u < n; u += NT) {
+        const uint32_t v = u - na;
+        const uint32_t *src = u < l.fn   ? a.fwd_new + (uint64_t)node * a.fwd_new_cap + u
+                              : u < na   ? a.rnew + (uint64_t)node * a.RB + (u - l.fn)
+                              : v < l.fo ? a.fwd_old + (uint64_t)node * a.fwd_old_cap + v
+                                         : a.rold + (uint64_t)node * a.RB + (v - l.fo);
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(s_id + u)),
+                     "l"(src)
+                     : "memory");
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
+template <int NT, int R, class RowsT>
+__device__ __forceinline__ void join_set_tiles(const RowsT &rows, const uint32_t *s_id, float *s_x, int na, int n,
+                                               int T) {
+    const int lane = pairs_lane<NT>(), nb = n - na, GA = (na + 3) >> 2, GB = (nb + 3) >> 2;
     const int TA = GA * (GA + 1) / 2;
     PairTile t[R];
     bool on[R];
     float acc[R][16];
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-        int k = lane + 32 * r;
+        int k = lane + NT * r;
         on[r] = k < T;
         t[r] = PairTile{0, 0, 0, 0};
         if (on[r]) {
@@ -343,7 +386,7 @@ __device__ __forceinline__ void join_warp_tiles(const RowsT &rows, JoinWarp &S, 
             }
         }
     }
-    pairs_distances<R>(rows, S.id, n, S.x, t, on, acc);
+    pairs_distances<NT, R>(rows, s_id, n, s_x, t, on, acc);
     const int dp = n | 1;
 #pragma unroll
     for (int r = 0; r < R; ++r) {
@@ -355,106 +398,169 @@ __device__ __forceinline__ void join_warp_tiles(const RowsT &rows, JoinWarp &S, 
             for (int y = 0; y < 4; ++y) {
                 const int i = t[r].a0 + x * t[r].as, j = t[r].b0 + y * t[r].bs;
                 if (i >= na || j >= (inA ? na : n)) continue;
-                S.x[i * dp + j] = acc[r][4 * x + y];
-                if (inA) S.x[j * dp + i] = acc[r][4 * x + y];
+                s_x[i * dp + j] = acc[r][4 * x + y];
+                if (inA) s_x[j * dp + i] = acc[r][4 * x + y];
             }
     }
-    __syncwarp();
 }
 
+// One node: ids in S.id[b] (landed and visible); the next node's ids are on
+// their way into S.id[b ^ 1].
+template <int NT, int ROWS, class RowsT>
+__device__ __forceinline__ void join_set(const JoinArgs &a, const RowsT &rows, JoinSet<NT, ROWS> &S, int b,
+                                         uint32_t node, const JoinLists &l, unsigned long long &emitted) {
+    constexpr int NW = NT / 32, PB = ROWS / 32; // warps; ballots per target
+    const int lane = kcna_lane(), warp = NW == 1 ? 0 : (int)(threadIdx.x >> 5);
+    const int na = l.na(), n = l.n(), T = l.tiles();
+    const uint32_t *id = S.id[b];
+    constexpr int RL = (ROWS + NT - 1) / NT;
+    float rad[RL];
+#pragma unroll
+    for (int u = 0; u < RL; ++u) { // consumed after the distances
+        const int i = pairs_lane<NT>() + NT * u;
+        rad[u] = i < n ? __ldg(a.radius + id[i]) : 0.f;
+    }
+    if (T <= NT)
+        join_set_tiles<NT, 1>(rows, id, S.x, na, n, T);
+    else if (T <= 2 * NT)
+        join_set_tiles<NT, 2>(rows, id, S.x, na, n, T);
+    else
+        join_set_tiles<NT, PT_MAXR>(rows, id, S.x, na, n, T);
+#pragma unroll
+    for (int u = 0; u < RL; ++u) {
+        const int i = pairs_lane<NT>() + NT * u;
+        if (i < n) S.rad[i] = rad[u];
+    }
+    pairs_sync<NT>(); // matrix and radii, for every thread
+    const int dp = n | 1;
+    // whether partner p (a row of the set) enters target t's buffer
+    auto dist = [&](int t, int p) { return t < na ? S.x[t * dp + p] : S.x[p * dp + t]; };
+    auto emits = [&](int t, int p) {
+        if (t < na ? p >= n || p == t : p >= na) return false;
+        return id[p] != id[t] && dist(t, p) <= S.rad[t];
+    };
+    const int nt = (n - warp + NW - 1) / NW; // this warp's targets: warp + NW * i
+    for (int i0 = 0; i0 < nt; i0 += 32) {
+        uint32_t m[PB], base = 0u, cnt = 0u; // of target i0 + lane
+#pragma unroll
+        for (int v = 0; v < PB; ++v) m[v] = 0u;
+        for (int i = i0; i < min(nt, i0 + 32); ++i) {
+            const int t = warp + NW * i;
+#pragma unroll
+            for (int v = 0; v < PB; ++v) {
+                const uint32_t bal = 32 * v < n ? __ballot_sync(KCNA_FULL, emits(t, lane + 32 * v)) : 0u;
+                if (lane == i - i0) m[v] = bal;
+            }
+        }
+#pragma unroll
+        for (int v = 0; v < PB; ++v) cnt += __popc(m[v]);
+        if (cnt) base = atomicAdd(a.cand_cnt + id[warp + NW * (i0 + lane)], cnt);
+        emitted += cnt;
+        for (int i = i0; i < min(nt, i0 + 32); ++i) {
+            const int t = warp + NW * i;
+            uint32_t at = __shfl_sync(KCNA_FULL, base, i - i0);
+            const uint64_t s0 = (uint64_t)id[t] * a.CB;
+#pragma unroll
+            for (int v = 0; v < PB; ++v) {
+                const uint32_t bits = __shfl_sync(KCNA_FULL, m[v], i - i0);
+                const int p = lane + 32 * v;
+                const uint32_t pos = at + __popc(bits & kcna_lanemask_lt());
+                if (((bits >> lane) & 1u) && pos < a.CB)
+                    kcna_cand_put(a.cand, s0 + pos,
+                                  kcna_key(dist(t, p), id[p], (uint32_t)(KCNA_FLAG_NEW | KCNA_FLAG_ISNEW)), node);
+                at += __popc(bits);
+            }
+        }
+    }
+    pairs_sync<NT>(); // the next node reuses the region
+}
+
+constexpr int JW_WARPS = 16; // of the warp version, one block an SM: they share nothing, but a block costs 1 KB
+
 template <class RowsT>
-__global__ void __launch_bounds__(JW_WARPS * 32, 3) join_warp_kernel(JoinArgs a, RowsT rows, uint32_t *big_list,
-                                                                    uint32_t *big_cnt) {
+__global__ void __launch_bounds__(JW_WARPS * 32, 1) join_warp_kernel(JoinArgs a, RowsT rows,
+                                                                     uint32_t *__restrict__ list,
+                                                                     uint32_t *__restrict__ cnt) {
     extern __shared__ __align__(16) unsigned char smem[];
     const int lane = kcna_lane();
     JoinWarp &S = reinterpret_cast<JoinWarp *>(smem)[threadIdx.x >> 5];
     unsigned long long pairs = 0, nrows = 0, emitted = 0;
-    for (uint32_t node = blockIdx.x * JW_WARPS + (threadIdx.x >> 5); node < a.N; node += gridDim.x * JW_WARPS) {
-        // new list A: forward new then a random subset (<= R) of reverse new; old list B likewise
-        const uint32_t fn = min(a.fwd_new_cnt[node], a.fwd_new_cap), fo = min(a.fwd_old_cnt[node], a.fwd_old_cap);
-        uint32_t rn = 0, ro = 0;
-        if (a.iter > 0) {
-            rn = min(a.rnew_cnt[node], a.R);
-            ro = min(a.rold_cnt[node], a.R);
+    const uint32_t gw = blockIdx.x * JW_WARPS + (threadIdx.x >> 5), G = gridDim.x * JW_WARPS;
+    // list sizes of 32 of this warp's nodes, one node per lane; the walk to the next node this version takes
+    JoinLists mine{0u, 0u, 0u, 0u};
+    uint64_t at = gw; // the next node to look at
+    int j = 0;        // its place among the 32
+    auto next = [&](JoinLists &l) -> uint32_t {
+        for (; at < a.N; at += G) {
+            if (j == 0) {
+                const uint64_t q = at + (uint64_t)lane * G;
+                mine = q < a.N ? join_lists(a, (uint32_t)q) : JoinLists{0u, 0u, 0u, 0u};
+            }
+            l.fn = __shfl_sync(KCNA_FULL, mine.fn, j);
+            l.rn = __shfl_sync(KCNA_FULL, mine.rn, j);
+            l.fo = __shfl_sync(KCNA_FULL, mine.fo, j);
+            l.ro = __shfl_sync(KCNA_FULL, mine.ro, j);
+            j = (j + 1) & 31;
+            if (l.na() == 0) continue;
+            if (!l.fits<32, JW_ROWS>()) {
+                if (lane == 0) {
+                    if (l.fits<JM_NT, JM_ROWS>())
+                        list[atomicAdd(cnt, 1u)] = (uint32_t)at;
+                    else
+                        list[a.N - 1 - atomicAdd(cnt + 1, 1u)] = (uint32_t)at;
+                }
+                continue;
+            }
+            const uint32_t node = (uint32_t)at;
+            at += G;
+            return node;
         }
-        if (fn + rn == 0) continue;
-        const uint32_t all = fn + rn + fo + ro;
-        const int na = (int)(fn + rn), n = (int)all, nb = n - na;
-        const int GA = (na + 3) >> 2, T = GA * (GA + 1) / 2 + GA * ((nb + 3) >> 2);
-        if (all > (uint32_t)JW_ROWS || T > PT_MAXT) {
-            if (lane == 0) big_list[atomicAdd(big_cnt, 1u)] = node;
-            continue;
-        }
-        for (int i = lane; i < n; i += 32) {
-            const uint32_t u = (uint32_t)i, v = u - (uint32_t)na;
-            const uint32_t id = u < fn            ? a.fwd_new[(uint64_t)node * a.fwd_new_cap + u]
-                                : u < (uint32_t)na ? a.rnew[(uint64_t)node * a.RB + (u - fn)]
-                                : v < fo           ? a.fwd_old[(uint64_t)node * a.fwd_old_cap + v]
-                                                   : a.rold[(uint64_t)node * a.RB + (v - fo)];
-            S.id[i] = id;
-            S.rad[i] = __ldg(a.radius + id);
-        }
+        return KCNA_NONE;
+    };
+    JoinLists l, ln;
+    uint32_t node = next(l);
+    if (node != KCNA_NONE) join_load_ids<32>(a, node, l, S.id[0]);
+    for (int b = 0; node != KCNA_NONE; b ^= 1) {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncwarp();
-        if (T <= 32)
-            join_warp_tiles<1>(rows, S, na, n, T);
-        else if (T <= 64)
-            join_warp_tiles<2>(rows, S, na, n, T);
-        else
-            join_warp_tiles<PT_MAXR>(rows, S, na, n, T);
-        pairs += (unsigned long long)((uint64_t)na * (na - 1) / 2 + (uint64_t)na * nb);
-        nrows += (unsigned long long)n;
-        const int dp = n | 1;
-        // whether partner p (a row of the set) enters target t's buffer, and at which distance
-        auto emits = [&](int t, int p, float &dd) {
-            if (t < na ? p >= n || p == t : p >= na) return false;
-            dd = t < na ? S.x[t * dp + p] : S.x[p * dp + t];
-            return S.id[p] != S.id[t] && dd <= S.rad[t];
-        };
-        uint32_t m0[2] = {0u, 0u}, m1[2] = {0u, 0u}, base[2] = {0u, 0u}; // of targets lane and lane + 32
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            for (int t = 32 * h; t < min(n, 32 * h + 32); ++t) {
-                float dd;
-                const uint32_t b0 = __ballot_sync(KCNA_FULL, emits(t, lane, dd));
-                const uint32_t b1 = n > 32 ? __ballot_sync(KCNA_FULL, emits(t, lane + 32, dd)) : 0u;
-                if (lane == (t & 31)) {
-                    m0[h] = b0;
-                    m1[h] = b1;
-                }
-            }
-        }
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const uint32_t cnt = __popc(m0[h]) + __popc(m1[h]);
-            if (cnt) base[h] = atomicAdd(a.cand_cnt + S.id[32 * h + lane], cnt);
-            emitted += cnt;
-        }
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            for (int t = 32 * h; t < min(n, 32 * h + 32); ++t) {
-                const uint32_t b0 = __shfl_sync(KCNA_FULL, m0[h], t & 31), b1 = __shfl_sync(KCNA_FULL, m1[h], t & 31);
-                const uint32_t at = __shfl_sync(KCNA_FULL, base[h], t & 31);
-                const uint64_t s0 = (uint64_t)S.id[t] * a.CB;
-#pragma unroll
-                for (int v = 0; v < 2; ++v) {
-                    const uint32_t b = v ? b1 : b0;
-                    if (!((b >> lane) & 1u)) continue;
-                    const int p = lane + 32 * v;
-                    const uint32_t pos = at + (v ? __popc(b0) : 0) + __popc(b & kcna_lanemask_lt());
-                    const float dd = t < na ? S.x[t * dp + p] : S.x[p * dp + t];
-                    if (pos < a.CB)
-                        kcna_cand_put(a.cand, s0 + pos, kcna_key(dd, S.id[p], (uint32_t)(KCNA_FLAG_NEW | KCNA_FLAG_ISNEW)),
-                                      node);
-                }
-            }
-        }
-        __syncwarp(); // the next node reuses the region
+        const uint32_t nn = next(ln);
+        if (nn != KCNA_NONE) join_load_ids<32>(a, nn, ln, S.id[b ^ 1]);
+        join_set<32, JW_ROWS>(a, rows, S, b, node, l, emitted);
+        pairs += (unsigned long long)l.na() * (l.na() - 1) / 2 + (unsigned long long)l.na() * (l.fo + l.ro);
+        nrows += (unsigned long long)l.n();
+        node = nn;
+        l = ln;
     }
     emitted = kcna_warp_sum(emitted);
     if (lane == 0) {
         atomicAdd(a.counters + 0, pairs);
         atomicAdd(a.counters + 5, nrows);
         atomicAdd(a.counters + 6, emitted);
+    }
+}
+
+template <class RowsT>
+__global__ void __launch_bounds__(JM_NT, 4) join_mid_kernel(JoinArgs a, RowsT rows, const uint32_t *__restrict__ list,
+                                                            const uint32_t *__restrict__ cnt) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    JoinMid &S = *reinterpret_cast<JoinMid *>(smem);
+    const uint32_t n_mid = cnt[0];
+    unsigned long long pairs = 0, nrows = 0, emitted = 0;
+    for (uint32_t i = blockIdx.x; i < n_mid; i += gridDim.x) {
+        const uint32_t node = list[i];
+        const JoinLists l = join_lists(a, node);
+        join_load_ids<JM_NT>(a, node, l, S.id[0]);
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();
+        join_set<JM_NT, JM_ROWS>(a, rows, S, 0, node, l, emitted);
+        pairs += (unsigned long long)l.na() * (l.na() - 1) / 2 + (unsigned long long)l.na() * (l.fo + l.ro);
+        nrows += (unsigned long long)l.n();
+    }
+    emitted = kcna_warp_sum(emitted);
+    if (kcna_lane() == 0 && emitted) atomicAdd(a.counters + 6, emitted);
+    if (threadIdx.x == 0 && nrows) {
+        atomicAdd(a.counters + 0, pairs);
+        atomicAdd(a.counters + 5, nrows);
     }
 }
 
@@ -1195,7 +1301,7 @@ kcna_status kcna_nnd_alloc(kcna_ctx *c, const kcna_params *p, uint32_t maxl) {
     KCNA_TRY(kcna_alloc(c, &c->cand, 2 * N * c->CB, "candidate buffers"));
     KCNA_TRY(kcna_alloc(c, &c->cand_cnt, N, "cand_cnt"));
     KCNA_TRY(kcna_alloc(c, &c->big_list, N, "merge queue"));
-    KCNA_TRY(kcna_alloc(c, &c->big_cnt, 1, "merge queue count"));
+    KCNA_TRY(kcna_alloc(c, &c->big_cnt, 2, "merge queue count"));
     if (!c->counters) KCNA_TRY(kcna_alloc(c, &c->counters, 64, "counters"));
     cudaStream_t s = c->stream;
     KCNA_TRY(kcna_cuda_check(c, cudaMemsetAsync(c->cand_cnt, 0, N * 4, s), "memset"));
@@ -1217,7 +1323,7 @@ kcna_status kcna_cand_alloc(kcna_ctx *c, const kcna_params *p) {
     KCNA_TRY(kcna_alloc(c, &c->cand, 2 * N * c->CB, "candidate buffers"));
     KCNA_TRY(kcna_alloc(c, &c->cand_cnt, N, "cand_cnt"));
     KCNA_TRY(kcna_alloc(c, &c->big_list, N, "merge queue"));
-    KCNA_TRY(kcna_alloc(c, &c->big_cnt, 1, "merge queue count"));
+    KCNA_TRY(kcna_alloc(c, &c->big_cnt, 2, "merge queue count"));
     if (!c->counters) KCNA_TRY(kcna_alloc(c, &c->counters, 64, "counters"));
     KCNA_TRY(kcna_cuda_check(c, cudaMemsetAsync(c->cand_cnt, 0, N * 4, c->stream), "memset"));
     return KCNA_OK;
@@ -1279,7 +1385,7 @@ kcna_status kcna_nnd_join(kcna_ctx *c, const kcna_params *p, int iter, uint64_t 
     // found (src/kgraph.cpp:1104,1116): cleared for every node, then set by the
     // merge for the joiners whose candidates it inserts below K
     KCNA_TRY(kcna_cuda_check(c, cudaMemsetAsync(c->found, 0, c->n, c->stream), "memset"));
-    KCNA_TRY(kcna_cuda_check(c, cudaMemsetAsync(c->big_cnt, 0, 4, c->stream), "memset"));
+    KCNA_TRY(kcna_cuda_check(c, cudaMemsetAsync(c->big_cnt, 0, 8, c->stream), "memset"));
     KCNA_TRY(kcna_phase_begin(c));
     if ((c->gram_exact || c->bf16_screen) && kcna_join_tc_fits(a)) {
         KCNA_TRY(kcna_join_tc_launch(c, a));
@@ -1302,23 +1408,29 @@ kcna_status kcna_nnd_join(kcna_ctx *c, const kcna_params *p, int iter, uint64_t 
             KCNA_TRY(kcna_cuda_check(c, cudaGetLastError(), "rescore_kernel"));
         }
     } else {
-        // warp per node; the nodes it queues (merge's queue, idle here) go to the block kernel
+        // the warp version queues larger nodes (in the merge's queue, idle here) for the other two
         auto launch = [&](auto rows) -> kcna_status {
-            auto warp_kern = join_warp_kernel<decltype(rows)>;
-            const size_t wsm = JW_WARPS * sizeof(JoinWarp);
-            int per_sm = 0;
-            KCNA_TRY(kcna_cuda_check(c, cudaFuncSetAttribute(warp_kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                             (int)wsm),
-                                     "join smem attr"));
-            KCNA_TRY(kcna_cuda_check(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, warp_kern, JW_WARPS * 32,
-                                                                                     wsm),
-                                     "join occupancy"));
             const uint32_t sms = (uint32_t)std::max(c->num_sms, 1);
-            const uint32_t grid = std::min(kcna_div_up(c->n, JW_WARPS), sms * (uint32_t)std::max(per_sm, 1));
-            warp_kern<<<grid, JW_WARPS * 32, wsm, c->stream>>>(a, rows, c->big_list, c->big_cnt);
-            KCNA_LAUNCHED(c);
+            auto grid = [&](auto kern, int threads, size_t smem, uint32_t *out) -> kcna_status {
+                int per_sm = 0;
+                KCNA_TRY(kcna_cuda_check(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                                 (int)std::max<size_t>(smem, 48 * 1024)),
+                                         "join smem attr"));
+                KCNA_TRY(kcna_cuda_check(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem),
+                                         "join occupancy"));
+                *out = std::min(kcna_div_up(c->n, threads == JM_NT ? 1 : threads / 32), sms * (uint32_t)std::max(per_sm, 1));
+                return KCNA_OK;
+            };
+            auto warp_kern = join_warp_kernel<decltype(rows)>;
+            auto mid_kern = join_mid_kernel<decltype(rows)>;
+            const size_t wsm = JW_WARPS * sizeof(JoinWarp), msm = sizeof(JoinMid);
+            uint32_t wg = 0, mg = 0;
+            KCNA_TRY(grid(warp_kern, JW_WARPS * 32, wsm, &wg));
+            KCNA_TRY(grid(mid_kern, JM_NT, msm, &mg));
+            warp_kern<<<wg, JW_WARPS * 32, wsm, c->stream>>>(a, rows, c->big_list, c->big_cnt);
+            mid_kern<<<mg, JM_NT, msm, c->stream>>>(a, rows, c->big_list, c->big_cnt);
             join_kernel<<<std::min(c->n, sms * 3), JT, sm, c->stream>>>(a, rows, c->big_list, c->big_cnt);
-            KCNA_LAUNCHED(c);
+            c->launches += 3;
             return kcna_cuda_check(c, cudaGetLastError(), "join_kernel");
         };
         if (c->bf16_exact)
