@@ -594,52 +594,37 @@ struct MergeArgs {
     uint32_t n_nodes;
 };
 
-// Warp-per-node merge, survivors first.  Every candidate is looked up in the
-// node's sorted pool by binary search (shared memory): a candidate equal to a
-// pool entry, or one that would land at rank >= limit, is dropped.  In a
-// converging NN-descent almost every candidate is such a repeat, so only the
-// few survivors are sorted, deduplicated and merged, and only the pool entries
-// they displace are written.  A node with more than SURV survivors is
-// queued for the block merge (merge_kernel).  Same result as merging all
-// candidates.  Persistent: each warp takes nodes grid-stride, so a block
-// meets its barrier once at the end instead of waiting for its slowest node.
-// SURV is 512, or 1024 while the previous merge queued more than n/32 nodes
-// (the first iterations, when the pools are filling): twice the shared memory
-// per warp and fewer warps per SM, but fewer nodes left to the block merge;
-// refinement merges, with few survivors per node, take 128.
-// With CREDIT (NN-descent merges) every survivor also keeps the index of its
-// candidate slot (16 bits, CB <= 8192) and moves with its key through the
-// sort; before the survivors are deduplicated, each distinct survivor placed
-// at rank < K loads the joiners of its copies (beside their keys) and
-// credits the lowest.  Three blocks of eight warps still share an SM; with
-// 1024 survivor slots a block has seven warps so that two blocks share one.
-constexpr int MW_WARPS = 8;
-__host__ __device__ constexpr int merge_warps(int surv, bool credit) { return surv == 1024 && credit ? 7 : MW_WARPS; }
-__host__ __device__ constexpr size_t merge_warp_bytes(uint32_t cap, int surv, bool credit) {
-    return ((size_t)cap * 8 + (size_t)surv * 8 + 16 + (credit ? (size_t)surv * 2 : 0) + 15) & ~(size_t)15;
+// Merge of a refinement round (no credit, few survivors): warp per node,
+// survivors first.  Every candidate is looked up in the node's sorted pool by
+// binary search (shared memory): a candidate equal to a pool entry, or one that
+// would land at rank >= limit, is dropped.  Only the few survivors are sorted,
+// deduplicated and merged, and only the pool entries they displace are written.
+// A node with more than MW_SURV survivors is queued for the block merge
+// (merge_kernel).  Same result as merging all candidates.  Persistent: each
+// warp takes nodes grid-stride, so a block meets its barrier once at the end
+// instead of waiting for its slowest node.
+constexpr int MW_WARPS = 8, MW_SURV = 128; // five blocks share an SM
+__host__ __device__ constexpr size_t merge_warp_bytes(uint32_t cap) {
+    return ((size_t)cap * 8 + (size_t)MW_SURV * 8 + 16 + 15) & ~(size_t)15;
 }
 
-template <int SURV, bool CREDIT>
 __global__ void __launch_bounds__(MW_WARPS * 32) merge_warp_kernel(MergeArgs a, uint32_t N, uint32_t *big_list,
                                                                   uint32_t *big_cnt) {
     extern __shared__ __align__(16) unsigned char smem[];
     const int w = threadIdx.x >> 5, lane = kcna_lane();
-    const size_t per_warp = merge_warp_bytes(a.cap, SURV, CREDIT);
+    const size_t per_warp = merge_warp_bytes(a.cap);
     unsigned char *base = smem + w * per_warp;
     uint64_t *s_pool = reinterpret_cast<uint64_t *>(base);
     uint64_t *s_sv = s_pool + a.cap;         // survivors (keys without flags)
-    uint64_t *s_last = s_sv + SURV;          // key landing at rank limit-1
-    uint16_t *s_j = reinterpret_cast<uint16_t *>(s_last + 2); // CREDIT: each survivor's candidate slot
+    uint64_t *s_last = s_sv + MW_SURV;       // key landing at rank limit-1
     __shared__ unsigned long long s_stat[4]; // flagged, inserted, candidates, entries
     if (threadIdx.x < 4) s_stat[threadIdx.x] = 0;
     __syncthreads();
-    constexpr int NW = merge_warps(SURV, CREDIT);
-    for (uint32_t node = blockIdx.x * NW + w; node < N; node += gridDim.x * NW) {
+    for (uint32_t node = blockIdx.x * MW_WARPS + w; node < N; node += gridDim.x * MW_WARPS) {
         const uint32_t raw = a.cand_cnt[node];
         // a refinement round leaves most pools without candidates: their pool,
-        // count and radius stand (an NN-descent merge still counts every
-        // pool's flagged entries for its delta, so it visits them all)
-        if (!CREDIT && raw == 0) continue;
+        // count and radius stand
+        if (raw == 0) continue;
         const uint32_t nc = min(raw, a.CB);
         const uint32_t np = min(a.pool_cnt[node], a.limit);
         uint64_t *gp = a.pool + (uint64_t)node * a.cap;
@@ -677,57 +662,17 @@ __global__ void __launch_bounds__(MW_WARPS * 32) merge_warp_kernel(MergeArgs a, 
                 }
                 const unsigned m = __ballot_sync(KCNA_FULL, surv);
                 const uint32_t pos = ns + __popc(m & kcna_lanemask_lt());
-                if (surv && pos < (uint32_t)SURV) {
-                    s_sv[pos] = k;
-                    if (CREDIT) s_j[pos] = (uint16_t)j;
-                }
+                if (surv && pos < (uint32_t)MW_SURV) s_sv[pos] = k;
                 ns += __popc(m);
             }
         }
-        if (ns > (uint32_t)SURV) {
+        if (ns > (uint32_t)MW_SURV) {
             if (lane == 0) big_list[atomicAdd(big_cnt, 1u)] = node;
         } else {
             uint32_t nu = 0; // distinct survivors
             if (ns > 0) {
                 __syncwarp();
-                if (CREDIT) {
-                    kcna_warp_sort_n<true>(s_sv, s_j, (int)ns);
-                    // copies of one key are adjacent: each distinct survivor whose
-                    // rank (distinct index + position in the pool) is below K
-                    // credits the lowest joiner among its copies.  Four batches of
-                    // 32 at a time: their first joiners are loaded together, so the
-                    // L2 round trips overlap.
-                    uint32_t q0 = 0;
-                    for (uint32_t b0 = 0; b0 < ns; b0 += 128) {
-                        uint64_t kv[4];
-                        uint32_t bv[4];
-                        bool cr[4];
-#pragma unroll
-                        for (int u = 0; u < 4; ++u) {
-                            const uint32_t j = b0 + 32 * u + lane;
-                            const uint64_t k = j < ns ? s_sv[j] : KCNA_EMPTY_KEY;
-                            const uint64_t prev = j > 0 && j < ns ? s_sv[j - 1] : KCNA_EMPTY_KEY;
-                            const bool start = j < ns && (j == 0 || (prev >> 2) != (k >> 2));
-                            const unsigned m = __ballot_sync(KCNA_FULL, start);
-                            const uint32_t q = q0 + __popc(m & kcna_lanemask_lt());
-                            q0 += __popc(m);
-                            cr[u] = start && q + (uint32_t)kcna_lower_bound(s_pool, (int)np, k) < a.K;
-                            kv[u] = k;
-                            bv[u] = cr[u] ? (uint32_t)gc[2 * s_j[j] + 1] : KCNA_NONE;
-                        }
-#pragma unroll
-                        for (int u = 0; u < 4; ++u) {
-                            if (!cr[u]) continue;
-                            uint32_t best = bv[u];
-                            for (uint32_t x = b0 + 32 * u + lane + 1; x < ns && (s_sv[x] >> 2) == (kv[u] >> 2); ++x)
-                                best = min(best, (uint32_t)gc[2 * s_j[x] + 1]);
-                            if (best < a.n_nodes) a.found[best] = 1;
-                        }
-                    }
-                    __syncwarp();
-                } else {
-                    kcna_warp_sort_n<false>(s_sv, nullptr, (int)ns);
-                }
+                kcna_warp_sort_n(s_sv, (int)ns);
                 // drop repeats among survivors (same distance and id are adjacent);
                 // compaction moves entries down, so the previous key comes from
                 // registers, not from the array being rewritten
@@ -834,7 +779,232 @@ __device__ uint32_t block_exclusive_scan(uint32_t *data, int n, uint32_t *s_warp
     return data[n];
 }
 
-// Block merge of nodes with many candidates (queued by merge_warp_kernel).
+// NN-descent's merge: a block of four warps per node, survivors first.  As in
+// merge_warp_kernel every candidate is looked up in the node's sorted pool; in
+// a converging NN-descent most are repeats.  The survivors go into a small hash
+// table (open addressing on the id; one id has one distance, so equal keys are
+// the same candidate emitted by several joiners), so that only distinct ones
+// are merged; beside each stands the lowest joiner that emitted it (the slot's
+// second word, fetched with the key), which is credited when the survivor
+// lands at rank < K.
+// Where the survivors land needs no sort: the search says between which pool
+// entries each falls (its bucket), so bucket counts and their prefix sums give
+// every pool entry its shift and every survivor its rank but for the order
+// inside a bucket, which is counted (one or two entries; some fifty while the
+// pools hold a dozen).
+// What bounds it is the latency of dependent shared-memory steps: a warp per
+// node issued every tenth cycle with three warps a scheduler, and a node's
+// arrays (22 KB) allow no more.  Four warps share them here, nine blocks an SM
+// (their 54 registers a thread allow no more either).  The pool lies as two arrays: the search reads the 4-byte distances
+// only, and equal distances are told apart by the id once at the end.
+// 400,003 rows, the four merges of a learned build: 58 ms with a warp per node
+// and a sort of all survivors with their repeats, 26 ms now (9 nodes of each
+// SM in flight; the table alone, with a warp per node, gave 50).
+// MS_H: table slots (a prime, for the double hashing).  A node with more than
+// MS_CAP distinct survivors is queued for the block merge; the count is read
+// before each warp's batch of 32, and the four warps' batches fit beside it.
+constexpr int MS_NT = 128, MS_H = 1021, MS_CAP = MS_H - MS_NT - 1;
+__host__ __device__ constexpr size_t merge_set_bytes(uint32_t cap) {
+    return (size_t)MS_H * 8 + (size_t)cap * 8 + (size_t)MS_H * 4 + (size_t)(cap + 2) * 4 + (size_t)MS_H * 4;
+}
+
+__global__ void __launch_bounds__(MS_NT, 9) merge_set_kernel(MergeArgs a, uint32_t N, uint32_t *big_list,
+                                                            uint32_t *big_cnt) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    uint64_t *s_sv = reinterpret_cast<uint64_t *>(smem);       // the table of distinct survivors (keys without flags)
+    uint32_t *s_pd = reinterpret_cast<uint32_t *>(s_sv + MS_H);   // the pool: distance bits
+    uint32_t *s_pi = s_pd + a.cap;                             // and id with flags
+    uint32_t *s_joiner = s_pi + a.cap;                         // lowest joiner of a table slot
+    uint32_t *s_off = s_joiner + MS_H;                            // cap + 2: bucket counts, starts, ends
+    uint16_t *s_slot = reinterpret_cast<uint16_t *>(s_off + a.cap + 2), *s_b = s_slot + MS_H; // slots in bucket order; bucket of a slot
+    __shared__ uint32_t s_warp[MS_NT / 32], s_flagged, s_placed;
+    __shared__ uint64_t s_last; // key landing at rank limit-1
+    __shared__ volatile uint32_t s_nu;
+    const int tid = threadIdx.x, lane = tid & 31;
+    unsigned long long t_flagged = 0, t_placed = 0, t_cand = 0, t_entries = 0; // thread 0
+    auto clear_table = [&]() {
+        for (int i = tid; i < MS_H; i += MS_NT) {
+            s_sv[i] = KCNA_EMPTY_KEY;
+            s_joiner[i] = KCNA_NONE;
+        }
+        for (uint32_t i = tid; i < a.cap + 2; i += MS_NT) s_off[i] = 0;
+    };
+    clear_table();
+    uint32_t raw_n = blockIdx.x < N ? a.cand_cnt[blockIdx.x] : 0u; // of the next node, loaded a node ahead
+    uint32_t np_n = blockIdx.x < N ? a.pool_cnt[blockIdx.x] : 0u;
+    for (uint32_t node = blockIdx.x; node < N; node += gridDim.x) {
+        const uint32_t raw = raw_n, np = min(np_n, a.limit);
+        if (node + gridDim.x < N) {
+            raw_n = a.cand_cnt[node + gridDim.x];
+            np_n = a.pool_cnt[node + gridDim.x];
+        }
+        const uint32_t nc = min(raw, a.CB);
+        uint64_t *gp = a.pool + (uint64_t)node * a.cap;
+        const ulonglong2 *gc = reinterpret_cast<const ulonglong2 *>(a.cand) + (uint64_t)node * a.CB; // key, joiner
+        // candidates in groups of 256 (two per thread), the next group's loads in
+        // flight while this group is searched, the two searches side by side
+        constexpr int CG = 2;
+        ulonglong2 nxt[CG];
+        auto fetch = [&](int u, uint32_t j) { nxt[u] = j < nc ? gc[j] : make_ulonglong2(KCNA_EMPTY_KEY, KCNA_NONE); };
+#pragma unroll
+        for (int u = 0; u < CG; ++u) fetch(u, MS_NT * u + tid);
+#pragma unroll 4
+        for (uint32_t i = tid; i < np; i += MS_NT) {
+            const uint64_t k = gp[i];
+            s_pd[i] = (uint32_t)(k >> 32);
+            s_pi[i] = (uint32_t)k;
+        }
+        if (tid == 0) {
+            s_nu = 0;
+            s_flagged = s_placed = 0;
+            s_last = KCNA_EMPTY_KEY;
+        }
+        __syncthreads();
+        const int top = np ? 1 << (31 - __clz(np)) : 0, last = max((int)np - 1, 0); // largest step of the search
+        for (uint32_t b0 = 0; b0 < nc; b0 += MS_NT * CG) {
+            uint32_t d[CG], id[CG], joiner[CG];
+            int b[CG];
+            bool surv[CG];
+#pragma unroll
+            for (int u = 0; u < CG; ++u) {
+                d[u] = (uint32_t)(nxt[u].x >> 32);
+                id[u] = kcna_key_id(nxt[u].x);
+                joiner[u] = (uint32_t)nxt[u].y;
+                // a candidate, not the padding or a dropped one
+                surv[u] = kcna_key_noflags(nxt[u].x) != KCNA_EMPTY_KEY_NOFLAGS;
+                b[u] = 0;
+                fetch(u, b0 + MS_NT * CG + MS_NT * u + tid);
+            }
+            // entries nearer than each candidate
+            for (int step = top; step; step >>= 1) {
+#pragma unroll
+                for (int u = 0; u < CG; ++u) {
+                    const int t = b[u] + step - 1;
+                    const uint32_t v = s_pd[min(t, last)];
+                    b[u] += (t <= last) & (v < d[u]) ? step : 0;
+                }
+            }
+            // survivors, and what their table slot holds so far
+            uint32_t h[CG];
+            uint64_t seen[CG];
+#pragma unroll
+            for (int u = 0; u < CG; ++u) {
+                h[u] = __umulhi(id[u] * 0x9E3779B1u, (uint32_t)MS_H);
+                seen[u] = s_sv[h[u]];
+                // entries at the candidate's distance: by id; its own twin drops it
+                while (b[u] < (int)np && s_pd[b[u]] == d[u]) {
+                    const uint32_t e = s_pi[b[u]] >> 2;
+                    if (e >= id[u]) {
+                        if (e == id[u]) surv[u] = false;
+                        break;
+                    }
+                    ++b[u];
+                }
+                if ((uint32_t)b[u] >= a.limit) surv[u] = false;
+            }
+#pragma unroll
+            for (int u = 0; u < CG; ++u) {
+                bool fresh = false;
+                if (s_nu > (uint32_t)MS_CAP) surv[u] = false; // table full: the block merge takes the node
+                if (surv[u]) {
+                    // double hashing: in a table three quarters full, runs of taken slots
+                    // would keep a warp's unluckiest lane probing for tens of steps
+                    const uint64_t k = ((uint64_t)d[u] << 32) | ((uint64_t)id[u] << 2);
+                    uint32_t x = h[u];
+                    const uint32_t step = 1u + __umulhi(id[u] * 0x85EBCA6Bu, (uint32_t)(MS_H - 1));
+                    for (int probe = 0; probe < MS_H && seen[u] != k; ++probe) { // a slot is free, or holds k
+                        if (seen[u] == KCNA_EMPTY_KEY) {
+                            seen[u] = atomicCAS(reinterpret_cast<unsigned long long *>(s_sv + x), KCNA_EMPTY_KEY, k);
+                            fresh = seen[u] == KCNA_EMPTY_KEY;
+                            if (fresh || seen[u] == k) break;
+                        }
+                        x += step;
+                        x -= x >= (uint32_t)MS_H ? (uint32_t)MS_H : 0u;
+                        seen[u] = s_sv[x];
+                    }
+                    if (joiner[u] < s_joiner[x]) atomicMin(s_joiner + x, joiner[u]);
+                    if (fresh) {
+                        s_b[x] = (uint16_t)b[u];
+                        atomicAdd(s_off + b[u], 1u);
+                    }
+                }
+                const unsigned m = __ballot_sync(KCNA_FULL, fresh);
+                if (m && lane == 0) atomicAdd(const_cast<uint32_t *>(&s_nu), (uint32_t)__popc(m));
+            }
+        }
+        __syncthreads();
+        const uint32_t nu = s_nu;
+        if (nu > (uint32_t)MS_CAP) {
+            if (tid == 0) big_list[atomicAdd(big_cnt, 1u)] = node;
+        } else {
+            const uint32_t newcnt = min(a.limit, np + nu);
+            uint32_t flagged = 0, placed = 0;
+            if (nu > 0) { // survivors in bucket order; s_off[b] ends as the end of bucket b
+                block_exclusive_scan(s_off, (int)np + 1, s_warp);
+                for (int i = tid; i < MS_H; i += MS_NT)
+                    if (s_sv[i] != KCNA_EMPTY_KEY) s_slot[atomicAdd(s_off + s_b[i], 1u)] = (uint16_t)i;
+                __syncthreads();
+            }
+            // pool entries: shifted by the survivors below them
+#pragma unroll 4
+            for (uint32_t i = tid; i < np; i += MS_NT) {
+                const uint64_t k = ((uint64_t)s_pd[i] << 32) | s_pi[i];
+                const uint32_t sh = s_off[i], r = i + sh; // all zero without survivors
+                if (r < newcnt) {
+                    if (sh) gp[r] = k;
+                    if (r < a.K && (k & KCNA_FLAG_NEW)) ++flagged;
+                    if (r + 1 == a.limit) s_last = k;
+                }
+            }
+            // survivors at their rank
+            for (uint32_t j = tid; j < nu; j += MS_NT) {
+                const uint32_t slot = s_slot[j], b = s_b[slot], lo = b ? s_off[b - 1] : 0u, hi = s_off[b];
+                const uint64_t k = s_sv[slot];
+                uint32_t r = b + lo;
+                if (hi - lo > 1) {
+#pragma unroll 4
+                    for (uint32_t x = lo; x < hi; ++x) r += s_sv[s_slot[x]] < k ? 1u : 0u;
+                }
+                if (r >= newcnt) continue;
+                gp[r] = k | KCNA_FLAG_NEW | KCNA_FLAG_ISNEW;
+                ++placed;
+                if (r < a.K) {
+                    ++flagged;
+                    const uint32_t best = s_joiner[slot];
+                    if (best < a.n_nodes) a.found[best] = 1;
+                }
+                if (r + 1 == a.limit) s_last = k;
+            }
+            flagged = kcna_warp_sum(flagged);
+            placed = kcna_warp_sum(placed);
+            if (lane == 0) {
+                if (flagged) atomicAdd(&s_flagged, flagged);
+                if (placed) atomicAdd(&s_placed, placed);
+            }
+            __syncthreads();
+            if (tid == 0) {
+                t_flagged += s_flagged;
+                t_placed += s_placed;
+                t_cand += nc;
+                t_entries += newcnt;
+                if (raw > a.CB) atomicAdd(a.counters + 2, (unsigned long long)(raw - a.CB));
+                a.pool_cnt[node] = newcnt;
+                a.cand_cnt[node] = 0;
+                a.radius[node] = newcnt >= a.limit ? kcna_key_dist(s_last) : __uint_as_float(0x7F800000u);
+            }
+        }
+        __syncthreads(); // the next node reuses the arrays
+        if (nu > 0) clear_table();
+    }
+    if (tid == 0) {
+        if (t_flagged) atomicAdd(a.counters + 1, t_flagged);
+        if (t_placed) atomicAdd(a.counters + 3, t_placed);
+        if (t_cand) atomicAdd(a.counters + 7, t_cand);
+        if (t_entries) atomicAdd(a.counters + 9, t_entries);
+    }
+}
+
+// Block merge of nodes with many survivors (queued by the two kernels above).
 // Each candidate is placed by binary search into the gap of the sorted pool
 // it falls in (its bucket: the number of pool entries below it); candidates
 // equal to a pool entry or with bucket >= limit are dropped.  A counting sort
@@ -1468,48 +1638,32 @@ kcna_status kcna_merge(kcna_ctx *c, uint32_t limit, uint32_t K, uint64_t *overfl
     KCNA_TRY(kcna_cuda_check(c, cudaFuncSetAttribute(merge_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                      (int)std::max<size_t>(sm, 48 * 1024)),
                              "merge smem attr"));
-    const char *wd = getenv("KCNA_MERGE_WIDE_DIV"); // tuning override of the threshold below
-    const uint32_t wide_div = wd ? std::max(1, atoi(wd)) : 32; // 64 and 16 measured slower at C2 1M
-    const bool wide = c->merge_big_last > c->n / wide_div; // many nodes overflowed the survivor buffer last time
-    const char *sv = getenv("KCNA_MERGE_SURV");   // tuning override: 128, 512 or 1024
-    // refinement merges (no credit) meet few survivors per node: 128 slots per
-    // warp, so that five blocks instead of three share an SM
-    const int surv = sv ? (atoi(sv) >= 1024 ? 1024 : atoi(sv) >= 512 ? 512 : 128)
-                        : wide ? 1024 : credit_found ? 512 : 128;
-    const int nw = merge_warps(surv, credit_found);
-    const size_t smw = merge_warp_bytes(c->cap, surv, credit_found) * nw;
-    auto launch_warp = [&](auto kern) -> kcna_status {
+    auto launch = [&](auto kern, int threads, uint32_t per_block, size_t smem) -> kcna_status {
         KCNA_TRY(kcna_cuda_check(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                         (int)std::max<size_t>(smw, 48 * 1024)),
+                                                         (int)std::max<size_t>(smem, 48 * 1024)),
                                  "merge smem attr"));
-        int mw_per_sm = 0;
-        KCNA_TRY(kcna_cuda_check(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&mw_per_sm, kern, nw * 32, smw),
+        int per_sm = 0;
+        KCNA_TRY(kcna_cuda_check(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem),
                                  "merge occupancy"));
-        const uint32_t mw_grid = (uint32_t)std::min<uint64_t>(
-            kcna_div_up(c->n, nw), (uint64_t)std::max(c->num_sms, 1) * std::max(mw_per_sm, 1));
+        const uint32_t grid = std::min(kcna_div_up(c->n, per_block),
+                                       (uint32_t)std::max(c->num_sms, 1) * (uint32_t)std::max(per_sm, 1));
         KCNA_TRY(kcna_cuda_check(c, cudaMemsetAsync(c->counters, 0, 10 * 8, c->stream), "memset"));
         KCNA_TRY(kcna_cuda_check(c, cudaMemsetAsync(c->big_cnt, 0, 4, c->stream), "memset"));
         KCNA_TRY(kcna_phase_begin(c));
-        kern<<<mw_grid, nw * 32, smw, c->stream>>>(a, c->n, c->big_list, c->big_cnt);
+        kern<<<grid, threads, smem, c->stream>>>(a, c->n, c->big_list, c->big_cnt);
         return KCNA_OK;
     };
-    // the template must match the shared memory sized above
-    if (credit_found)
-        KCNA_TRY(surv == 1024 ? launch_warp(merge_warp_kernel<1024, true>) : launch_warp(merge_warp_kernel<512, true>));
+    if (!credit_found)
+        KCNA_TRY(launch(merge_warp_kernel, MW_WARPS * 32, MW_WARPS, merge_warp_bytes(c->cap) * MW_WARPS));
     else
-        KCNA_TRY(surv == 1024  ? launch_warp(merge_warp_kernel<1024, false>)
-                 : surv == 512 ? launch_warp(merge_warp_kernel<512, false>)
-                               : launch_warp(merge_warp_kernel<128, false>));
+        KCNA_TRY(launch(merge_set_kernel, MS_NT, 1, merge_set_bytes(c->cap)));
     merge_kernel<<<std::max(1, c->num_sms) * 4, MT, sm, c->stream>>>(a, c->big_list, c->big_cnt);
     c->launches += 2;
     KCNA_TRY(kcna_cuda_check(c, cudaGetLastError(), "merge_kernel"));
     KCNA_TRY(kcna_phase_end(c, KCNA_PHASE_MERGE));
     unsigned long long h[10] = {};
-    uint32_t hb = 0;
     KCNA_TRY(kcna_cuda_check(c, cudaMemcpyAsync(h, c->counters, 10 * 8, cudaMemcpyDeviceToHost, c->stream), "d2h"));
-    KCNA_TRY(kcna_cuda_check(c, cudaMemcpyAsync(&hb, c->big_cnt, 4, cudaMemcpyDeviceToHost, c->stream), "d2h"));
     KCNA_TRY(kcna_cuda_check(c, cudaStreamSynchronize(c->stream), "merge sync"));
-    c->merge_big_last = hb;
     c->cand_merged += h[7];
     c->pool_entries_merged += h[9];
     if (merged) *merged = h[7];
@@ -1643,7 +1797,6 @@ kcna_status kcna_nndescent_run(kcna_ctx *c, const kcna_params *pin, kcna_stats *
     const uint32_t maxl = std::max(std::max(P.L, P.K), std::max(P.search_L, P.search_K));
     if (maxl > 1024) return kcna_fail(c, KCNA_E_ARG, "max(L, K, search_L, search_K) must be <= 1024");
     st->maxl = maxl;
-    c->merge_big_last = c->n; // the first merges fill the pools: wide survivor buffers
     KCNA_TRY(kcna_nnd_alloc(c, &P, maxl));
     KCNA_TRY(kcna_controls_setup(c, &P, maxl));
     // join iterations count from 1 when the first lists come from an update step

@@ -45,41 +45,13 @@ __device__ __forceinline__ void kcna_warp_bitonic(uint64_t *s, int n) {
     __syncwarp();
 }
 
-// Ascending bitonic sort of n (a power of two) keys in shared memory by one
-// warp, each carrying a 16-bit value that moves with it (values of equal keys
-// end in no particular order).
-__device__ __forceinline__ void kcna_warp_bitonic_kv16(uint64_t *s, uint16_t *v, int n) {
-    const int lane = kcna_lane();
-    for (int size = 2; size <= n; size <<= 1) {
-        for (int stride = size >> 1; stride > 0; stride >>= 1) {
-            __syncwarp();
-            for (int t = lane; t < (n >> 1); t += 32) {
-                int i = ((t & ~(stride - 1)) << 1) | (t & (stride - 1));
-                int j = i + stride;
-                bool asc = (i & size) == 0;
-                uint64_t a = s[i], b = s[j];
-                if ((a > b) == asc) {
-                    s[i] = b;
-                    s[j] = a;
-                    const uint16_t va = v[i];
-                    v[i] = v[j];
-                    v[j] = va;
-                }
-            }
-        }
-    }
-    __syncwarp();
-}
-
 // Ascending sort of s[0, n), any n >= 1, by one warp in shared memory: the
 // bitonic network in its flip form (every comparator puts the smaller key at
 // the lower index), padded to the next power of two with virtual +infinite
 // keys.  A comparator that touches a virtual key leaves both in place, so
 // only the comparators inside [0, n) run and nothing beyond n is read or
-// written.  With KV every key carries a 16-bit value from v (values of equal
-// keys end in no particular order).
-template <bool KV>
-__device__ __forceinline__ void kcna_warp_sort_n(uint64_t *s, uint16_t *v, int n) {
+// written.
+__device__ __forceinline__ void kcna_warp_sort_n(uint64_t *s, int n) {
     const int lane = kcna_lane();
     int p2 = 1;
     while (p2 < n) p2 <<= 1;
@@ -99,11 +71,6 @@ __device__ __forceinline__ void kcna_warp_sort_n(uint64_t *s, uint16_t *v, int n
                 if (b < a) {
                     s[i] = b;
                     s[j] = a;
-                    if (KV) {
-                        const uint16_t va = v[i];
-                        v[i] = v[j];
-                        v[j] = va;
-                    }
                 }
             }
         }
