@@ -182,6 +182,9 @@ void kcna_log(kcna_ctx *c, const kcna_params *p, const char *fmt, ...);
 // [0, n) of X; q_self (device, may be null) gives a row id to exclude per query.
 kcna_status kcna_knn_device(kcna_ctx *c, const float *dQ, uint32_t m, const uint32_t *q_self, uint32_t k,
                             uint32_t *d_out_ids, float *d_out_d);
+// kcna_knn_tc.cu: for each query, the ids of the rows that may lie within its bound (d <= 128)
+kcna_status kcna_knn_filter(kcna_ctx *c, const float *dQ, uint32_t m, const uint32_t *thresh, uint32_t *cand,
+                            uint32_t *cnt, uint32_t cap);
 // gathers rows ids[0..m) of X into dst (m x ld)
 kcna_status kcna_gather_rows(kcna_ctx *c, const uint32_t *d_ids, uint32_t m, float *dst);
 

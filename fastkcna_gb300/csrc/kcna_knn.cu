@@ -4,7 +4,9 @@
 // :363-387) and SearchOracle::search (:332-361): for each query, the k rows
 // with the smallest squared L2 distance, ties broken by the lower id (the
 // reference scans ids in order and inserts equal distances after existing
-// ones, src/kgraph.cpp:227-260).  Two kernels:
+// ones, src/kgraph.cpp:227-260).
+//
+// Small bases: two kernels,
 //   1. a tiled distance kernel (32 queries x 128 rows per block, 4x4 register
 //      micro-tiles, dimensions staged through shared memory in chunks of 32)
 //      computing the canonical FMA-chain distance of every pair;
@@ -12,7 +14,23 @@
 //      the distance bits find the k-th smallest distance T, then every row with
 //      distance < T plus the lowest ids among rows with distance == T are kept
 //      and sorted by (distance, id).
+// Larger ones: writing every distance and reading it four times costs more
+// than computing it (7.3 of 17.7 ms for 1,000 queries against 1,000,000 x 128
+// rows), and the computation itself can be spared for all but a few thousand
+// rows per query:
+//   1. distances to every (n / s)-th row; the max(k, 32)-th smallest of them is
+//      a bound T on the k-th smallest of all;
+//   2. the rows that may lie within T: screened on tensor cores where the work
+//      is large and d <= 128 (kcna_knn_tc.cu), else by the tiled kernel, which
+//      then keeps a pair only if its distance is at most T;
+//   3. per query, canonical distances of the rows handed on (where 2 screened)
+//      and the selection among them.
+// s is chosen so that about 4,096 rows remain; a query whose list of 8,192
+// overflows, or comes up short (NaN), is done again the first way.
+// The size above: 2.05 ms a call (0.26 sample, 0.08 bounds, 1.07 screen, 0.58
+// selection).
 #include <algorithm>
+#include <vector>
 
 #include "kcna_internal.h"
 #include "kcna_sort.cuh"
@@ -21,10 +39,20 @@ namespace {
 
 constexpr int TQ = 32, TB = 128, KC = 32, KCP = KC + 4;
 
+// FILTER: instead of writing every distance, append (distance, id) to the
+// query's list when the distance is at most thresh[q].
+// Base row b is row b * stride of X.
+struct DistOut {
+    float *D;
+    uint64_t ldD;
+    const uint32_t *thresh;
+    uint64_t *cand;
+    uint32_t *cnt, cap;
+};
+template <bool FILTER>
 __global__ void __launch_bounds__(256) dist_tile_kernel(const float *__restrict__ Q, uint32_t m,
-                                                        const float *__restrict__ X, uint32_t n, int ld,
-                                                        const uint32_t *__restrict__ q_self, float *__restrict__ D,
-                                                        uint64_t ldD) {
+                                                        const float *__restrict__ X, uint32_t n, uint32_t stride,
+                                                        int ld, const uint32_t *__restrict__ q_self, DistOut o) {
     __shared__ __align__(16) float Qs[TQ][KCP];
     __shared__ __align__(16) float Xs[TB][KCP];
     const int tid = threadIdx.x, tx = tid & 31, ty = tid >> 5;
@@ -48,7 +76,7 @@ __global__ void __launch_bounds__(256) dist_tile_kernel(const float *__restrict_
             int idx = tid + s * 256;
             int r = idx >> 3, c = (idx & 7) * 4;
             float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (b0 + r < n && k0 + c < ld) v = __ldg(reinterpret_cast<const float4 *>(X + (b0 + r) * ld + k0 + c));
+            if (b0 + r < n && k0 + c < ld) v = __ldg(reinterpret_cast<const float4 *>(X + (b0 + r) * stride * ld + k0 + c));
             *reinterpret_cast<float4 *>(&Xs[r][c]) = v;
         }
         __syncthreads();
@@ -75,7 +103,13 @@ __global__ void __launch_bounds__(256) dist_tile_kernel(const float *__restrict_
         for (int j = 0; j < 4; ++j) {
             uint64_t b = b0 + tx + 32 * j;
             if (b >= n) continue;
-            D[(uint64_t)q * ldD + b] = (b == self) ? __uint_as_float(0x7F800000u) : acc[i][j];
+            const bool own = b * stride == self;
+            if (!FILTER) {
+                o.D[(uint64_t)q * o.ldD + b] = own ? __uint_as_float(0x7F800000u) : acc[i][j];
+            } else if (!own && __float_as_uint(acc[i][j]) <= o.thresh[q]) {
+                const uint32_t p = atomicAdd(o.cnt + q, 1u);
+                if (p < o.cap) o.cand[(uint64_t)q * o.cap + p] = ((uint64_t)__float_as_uint(acc[i][j]) << 32) | (b * stride);
+            }
         }
     }
 }
@@ -85,30 +119,39 @@ constexpr int SEL_BINS = 4096;
 constexpr int SEL_MAXK = 1024;
 constexpr int SEL_TIES = 1024;
 
-// Finds the bin holding the want-th (0-based) element; returns bin and the
-// number of elements in lower bins.  hist has nb bins (multiple of SEL_T).
-__device__ void find_bin(const uint32_t *hist, int nb, uint32_t want, uint32_t *s_scan, int *out_bin,
-                         uint32_t *out_before) {
-    const int per = nb / SEL_T;
+constexpr uint32_t KNN_CAP = 8192;       // rows handed on per query at most
+constexpr uint32_t SEL_CACHE = 40960;    // a distance row up to this length is read once, into shared memory
+
+struct SelectShared {
+    uint32_t hist[SEL_BINS];
+    uint32_t scan[SEL_T / 32];
+    int bin;
+    uint32_t before, nout, ntie;
+};
+
+// Finds the bin holding the want-th (0-based) element, S.bin, and the number
+// of elements in lower bins, S.before; nb bins (a multiple of SEL_T).
+__device__ void find_bin(SelectShared &S, int nb, uint32_t want) {
+    const int per = nb / SEL_T, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint32_t local = 0;
-    for (int i = 0; i < per; ++i) local += hist[threadIdx.x * per + i];
-    s_scan[threadIdx.x] = local;
-    __syncthreads();
-    // inclusive Hillis-Steele scan over SEL_T partial sums
-    for (int off = 1; off < SEL_T; off <<= 1) {
-        uint32_t v = threadIdx.x >= off ? s_scan[threadIdx.x - off] : 0;
-        __syncthreads();
-        s_scan[threadIdx.x] += v;
-        __syncthreads();
+    for (int i = 0; i < per; ++i) local += S.hist[threadIdx.x * per + i];
+    uint32_t incl = local;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(KCNA_FULL, incl, o);
+        if (lane >= o) incl += v;
     }
-    uint32_t incl = s_scan[threadIdx.x], excl = incl - local;
+    if (lane == 31) S.scan[warp] = incl;
+    __syncthreads();
+    for (int w = 0; w < warp; ++w) incl += S.scan[w];
+    const uint32_t excl = incl - local;
     if (want >= excl && want < incl) {
         uint32_t run = excl;
         for (int i = 0; i < per; ++i) {
-            uint32_t h = hist[threadIdx.x * per + i];
+            const uint32_t h = S.hist[threadIdx.x * per + i];
             if (want < run + h) {
-                *out_bin = threadIdx.x * per + i;
-                *out_before = run;
+                S.bin = threadIdx.x * per + i;
+                S.before = run;
                 break;
             }
             run += h;
@@ -117,53 +160,54 @@ __device__ void find_bin(const uint32_t *hist, int nb, uint32_t want, uint32_t *
     __syncthreads();
 }
 
-__global__ void __launch_bounds__(SEL_T) select_kernel(const float *__restrict__ D, uint64_t ldD, uint32_t n,
-                                                       uint32_t k, uint32_t q_base, uint32_t *__restrict__ out_ids,
-                                                       float *__restrict__ out_d, int *err) {
-    __shared__ uint32_t hist[SEL_BINS];
-    __shared__ uint32_t s_scan[SEL_T];
-    __shared__ uint64_t s_out[SEL_MAXK];
-    __shared__ uint64_t s_tie[SEL_TIES];
-    __shared__ int s_bin;
-    __shared__ uint32_t s_before, s_nout, s_ntie;
-    const uint32_t *row = reinterpret_cast<const uint32_t *>(D + (uint64_t)blockIdx.x * ldD);
-    uint32_t want = k - 1, prefix = 0;
-    // three passes: bits 31..20, 19..8, 7..0
+// The want-th (0-based) smallest of the n words at(j), by the whole block:
+// bits 31..20, 19..8, 7..0.
+template <class At>
+__device__ uint32_t kth_word(SelectShared &S, uint32_t n, uint32_t want, At at) {
+    uint32_t prefix = 0;
     const int shifts[3] = {20, 8, 0};
     const int widths[3] = {12, 12, 8};
     for (int pass = 0; pass < 3; ++pass) {
         const int sh = shifts[pass], nb = 1 << widths[pass];
-        for (int i = threadIdx.x; i < SEL_BINS; i += SEL_T) hist[i] = 0;
+        for (int i = threadIdx.x; i < max(nb, SEL_T); i += SEL_T) S.hist[i] = 0;
         __syncthreads();
         const int hsh = sh + widths[pass];
         for (uint32_t j = threadIdx.x; j < n; j += SEL_T) {
-            uint32_t v = row[j];
-            if (pass == 0 || (v >> hsh) == prefix) atomicAdd(&hist[(v >> sh) & (nb - 1)], 1u);
+            const uint32_t v = at(j);
+            if (pass == 0 || (v >> hsh) == prefix) atomicAdd(&S.hist[(v >> sh) & (nb - 1)], 1u);
         }
         __syncthreads();
-        find_bin(hist, nb < SEL_T ? SEL_T : nb, want, s_scan, &s_bin, &s_before);
-        prefix = (prefix << widths[pass]) | (uint32_t)s_bin;
-        want -= s_before;
+        find_bin(S, max(nb, SEL_T), want);
+        prefix = (prefix << widths[pass]) | (uint32_t)S.bin;
+        want -= S.before;
         __syncthreads();
     }
-    const uint32_t T = prefix; // k-th smallest distance bits
+    return prefix;
+}
+
+// The k smallest (distance, id) of n entries, dist(j) and id(j), sorted, to
+// out; by the whole block.
+template <class Dist, class Id>
+__device__ void select_k(SelectShared &S, uint64_t *s_out, uint64_t *s_tie, uint32_t n, uint32_t k, Dist dist, Id id,
+                         uint32_t *out_ids, float *out_d, int *err) {
+    const uint32_t T = kth_word(S, n, k - 1, dist); // k-th smallest distance bits
     if (threadIdx.x == 0) {
-        s_nout = 0;
-        s_ntie = 0;
+        S.nout = 0;
+        S.ntie = 0;
     }
     __syncthreads();
     for (uint32_t j = threadIdx.x; j < n; j += SEL_T) {
-        uint32_t v = row[j];
+        const uint32_t v = dist(j);
         if (v < T) {
-            uint32_t p = atomicAdd(&s_nout, 1u);
-            if (p < SEL_MAXK) s_out[p] = ((uint64_t)v << 32) | j;
+            uint32_t p = atomicAdd(&S.nout, 1u);
+            if (p < SEL_MAXK) s_out[p] = ((uint64_t)v << 32) | id(j);
         } else if (v == T) {
-            uint32_t p = atomicAdd(&s_ntie, 1u);
-            if (p < SEL_TIES) s_tie[p] = ((uint64_t)v << 32) | j;
+            uint32_t p = atomicAdd(&S.ntie, 1u);
+            if (p < SEL_TIES) s_tie[p] = ((uint64_t)v << 32) | id(j);
         }
     }
     __syncthreads();
-    uint32_t nless = s_nout, ntie = s_ntie;
+    uint32_t nless = S.nout, ntie = S.ntie;
     if (ntie > SEL_TIES) kcna_set_err(err, KCNA_DERR_TIES);
     if (nless >= k) kcna_set_err(err, KCNA_DERR_BOUNDS);
     ntie = min(ntie, (uint32_t)SEL_TIES);
@@ -176,12 +220,101 @@ __global__ void __launch_bounds__(SEL_T) select_kernel(const float *__restrict__
     int kp = kcna_pow2_ceil_d((int)k);
     for (int i = k + threadIdx.x; i < kp; i += SEL_T) s_out[i] = KCNA_EMPTY_KEY;
     kcna_cta_bitonic(s_out, kp);
-    const uint64_t ob = (uint64_t)(q_base + blockIdx.x) * k;
     for (uint32_t i = threadIdx.x; i < k; i += SEL_T) {
         uint64_t key = s_out[i];
-        out_ids[ob + i] = (uint32_t)key;
-        out_d[ob + i] = __uint_as_float((uint32_t)(key >> 32));
+        out_ids[i] = (uint32_t)key;
+        out_d[i] = __uint_as_float((uint32_t)(key >> 32));
     }
+}
+
+// CACHED: the distance row fits shared memory and is read once.
+template <bool CACHED>
+__global__ void __launch_bounds__(SEL_T) select_kernel(const float *__restrict__ D, uint64_t ldD, uint32_t n,
+                                                       uint32_t k, uint32_t q_base, uint32_t *__restrict__ out_ids,
+                                                       float *__restrict__ out_d, int *err) {
+    extern __shared__ __align__(16) uint32_t s_row[]; // CACHED: n words
+    __shared__ SelectShared S;
+    __shared__ uint64_t s_out[SEL_MAXK], s_tie[SEL_TIES];
+    const uint32_t *row = reinterpret_cast<const uint32_t *>(D + (uint64_t)blockIdx.x * ldD);
+    if (CACHED) {
+#pragma unroll 8
+        for (uint32_t j = threadIdx.x; j < n; j += SEL_T) s_row[j] = row[j];
+        row = s_row;
+        __syncthreads();
+    }
+    const uint64_t ob = (uint64_t)(q_base + blockIdx.x) * k;
+    select_k(S, s_out, s_tie, n, k, [&](uint32_t j) { return row[j]; }, [](uint32_t j) { return j; }, out_ids + ob,
+             out_d + ob, err);
+}
+
+// Bound of each query: the rank-th smallest of its s sampled distances; also
+// clears the query's count.
+template <bool CACHED>
+__global__ void __launch_bounds__(SEL_T) knn_bound_kernel(const float *__restrict__ D, uint32_t s, uint32_t rank,
+                                                          uint32_t *__restrict__ thresh, uint32_t *__restrict__ cnt) {
+    extern __shared__ __align__(16) uint32_t s_row[];
+    __shared__ SelectShared S;
+    const uint32_t *row = reinterpret_cast<const uint32_t *>(D + (uint64_t)blockIdx.x * s);
+    if (CACHED) {
+#pragma unroll 8
+        for (uint32_t j = threadIdx.x; j < s; j += SEL_T) s_row[j] = row[j];
+        row = s_row;
+        __syncthreads();
+    }
+    const uint32_t T = kth_word(S, s, rank - 1, [&](uint32_t j) { return row[j]; });
+    if (threadIdx.x == 0) {
+        thresh[blockIdx.x] = T;
+        cnt[blockIdx.x] = 0;
+    }
+}
+
+// Selection among the rows handed on; SCREENED: they are ids only, and their
+// canonical distances are computed here, a row per thread, sixteen loads in
+// flight.  A query with too many or too few counts in *redo.
+template <bool SCREENED>
+__global__ void __launch_bounds__(SEL_T) knn_final_kernel(const float *__restrict__ Q, const float *__restrict__ X,
+                                                          int ld, const uint32_t *__restrict__ q_self,
+                                                          const uint64_t *__restrict__ cand,
+                                                          const uint32_t *__restrict__ cand_ids,
+                                                          const uint32_t *__restrict__ cnt, uint32_t k, uint32_t q_base,
+                                                          uint32_t *__restrict__ out_ids, float *__restrict__ out_d,
+                                                          uint32_t *redo, int *err) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    uint64_t *s_key = reinterpret_cast<uint64_t *>(smem); // KNN_CAP (distance, id)
+    float4 *s_q = reinterpret_cast<float4 *>(s_key + KNN_CAP); // SCREENED: the query
+    __shared__ SelectShared S;
+    __shared__ uint64_t s_out[SEL_MAXK], s_tie[SEL_TIES];
+    const uint32_t q = blockIdx.x, n = cnt[q];
+    const uint32_t self = q_self ? q_self[q] : KCNA_NONE;
+    if (n > KNN_CAP || n < k) {
+        if (threadIdx.x == 0) atomicAdd(redo, 1u);
+        return;
+    }
+    if (SCREENED) {
+        const int nv = ld >> 2;
+        for (int i = threadIdx.x; i < nv; i += SEL_T) s_q[i] = reinterpret_cast<const float4 *>(Q + (uint64_t)q * ld)[i];
+        __syncthreads();
+        for (uint32_t j = threadIdx.x; j < n; j += SEL_T) {
+            const uint32_t id = cand_ids[(uint64_t)q * KNN_CAP + j];
+            const float4 *x = reinterpret_cast<const float4 *>(X + (uint64_t)id * ld);
+            float acc = 0.f;
+            for (int k0 = 0; k0 < nv; k0 += 16) {
+                float4 v[16];
+#pragma unroll
+                for (int u = 0; u < 16; ++u) v[u] = __ldg(x + min(k0 + u, nv - 1));
+#pragma unroll
+                for (int u = 0; u < 16; ++u)
+                    if (k0 + u < nv) acc = kcna_acc4(acc, s_q[k0 + u], v[u]);
+            }
+            s_key[j] = ((uint64_t)(id == self ? 0x7F800000u : __float_as_uint(acc)) << 32) | id;
+        }
+    } else {
+        for (uint32_t j = threadIdx.x; j < n; j += SEL_T) s_key[j] = cand[(uint64_t)q * KNN_CAP + j];
+    }
+    __syncthreads();
+    const uint64_t ob = (uint64_t)(q_base + q) * k;
+    select_k(S, s_out, s_tie, n, k, [&](uint32_t j) { return (uint32_t)(s_key[j] >> 32); },
+             [&](uint32_t j) { return (uint32_t)s_key[j]; }, out_ids + ob, out_d + ob, err);
 }
 
 __global__ void gather_rows_kernel(const float *__restrict__ X, int ld, const uint32_t *__restrict__ ids, uint32_t m,
@@ -208,10 +341,9 @@ kcna_status kcna_gather_rows(kcna_ctx *c, const uint32_t *d_ids, uint32_t m, flo
     return kcna_cuda_check(c, cudaGetLastError(), "gather_rows");
 }
 
-kcna_status kcna_knn_device(kcna_ctx *c, const float *dQ, uint32_t m, const uint32_t *q_self, uint32_t k,
-                            uint32_t *d_out_ids, float *d_out_d) {
-    if (k == 0 || k > SEL_MAXK || k > c->n) return kcna_fail(c, KCNA_E_ARG, "knn: k must be in [1, min(1024, n)]");
-    if (q_self && k >= c->n) return kcna_fail(c, KCNA_E_ARG, "knn: k must be < n when self is excluded");
+// Every distance written, then selected from.
+static kcna_status knn_all(kcna_ctx *c, const float *dQ, uint32_t m, const uint32_t *q_self, uint32_t k,
+                           uint32_t *d_out_ids, float *d_out_d) {
     // distance rows for a batch of queries; batch bounded to ~1 GiB of scratch
     uint64_t row_bytes = (uint64_t)c->n * sizeof(float);
     uint32_t batch = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(m, (1ull << 30) / row_bytes));
@@ -220,15 +352,116 @@ kcna_status kcna_knn_device(kcna_ctx *c, const float *dQ, uint32_t m, const uint
     void *buf = nullptr;
     KCNA_TRY(kcna_scratch(c, (uint64_t)batch * row_bytes, &buf));
     float *D = (float *)buf;
+    const bool cached = c->n <= SEL_CACHE;
+    if (cached)
+        KCNA_TRY(kcna_cuda_check(c, cudaFuncSetAttribute(select_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                         (int)(SEL_CACHE * 4)),
+                                 "select smem attr"));
     for (uint32_t q0 = 0; q0 < m; q0 += batch) {
         uint32_t mb = std::min(batch, m - q0);
         dim3 grid(kcna_div_up(c->n, TB), kcna_div_up(mb, TQ));
-        dist_tile_kernel<<<grid, 256, 0, c->stream>>>(dQ + (uint64_t)q0 * c->ld, mb, c->X, c->n, (int)c->ld,
-                                                      q_self ? q_self + q0 : nullptr, D, c->n);
+        dist_tile_kernel<false><<<grid, 256, 0, c->stream>>>(dQ + (uint64_t)q0 * c->ld, mb, c->X, c->n, 1, (int)c->ld,
+                                                             q_self ? q_self + q0 : nullptr,
+                                                             DistOut{D, c->n, nullptr, nullptr, nullptr, 0});
         KCNA_LAUNCHED(c);
-        select_kernel<<<mb, SEL_T, 0, c->stream>>>(D, c->n, c->n, k, q0, d_out_ids, d_out_d, c->d_err);
+        if (cached)
+            select_kernel<true><<<mb, SEL_T, (size_t)c->n * 4, c->stream>>>(D, c->n, c->n, k, q0, d_out_ids, d_out_d,
+                                                                            c->d_err);
+        else
+            select_kernel<false><<<mb, SEL_T, 0, c->stream>>>(D, c->n, c->n, k, q0, d_out_ids, d_out_d, c->d_err);
         KCNA_LAUNCHED(c);
         KCNA_TRY(kcna_cuda_check(c, cudaGetLastError(), "knn kernels"));
     }
     return KCNA_OK;
+}
+
+// A bound per query from a sample, the rows that may lie within it, selection among those.
+static kcna_status knn_bounded(kcna_ctx *c, const float *dQ, uint32_t m, const uint32_t *q_self, uint32_t k, uint32_t s,
+                               uint32_t *d_out_ids, float *d_out_d) {
+    const uint32_t batch = std::min<uint32_t>(m, 2048), rank = std::max<uint32_t>(k, 32), stride = c->n / s;
+    // the tensor-core screen pays from about 0.1 ms of FP32 work on
+    const bool screened = c->ld <= 128 && (uint64_t)m * c->n * c->ld >= (1ull << 30);
+    uint64_t *cand = nullptr;
+    uint32_t *words = nullptr; // bounds, counts, and the number of queries to do again
+    kcna_status st = kcna_alloc(c, &cand, ((uint64_t)batch * KNN_CAP + (screened ? 1 : 0)) / (screened ? 2 : 1), "k-NN lists");
+    if (st == KCNA_OK) st = kcna_alloc(c, &words, 2 * (size_t)batch + 1, "k-NN bounds");
+    const bool cached = s <= SEL_CACHE;
+    const size_t fsm = KNN_CAP * 8 + (screened ? (size_t)c->ld * 4 : 0);
+    if (st == KCNA_OK && cached)
+        st = kcna_cuda_check(c, cudaFuncSetAttribute(knn_bound_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                     (int)(SEL_CACHE * 4)),
+                             "knn smem attr");
+    if (st == KCNA_OK)
+        st = kcna_cuda_check(c, cudaFuncSetAttribute(knn_final_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                     (int)fsm),
+                             "knn smem attr");
+    if (st == KCNA_OK)
+        st = kcna_cuda_check(c, cudaFuncSetAttribute(knn_final_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                     (int)fsm),
+                             "knn smem attr");
+    for (uint32_t q0 = 0; q0 < m && st == KCNA_OK; q0 += batch) {
+        const uint32_t mb = std::min(batch, m - q0);
+        void *buf = nullptr; // asked for each time: knn_all below may move the scratch
+        if ((st = kcna_scratch(c, (uint64_t)batch * s * 4, &buf)) != KCNA_OK) break;
+        float *D = (float *)buf;
+        const float *Q = dQ + (uint64_t)q0 * c->ld;
+        const uint32_t *self = q_self ? q_self + q0 : nullptr;
+        uint32_t *thresh = words, *cnt = words + batch, *redo = words + 2 * (size_t)batch;
+        cudaMemsetAsync(redo, 0, 4, c->stream);
+        dist_tile_kernel<false><<<dim3(kcna_div_up(s, TB), kcna_div_up(mb, TQ)), 256, 0, c->stream>>>(
+            Q, mb, c->X, s, stride, (int)c->ld, self, DistOut{D, s, nullptr, nullptr, nullptr, 0});
+        if (cached)
+            knn_bound_kernel<true><<<mb, SEL_T, (size_t)s * 4, c->stream>>>(D, s, rank, thresh, cnt);
+        else
+            knn_bound_kernel<false><<<mb, SEL_T, 0, c->stream>>>(D, s, rank, thresh, cnt);
+        c->launches += 2;
+        if (screened) {
+            if ((st = kcna_knn_filter(c, Q, mb, thresh, reinterpret_cast<uint32_t *>(cand), cnt, KNN_CAP)) != KCNA_OK) break;
+            knn_final_kernel<true><<<mb, SEL_T, fsm, c->stream>>>(Q, c->X, (int)c->ld, self, nullptr,
+                                                                  reinterpret_cast<uint32_t *>(cand), cnt, k, q0,
+                                                                  d_out_ids, d_out_d, redo, c->d_err);
+        } else {
+            dist_tile_kernel<true><<<dim3(kcna_div_up(c->n, TB), kcna_div_up(mb, TQ)), 256, 0, c->stream>>>(
+                Q, mb, c->X, c->n, 1, (int)c->ld, self, DistOut{nullptr, 0, thresh, cand, cnt, KNN_CAP});
+            knn_final_kernel<false><<<mb, SEL_T, fsm, c->stream>>>(Q, c->X, (int)c->ld, self, cand, nullptr, cnt, k, q0,
+                                                                   d_out_ids, d_out_d, redo, c->d_err);
+            c->launches += 1;
+        }
+        c->launches += 1;
+        uint32_t again = 0;
+        st = kcna_cuda_check(c, cudaGetLastError(), "knn kernels");
+        if (st == KCNA_OK) st = kcna_cuda_check(c, cudaMemcpyAsync(&again, redo, 4, cudaMemcpyDeviceToHost, c->stream), "d2h");
+        if (st == KCNA_OK) st = kcna_cuda_check(c, cudaStreamSynchronize(c->stream), "knn sync");
+        if (st != KCNA_OK || again == 0) continue;
+        if (again > 64) { // too many to do one by one
+            st = knn_all(c, Q, mb, self, k, d_out_ids + (uint64_t)q0 * k, d_out_d + (uint64_t)q0 * k);
+            continue;
+        }
+        std::vector<uint32_t> h(mb);
+        st = kcna_cuda_check(c, cudaMemcpyAsync(h.data(), cnt, (size_t)mb * 4, cudaMemcpyDeviceToHost, c->stream), "d2h");
+        if (st == KCNA_OK) st = kcna_cuda_check(c, cudaStreamSynchronize(c->stream), "knn sync");
+        for (uint32_t i = 0; i < mb && st == KCNA_OK; ++i)
+            if (h[i] > KNN_CAP || h[i] < k)
+                st = knn_all(c, Q + (uint64_t)i * c->ld, 1, self ? self + i : nullptr, k, d_out_ids + (uint64_t)(q0 + i) * k,
+                             d_out_d + (uint64_t)(q0 + i) * k);
+    }
+    kcna_release(c, cand);
+    kcna_release(c, words);
+    return st;
+}
+
+kcna_status kcna_knn_device(kcna_ctx *c, const float *dQ, uint32_t m, const uint32_t *q_self, uint32_t k,
+                            uint32_t *d_out_ids, float *d_out_d) {
+    if (k == 0 || k > SEL_MAXK || k > c->n) return kcna_fail(c, KCNA_E_ARG, "knn: k must be in [1, min(1024, n)]");
+    if (q_self && k >= c->n) return kcna_fail(c, KCNA_E_ARG, "knn: k must be < n when self is excluded");
+    // rows sampled for the bound: about 4,096 of n then lie within it.  Bases up
+    // to the cached selection's length take two launches the first way (20,000
+    // rows, one query: 14 us on the device); above, and where many queries meet
+    // them, the bound pays, unless k is so large that the sample is half the base
+    const uint64_t s = std::max<uint64_t>(std::max<uint64_t>(2048, 2 * (uint64_t)k),
+                                          (std::max<uint64_t>(k, 32) * c->n + 4095) / 4096);
+    const bool bounded = 2 * s <= c->n && s * 4 * 2048 <= (1ull << 31) &&
+                         (c->n > SEL_CACHE || ((uint64_t)m * c->n >= (1ull << 25) && c->n >= 16384));
+    if (bounded) return knn_bounded(c, dQ, m, q_self, k, (uint32_t)s, d_out_ids, d_out_d);
+    return knn_all(c, dQ, m, q_self, k, d_out_ids, d_out_d);
 }
