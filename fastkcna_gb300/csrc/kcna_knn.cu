@@ -118,9 +118,10 @@ constexpr int SEL_T = 512;
 constexpr int SEL_BINS = 4096;
 constexpr int SEL_MAXK = 1024;
 constexpr int SEL_TIES = 1024;
+constexpr int SEL_QUICK = 256;
 
 constexpr uint32_t KNN_CAP = 8192;       // rows handed on per query at most
-constexpr uint32_t SEL_CACHE = 40960;    // a distance row up to this length is read once, into shared memory
+constexpr uint32_t SEL_CACHE = 40960;    // a sample up to this length is read once, into shared memory; dispatch below
 
 struct SelectShared {
     uint32_t hist[SEL_BINS];
@@ -187,9 +188,55 @@ __device__ uint32_t kth_word(SelectShared &S, uint32_t n, uint32_t want, At at) 
 
 // The k smallest (distance, id) of n entries, dist(j) and id(j), sorted, to
 // out; by the whole block.
+// Up to k = SEL_QUICK the k-th smallest of the threads' own minima bounds the
+// k-th distance: k entries lie within it, and seldom more than a few over (the
+// expected number at k = SEL_QUICK is 355).  Those alone are collected and
+// sorted, with two reads of each entry and no histogram, whose atomics meet in
+// a few bins as distances share their leading bits: one query, k = 10 of 20,000
+// x 32 rows takes 57 us as a call, 68 with the histograms.  Larger k, or more than
+// SEL_MAXK entries within the bound, take the histogram passes.
 template <class Dist, class Id>
 __device__ void select_k(SelectShared &S, uint64_t *s_out, uint64_t *s_tie, uint32_t n, uint32_t k, Dist dist, Id id,
                          uint32_t *out_ids, float *out_d, int *err) {
+    if (k <= SEL_QUICK) {
+        constexpr int U = 8; // loads in flight
+        uint32_t lo = 0xFFFFFFFFu;
+        for (uint32_t j0 = threadIdx.x; j0 < n; j0 += U * SEL_T) {
+            uint32_t v[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) v[u] = j0 + u * SEL_T < n ? dist(j0 + u * SEL_T) : 0xFFFFFFFFu;
+#pragma unroll
+            for (int u = 0; u < U; ++u) lo = min(lo, v[u]);
+        }
+        s_tie[threadIdx.x] = lo;
+        if (threadIdx.x == 0) S.nout = 0;
+        kcna_cta_bitonic(s_tie, SEL_T); // syncs before and after
+        const uint32_t bound = (uint32_t)s_tie[k - 1];
+        for (uint32_t j0 = threadIdx.x; j0 < n; j0 += U * SEL_T) {
+            uint32_t v[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) v[u] = j0 + u * SEL_T < n ? dist(j0 + u * SEL_T) : 0xFFFFFFFFu;
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (j0 + u * SEL_T < n && v[u] <= bound) {
+                    const uint32_t p = atomicAdd(&S.nout, 1u);
+                    if (p < SEL_MAXK) s_out[p] = ((uint64_t)v[u] << 32) | id(j0 + u * SEL_T);
+                }
+        }
+        __syncthreads();
+        const uint32_t got = S.nout;
+        if (got <= SEL_MAXK) {
+            const int gp = kcna_pow2_ceil_d((int)got);
+            for (int i = got + threadIdx.x; i < gp; i += SEL_T) s_out[i] = KCNA_EMPTY_KEY;
+            kcna_cta_bitonic(s_out, gp);
+            for (uint32_t i = threadIdx.x; i < k; i += SEL_T) {
+                out_ids[i] = (uint32_t)s_out[i];
+                out_d[i] = __uint_as_float((uint32_t)(s_out[i] >> 32));
+            }
+            return;
+        }
+        __syncthreads(); // S.nout is written again below
+    }
     const uint32_t T = kth_word(S, n, k - 1, dist); // k-th smallest distance bits
     if (threadIdx.x == 0) {
         S.nout = 0;
@@ -227,21 +274,12 @@ __device__ void select_k(SelectShared &S, uint64_t *s_out, uint64_t *s_tie, uint
     }
 }
 
-// CACHED: the distance row fits shared memory and is read once.
-template <bool CACHED>
 __global__ void __launch_bounds__(SEL_T) select_kernel(const float *__restrict__ D, uint64_t ldD, uint32_t n,
                                                        uint32_t k, uint32_t q_base, uint32_t *__restrict__ out_ids,
                                                        float *__restrict__ out_d, int *err) {
-    extern __shared__ __align__(16) uint32_t s_row[]; // CACHED: n words
     __shared__ SelectShared S;
     __shared__ uint64_t s_out[SEL_MAXK], s_tie[SEL_TIES];
     const uint32_t *row = reinterpret_cast<const uint32_t *>(D + (uint64_t)blockIdx.x * ldD);
-    if (CACHED) {
-#pragma unroll 8
-        for (uint32_t j = threadIdx.x; j < n; j += SEL_T) s_row[j] = row[j];
-        row = s_row;
-        __syncthreads();
-    }
     const uint64_t ob = (uint64_t)(q_base + blockIdx.x) * k;
     select_k(S, s_out, s_tie, n, k, [&](uint32_t j) { return row[j]; }, [](uint32_t j) { return j; }, out_ids + ob,
              out_d + ob, err);
@@ -352,11 +390,6 @@ static kcna_status knn_all(kcna_ctx *c, const float *dQ, uint32_t m, const uint3
     void *buf = nullptr;
     KCNA_TRY(kcna_scratch(c, (uint64_t)batch * row_bytes, &buf));
     float *D = (float *)buf;
-    const bool cached = c->n <= SEL_CACHE;
-    if (cached)
-        KCNA_TRY(kcna_cuda_check(c, cudaFuncSetAttribute(select_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                         (int)(SEL_CACHE * 4)),
-                                 "select smem attr"));
     for (uint32_t q0 = 0; q0 < m; q0 += batch) {
         uint32_t mb = std::min(batch, m - q0);
         dim3 grid(kcna_div_up(c->n, TB), kcna_div_up(mb, TQ));
@@ -364,11 +397,7 @@ static kcna_status knn_all(kcna_ctx *c, const float *dQ, uint32_t m, const uint3
                                                              q_self ? q_self + q0 : nullptr,
                                                              DistOut{D, c->n, nullptr, nullptr, nullptr, 0});
         KCNA_LAUNCHED(c);
-        if (cached)
-            select_kernel<true><<<mb, SEL_T, (size_t)c->n * 4, c->stream>>>(D, c->n, c->n, k, q0, d_out_ids, d_out_d,
-                                                                            c->d_err);
-        else
-            select_kernel<false><<<mb, SEL_T, 0, c->stream>>>(D, c->n, c->n, k, q0, d_out_ids, d_out_d, c->d_err);
+        select_kernel<<<mb, SEL_T, 0, c->stream>>>(D, c->n, c->n, k, q0, d_out_ids, d_out_d, c->d_err);
         KCNA_LAUNCHED(c);
         KCNA_TRY(kcna_cuda_check(c, cudaGetLastError(), "knn kernels"));
     }
@@ -455,8 +484,8 @@ kcna_status kcna_knn_device(kcna_ctx *c, const float *dQ, uint32_t m, const uint
     if (k == 0 || k > SEL_MAXK || k > c->n) return kcna_fail(c, KCNA_E_ARG, "knn: k must be in [1, min(1024, n)]");
     if (q_self && k >= c->n) return kcna_fail(c, KCNA_E_ARG, "knn: k must be < n when self is excluded");
     // rows sampled for the bound: about 4,096 of n then lie within it.  Bases up
-    // to the cached selection's length take two launches the first way (20,000
-    // rows, one query: 14 us on the device); above, and where many queries meet
+    // to SEL_CACHE rows take two launches the first way (20,000
+    // rows, one query: 57 us with its copies); above, and where many queries meet
     // them, the bound pays, unless k is so large that the sample is half the base
     const uint64_t s = std::max<uint64_t>(std::max<uint64_t>(2048, 2 * (uint64_t)k),
                                           (std::max<uint64_t>(k, 32) * c->n + 4095) / 4096);

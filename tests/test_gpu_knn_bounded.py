@@ -43,6 +43,29 @@ def test_bounded_knn_equals_brute_force(index, oracle, kind, n, d, m, k):
     assert np.array_equal(gd[some], od)
 
 
+@pytest.mark.parametrize("kind,n,k", [
+    ("normal", 300, 300), ("normal", 511, 256), ("normal", 512, 256), ("normal", 513, 257),
+    ("normal", 4097, 256), ("normal", 20000, 10), ("nan", 4000, 256), ("levels", 3000, 256), ("levels", 9001, 7),
+])
+def test_small_base_selection(index, oracle, kind, n, k):
+    """Selection from every distance: both sides of the thread minima's largest
+    k, ragged rows per thread, and equal distances (six distinct ones, each held
+    by fewer rows than a tie list, by more than the collected list together)."""
+    d = 8
+    X, Q = _rows("normal" if kind == "levels" else kind, n, d, 21), _rows("normal", 3, d, 22)
+    if kind == "levels":
+        X[:] = 0
+        X[:, 0] = np.arange(n) % (6 if n < 6000 else 12)
+        Q[:] = 0
+    index.upload(X)
+    gi, gd = index.knn_queries(Q, k)
+    if kind == "nan":  # the oracle's insertion has no order for NaN; one more result takes the histogram passes
+        oi, od = (a[:, :k] for a in index.knn_queries(Q, k + 1))
+    else:
+        oi, od = oracle.knn_queries(X, Q, k)
+    assert np.array_equal(gi, oi) and np.array_equal(gd, od, equal_nan=True)
+
+
 def test_bounded_knn_of_own_rows(index, oracle):
     X = _rows("int", 50001, 128, 13)
     index.upload(X)
