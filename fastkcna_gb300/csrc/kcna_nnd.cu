@@ -1330,8 +1330,13 @@ __global__ void __launch_bounds__(SEL_WARPS * 32) select_reverse_kernel(uint32_t
 // beyond the target's radius becomes an empty key too (the merges skip those).
 // Warp per target: the target's row in shared memory and its first np pool
 // ids (np = min(count, limit), the entries the merge compares against) in an
-// open-addressing table of ht slots; lane per candidate.  ht = 0 skips the
-// repeat test.  (Adding the candidate ids to the table as well, to skip
+// open-addressing table of ht slots.  ht = 0 skips the repeat test.
+// The candidates left after that test are queued, and a lane takes one row of
+// 32 queued ones, eight 16-byte loads (a line) in flight: with a lane per
+// candidate as they come, repeats left most lanes idle, and a line was asked
+// for 16 bytes at a time after the table's share of the cache had lost it.
+// 150,007 x 96, pools of 260, 1.7e8 recomputed
+// pairs in six iterations: 32.6 ms before, 16.6 now.  (Adding the candidate ids to the table as well, to skip
 // repeats within the buffer, was measured slower: the larger table costs
 // occupancy and the inserts cost atomics.)
 __global__ void __launch_bounds__(256) rescore_kernel(const float *__restrict__ X, int ld, uint32_t N,
@@ -1342,6 +1347,7 @@ __global__ void __launch_bounds__(256) rescore_kernel(const float *__restrict__ 
                                                       uint32_t limit, uint32_t ht, unsigned long long *rescored,
                                                       unsigned long long *repeats) {
     extern __shared__ __align__(16) float s_rows[]; // 8 warps x ld, then 8 warps x ht table slots
+    __shared__ uint32_t s_queue[8][64];             // candidate indices waiting for their distance
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t t = blockIdx.x * 8 + w;
     if (t >= N) return;
@@ -1367,29 +1373,58 @@ __global__ void __launch_bounds__(256) rescore_kernel(const float *__restrict__ 
     uint64_t *buf = cand + 2 * (uint64_t)t * CB; // keys at even words
     const float4 *x4 = reinterpret_cast<const float4 *>(xt);
     unsigned long long n = 0, rep = 0;
-    for (uint32_t j = lane; j < nc; j += 32) {
-        const uint64_t k = buf[2 * j];
-        if (kcna_key_noflags(k) == KCNA_EMPTY_KEY_NOFLAGS) continue;
-        const uint32_t id = kcna_key_id(k);
-        bool in_pool = false;
-        if (ht) {
-            uint32_t h = (id * 0x9E3779B1u) & (ht - 1);
-            for (uint32_t probe = 0; probe < ht; ++probe, h = (h + 1) & (ht - 1)) {
-                const uint32_t e = tab[h];
-                if (e == id) in_pool = true;
-                if (e == id || e == KCNA_NONE) break;
+    uint32_t *queue = s_queue[w];
+    const int nv = ld >> 2;
+    uint32_t queued = 0; // at most 31 stay between rounds
+    for (uint32_t j0 = 0; j0 < nc; j0 += 32) {
+        const uint32_t j = j0 + lane;
+        bool want = false;
+        if (j < nc) {
+            const uint64_t k = buf[2 * j];
+            if (kcna_key_noflags(k) != KCNA_EMPTY_KEY_NOFLAGS) {
+                const uint32_t id = kcna_key_id(k);
+                want = true;
+                if (ht) {
+                    uint32_t h = (id * 0x9E3779B1u) & (ht - 1);
+                    for (uint32_t probe = 0; probe < ht; ++probe, h = (h + 1) & (ht - 1)) {
+                        const uint32_t e = tab[h];
+                        if (e == id) want = false;
+                        if (e == id || e == KCNA_NONE) break;
+                    }
+                }
+                if (!want) {
+                    buf[2 * j] = KCNA_EMPTY_KEY;
+                    ++rep;
+                }
             }
         }
-        if (in_pool) {
-            buf[2 * j] = KCNA_EMPTY_KEY;
-            ++rep;
-            continue;
+        const unsigned wm = __ballot_sync(KCNA_FULL, want);
+        if (want) queue[queued + __popc(wm & ((1u << lane) - 1u))] = j;
+        queued += __popc(wm);
+        __syncwarp();
+        const bool last = j0 + 32 >= nc;
+        while (queued >= 32 || (last && queued)) {
+            const uint32_t take = min(queued, 32u);
+            if ((uint32_t)lane < take) {
+                const uint32_t jq = queue[queued - take + lane];
+                const uint64_t k = buf[2 * jq];
+                const uint32_t id = kcna_key_id(k);
+                const float4 *xc = reinterpret_cast<const float4 *>(X + (uint64_t)id * ld);
+                float d = 0.f;
+                for (int q0 = 0; q0 < nv; q0 += 8) {
+                    float4 v[8];
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) v[u] = __ldg(xc + min(q0 + u, nv - 1));
+#pragma unroll
+                    for (int u = 0; u < 8; ++u)
+                        if (q0 + u < nv) d = kcna_acc4(d, x4[q0 + u], v[u]);
+                }
+                buf[2 * jq] = d <= rad ? kcna_key(d, id, kcna_key_flags(k)) : KCNA_EMPTY_KEY;
+                ++n;
+            }
+            queued -= take;
+            __syncwarp();
         }
-        const float4 *xc = reinterpret_cast<const float4 *>(X + (uint64_t)id * ld);
-        float d = 0.f;
-        for (int q = 0; q < (ld >> 2); ++q) d = kcna_acc4(d, x4[q], __ldg(xc + q));
-        buf[2 * j] = d <= rad ? kcna_key(d, id, kcna_key_flags(k)) : KCNA_EMPTY_KEY;
-        ++n;
     }
     n = kcna_warp_sum(n);
     rep = kcna_warp_sum(rep);
