@@ -1025,7 +1025,16 @@ struct P2kWarp {
     float rad[PJ_U];
 };
 static_assert(PJ_U * (PJ_COLS + 1) <= pairs_region(PJ_ROWS), "the distance matrix fits the rows' region");
-static_assert((PJ_U / 4) * (PJ_COLS / 4) <= 32 * PT_MAXR, "a tile's micro-tiles fit the lanes");
+// every pair of a unit: min(PJ_U, PJ_ROWS - nw) pushers by nw neighbours
+constexpr int p2k_most_tiles() {
+    int most = 0;
+    for (int nw = 1; nw <= PJ_COLS; ++nw) {
+        const int cap = PJ_U < PJ_ROWS - nw ? PJ_U : PJ_ROWS - nw, t = ((cap + 3) >> 2) * ((nw + 3) >> 2);
+        most = t > most ? t : most;
+    }
+    return most;
+}
+static_assert(p2k_most_tiles() <= 32 * PT_MAXR, "a unit's micro-tiles fit the lanes");
 
 // rows [0, nw): neighbours, the first nwN new; [nw, nw + nu): pushers, the first nuN new
 template <int R, class RowsT>
@@ -1178,13 +1187,21 @@ __global__ void __launch_bounds__(PJ_WARPS * 32, 1) p2k_warp_kernel(RowsT rows, 
         }
         __syncwarp();
         const bool more = next(nx);
-        const int T = ((nuN + 3) >> 2) * ((nw + 3) >> 2) + ((nu - nuN + 3) >> 2) * ((nwN + 3) >> 2);
+        // micro-tiles of the pairs that meet: the two kinds of pushers round up separately, and 53 to 58
+        // neighbours can then need up to 105; every pair takes 90 at most, and meets() below drops the rest
+        int T = ((nuN + 3) >> 2) * ((nw + 3) >> 2) + ((nu - nuN + 3) >> 2) * ((nwN + 3) >> 2);
+        int tN = nuN, twN = nwN; // as the tiles see them
+        if (T > 32 * PT_MAXR) {
+            tN = nu;
+            twN = nw;
+            T = ((nu + 3) >> 2) * ((nw + 3) >> 2);
+        }
         if (T <= 32)
-            p2k_warp_tiles<1>(rows, S, nw, nwN, nu, nuN, T);
+            p2k_warp_tiles<1>(rows, S, nw, twN, nu, tN, T);
         else if (T <= 64)
-            p2k_warp_tiles<2>(rows, S, nw, nwN, nu, nuN, T);
+            p2k_warp_tiles<2>(rows, S, nw, twN, nu, tN, T);
         else
-            p2k_warp_tiles<PT_MAXR>(rows, S, nw, nwN, nu, nuN, T);
+            p2k_warp_tiles<PT_MAXR>(rows, S, nw, twN, nu, tN, T);
         if (pos >= 0) S.rad[pos] = rad;
         __syncwarp();
         // count pass (lane i keeps pusher i's ballots), reservations together, write pass
