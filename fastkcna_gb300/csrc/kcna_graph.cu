@@ -41,30 +41,78 @@ __device__ __forceinline__ bool occludes(const PruneRule &r, float td, float djk
     return djk < pd;
 }
 
+// Row lengths whose batches are staged: three prunes of 60,000 unit rows, 40
+// kept, pools of 260, straight against staged: d = 8 2.0 / 2.2 ms, 32 5.1 / 4.0,
+// 96 16.2 / 12.3, 128 21.9 / 17.2, 160 27.7 / 23.2, 192 33.5 / 31.7, 256 45.4 /
+// 45.0 (the batches of ever fewer warps fit an SM).
+constexpr int PRUNE_STAGED_MIN = 32, PRUNE_STAGED_MAX = 192;
+// pitch in floats of a staged row: an odd number of 16-byte pieces, so that the lanes' rows lie in distinct banks
+__host__ __device__ constexpr int prune_pitch(int ld) { return ((ld >> 2) | 1) * 4; }
+__host__ __device__ constexpr size_t prune_staged_bytes(int ld) { return (size_t)(32 * prune_pitch(ld) + 4 * ld) * 4; }
+__device__ __forceinline__ void prune_copy16(float *dst, const RowsF32 *rows, uint32_t id, int c) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
+                 "l"(rows->p + (uint64_t)id * rows->ld + 4 * c)
+                 : "memory");
+}
+__device__ __forceinline__ void prune_copy16(float *dst, const RowsB16 *rows, uint32_t id, int c) {
+    *reinterpret_cast<float4 *>(dst) = rows->ld4(id, c);
+}
+
+// Lane of the n-th (0-based) set bit of m, below 32 whatever n.
+__device__ __forceinline__ int nth_bit(unsigned m, int n) {
+    int pos = 0;
+#pragma unroll
+    for (int w = 16; w; w >>= 1) {
+        const int c = __popc((m >> pos) & ((1u << w) - 1u));
+        if (n >= c) {
+            n -= c;
+            pos += w;
+        }
+    }
+    return pos;
+}
+
 // Occlusion prune of one candidate list by one warp, in the reference's order
 // (kept[0] = first candidate; each later candidate p is dropped when a kept t
 // has the same id or occludes it; stop at `range` kept), with the same result
 // as the sequential scan.  Almost every candidate is occluded by one of the
 // first kept neighbours, so each batch of 32 candidates (one per lane) is first
 // tested against kept[0..3] with four independent FMA chains (the candidate row
-// is read once, eight loads in flight); the few survivors are then tested one
-// at a time against kept[4..nk) with one lane per kept row; finally the batch
-// is resolved in candidate order (the first unoccluded lane is kept and tests
-// the later lanes).  Rows are read through R (FP32 or exact BF16 copy).
+// is read once, eight loads in flight); the survivors are then tested against
+// kept[4..nk), the (survivor, kept row) pairs dealt to the lanes; finally the
+// batch is resolved in candidate order (the first unoccluded lane is kept and
+// tests the later lanes; the last eight or fewer test all their pairs at once).
+// Instruction issue bounds it: with one survivor at a time against a lane per
+// kept row, and a round per kept candidate, half of the lanes had no pair (30,000
+// x 96, 40 kept: 16.5 of 32 lanes, 43 instructions a pair and warp).  Prune
+// of the 150,007 x 96 layer build 35.3 -> 23.9 ms, of 150,001 x 128 NSG 28 ->
+// 20.3 (staging alone 33.1 and 21.9), of the 40,009 x 960 tau-MNG 65 -> 54.
+// Rows are read through R (FP32 or exact BF16 copy).
 // With nk0 > 0 the scan continues a kept list kid/kd[0, nk0) (from a prune
 // that covered the candidates before `first`) at candidate `first`.
-template <class R, typename GetFn>
+//
+// STAGED (FP32 rows of PRUNE_STAGED_MIN to _MAX floats): the batch's rows come to
+// shared memory once (st: 32 rows, pitch prune_pitch(ld), then kept[0..3]) and
+// every test reads them there.  A candidate takes part in 3.4 tests on average
+// and its row was read again for each test within its batch, 16 bytes a lane
+// from 32 rows at a time, out of an L1 too small for the block's batches.
+template <bool STAGED = false, class R, typename GetFn>
 __device__ int warp_prune(const R &rows, uint32_t n_oracle, const PruneRule &rule, int first, int lim, int range,
-                          GetFn get, uint32_t *kid, float *kd, unsigned long long *comps, int nk0 = 0) {
+                          GetFn get, uint32_t *kid, float *kd, unsigned long long *comps, int nk0 = 0,
+                          float *st = nullptr) {
     const int lane = kcna_lane();
     const int nv = rows.ld >> 2;
     if (range <= 0) return 0;
     if (first >= lim) return nk0;
     int nk = nk0, start = first;
+    const int pitch = prune_pitch(rows.ld);
+    float *kept_rows = st + 32 * pitch; // STAGED: rows of kept[0..3], rows.ld apart
     if (nk0 == 0) {
         uint32_t id0;
         float d0;
         get(first, id0, d0);
+        if (STAGED)
+            for (int c = lane; c < nv; c += 32) reinterpret_cast<float4 *>(kept_rows)[c] = rows.ld4(id0, c);
         if (lane == 0) {
             kid[0] = id0;
             kd[0] = d0;
@@ -84,12 +132,39 @@ __device__ int warp_prune(const R &rows, uint32_t n_oracle, const PruneRule &rul
             live = id < n_oracle; // src/kgraph.cpp:1822 `if (p.id >= oracle.size()) continue;`
         }
         bool occ = false;
+        if (STAGED) {
+            const unsigned lm = __ballot_sync(KCNA_FULL, live);
+            int r = 0, c = lane;
+            while (c >= nv) c -= nv, ++r;
+            for (int i = 0; i < nv; ++i) { // 32 nv pieces of 16 bytes, r <= 31 throughout
+                const uint32_t rid = __shfl_sync(KCNA_FULL, id, r);
+                if ((lm >> r) & 1u) prune_copy16(st + r * pitch + 4 * c, &rows, rid, c);
+                c += 32;
+                while (c >= nv) c -= nv, ++r;
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+            __syncwarp();
+        }
+        const float4 *own = reinterpret_cast<const float4 *>(st + lane * pitch);
         // phase 1: kept[0..min(nk,4)), four independent chains, candidate row read once
         const int t1 = min(nk, 4);
         if (live) {
             const uint32_t k0 = kid[0], k1 = kid[t1 > 1 ? 1 : 0], k2 = kid[t1 > 2 ? 2 : 0], k3 = kid[t1 > 3 ? 3 : 0];
             float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
-            for (int b0 = 0; b0 < nv; b0 += 8) {
+            if (STAGED) {
+                const float4 *kr = reinterpret_cast<const float4 *>(kept_rows);
+                const float4 *r1 = kr + (t1 > 1 ? nv : 0), *r2 = kr + (t1 > 2 ? 2 * nv : 0), *r3 = kr + (t1 > 3 ? 3 * nv : 0);
+#pragma unroll 4
+                for (int k = 0; k < nv; ++k) {
+                    const float4 pv = own[k];
+                    a0 = kcna_acc4(a0, kr[k], pv);
+                    a1 = kcna_acc4(a1, r1[k], pv);
+                    a2 = kcna_acc4(a2, r2[k], pv);
+                    a3 = kcna_acc4(a3, r3[k], pv);
+                }
+            }
+            for (int b0 = STAGED ? nv : 0; b0 < nv; b0 += 8) {
                 float4 pv[8];
 #pragma unroll
                 for (int u = 0; u < 8; ++u) pv[u] = b0 + u < nv ? rows.ld4(id, b0 + u) : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -117,33 +192,95 @@ __device__ int warp_prune(const R &rows, uint32_t n_oracle, const PruneRule &rul
             }
         }
         unsigned rem = __ballot_sync(KCNA_FULL, live && !occ);
-        // phase 2: survivors against kept[4..nk), one lane per kept row
-        if (nk > 4) {
-            unsigned todo = rem;
-            while (todo) {
-                const int b = __ffs(todo) - 1;
-                todo &= todo - 1;
+        // phase 2: survivors against kept[4..nk), 32 kept rows at a time, one lane per pair
+        for (int t0 = 4; t0 < nk && rem; t0 += 32) {
+            const int len = min(32, nk - t0), total = __popc(rem) * len;
+            const int sel = nth_bit(rem, lane);
+            unsigned hit = 0;
+            for (int p0 = 0; p0 < total; p0 += 32) {
+                const int p = min(p0 + lane, total - 1), si = p / len, t = t0 + p - si * len;
+                const int b = __shfl_sync(KCNA_FULL, sel, si);
                 const uint32_t bid = __shfl_sync(KCNA_FULL, id, b);
                 const float bd = __shfl_sync(KCNA_FULL, pd, b);
-                bool hit = false;
-                for (int t0 = 4; t0 < nk && !hit; t0 += 32) {
-                    const int t = t0 + lane;
-                    bool h = false;
-                    if (t < nk) {
-                        if (kid[t] == bid) {
-                            h = true;
+                bool h = false;
+                if (p0 + lane < total) {
+                    if (kid[t] == bid) {
+                        h = true;
+                    } else {
+                        ++cc;
+                        float djk = 0.f;
+                        if (STAGED) {
+                            const float4 *xb = reinterpret_cast<const float4 *>(st + b * pitch);
+                            for (int k0 = 0; k0 < nv; k0 += 8) {
+                                float4 v[8];
+#pragma unroll
+                                for (int u = 0; u < 8; ++u) v[u] = rows.ld4(kid[t], min(k0 + u, nv - 1));
+#pragma unroll
+                                for (int u = 0; u < 8; ++u)
+                                    if (k0 + u < nv) djk = kcna_acc4(djk, v[u], xb[k0 + u]);
+                            }
                         } else {
-                            ++cc;
-                            h = occludes(rule, kd[t], rows_l2(rows, kid[t], bid), bd);
+                            djk = rows_l2(rows, kid[t], bid);
                         }
+                        h = occludes(rule, kd[t], djk, bd);
                     }
-                    hit = __ballot_sync(KCNA_FULL, h) != 0;
                 }
-                if (hit) rem &= ~(1u << b);
+                hit |= __reduce_or_sync(KCNA_FULL, h ? 1u << b : 0u);
             }
+            rem &= ~hit;
         }
         // in-batch resolution, in candidate order
         while (rem && nk < range) {
+            const int left = __popc(rem);
+            if (left > 1 && left <= 8) { // the pairs of the last few (28 at most), one lane each: pair (i, j), i < j, is j (j - 1) / 2 + i
+                const int sel = nth_bit(rem, lane);
+                const int j = 1 + (lane >= 1) + (lane >= 3) + (lane >= 6) + (lane >= 10) + (lane >= 15) + (lane >= 21);
+                const int i = lane - j * (j - 1) / 2;
+                const bool pair = lane < left * (left - 1) / 2;
+                const int la = __shfl_sync(KCNA_FULL, sel, i & 7), lb = __shfl_sync(KCNA_FULL, sel, j & 7);
+                const uint32_t ia = __shfl_sync(KCNA_FULL, id, la), ib = __shfl_sync(KCNA_FULL, id, lb);
+                const float da = __shfl_sync(KCNA_FULL, pd, la), db = __shfl_sync(KCNA_FULL, pd, lb);
+                const bool same = ia == ib;
+                bool oc = same;
+                if (pair && !same) {
+                    float djk = 0.f;
+                    if (STAGED) {
+                        const float4 *xi = reinterpret_cast<const float4 *>(st + la * pitch);
+                        const float4 *xj = reinterpret_cast<const float4 *>(st + lb * pitch);
+#pragma unroll 4
+                        for (int k = 0; k < nv; ++k) djk = kcna_acc4(djk, xi[k], xj[k]);
+                    } else {
+                        djk = rows_l2(rows, ia, ib);
+                    }
+                    oc = occludes(rule, da, djk, db);
+                }
+                const unsigned occ_pairs = __ballot_sync(KCNA_FULL, pair && oc), same_pairs = __ballot_sync(KCNA_FULL, pair && same);
+                unsigned m = (1u << left) - 1u;
+                while (m && nk < range) {
+                    const int x = __ffs(m) - 1, lx = __shfl_sync(KCNA_FULL, sel, x);
+                    const uint32_t xid = __shfl_sync(KCNA_FULL, id, lx);
+                    const float xd = __shfl_sync(KCNA_FULL, pd, lx);
+                    if (lane == 0) {
+                        kid[nk] = xid;
+                        kd[nk] = xd;
+                    }
+                    if (STAGED && nk < 4)
+                        for (int c = lane; c < nv; c += 32)
+                            reinterpret_cast<float4 *>(kept_rows)[nk * nv + c] =
+                                reinterpret_cast<const float4 *>(st + lx * pitch)[c];
+                    ++nk;
+                    m &= ~((2u << x) - 1u);
+                    bool gone = false;
+                    if (lane < 8 && (m >> lane) & 1u) { // the lane-th of them, after x
+                        const int q = lane * (lane - 1) / 2 + x;
+                        gone = (occ_pairs >> q) & 1u;
+                        cc += !((same_pairs >> q) & 1u);
+                    }
+                    m &= ~__ballot_sync(KCNA_FULL, gone);
+                }
+                __syncwarp();
+                break;
+            }
             const int a = __ffs(rem) - 1;
             const uint32_t aid = __shfl_sync(KCNA_FULL, id, a);
             const float ad = __shfl_sync(KCNA_FULL, pd, a);
@@ -151,6 +288,9 @@ __device__ int warp_prune(const R &rows, uint32_t n_oracle, const PruneRule &rul
                 kid[nk] = aid;
                 kd[nk] = ad;
             }
+            const float4 *xa = reinterpret_cast<const float4 *>(st + a * pitch);
+            if (STAGED && nk < 4)
+                for (int c = lane; c < nv; c += 32) reinterpret_cast<float4 *>(kept_rows)[nk * nv + c] = xa[c];
             ++nk;
             __syncwarp();
             rem &= ~((2u << a) - 1u); // lanes after a
@@ -161,11 +301,19 @@ __device__ int warp_prune(const R &rows, uint32_t n_oracle, const PruneRule &rul
                     o2 = true;
                 } else {
                     ++cc;
-                    o2 = occludes(rule, ad, rows_l2(rows, aid, id), pd);
+                    float djk = 0.f;
+                    if (STAGED) {
+#pragma unroll 4
+                        for (int k = 0; k < nv; ++k) djk = kcna_acc4(djk, xa[k], own[k]);
+                    } else {
+                        djk = rows_l2(rows, aid, id);
+                    }
+                    o2 = occludes(rule, ad, djk, pd);
                 }
             }
             rem &= ~__ballot_sync(KCNA_FULL, o2);
         }
+        if (STAGED) __syncwarp(); // the batch's rows are read
     }
     cc = kcna_warp_sum(cc);
     if (lane == 0 && comps && cc) atomicAdd(comps, cc);
@@ -175,7 +323,7 @@ __device__ int warp_prune(const R &rows, uint32_t n_oracle, const PruneRule &rul
 
 constexpr int PW = 4; // warps per prune block
 
-template <class R>
+template <bool STAGED, class R>
 __global__ void __launch_bounds__(PW * 32) prune_kernel(R rows, uint32_t N, const uint64_t *__restrict__ pool,
                                                         const uint32_t *__restrict__ pool_cnt, uint32_t cap,
                                                         PruneRule rule, int range, int maxc,
@@ -185,9 +333,10 @@ __global__ void __launch_bounds__(PW * 32) prune_kernel(R rows, uint32_t N, cons
                                                         const uint32_t *__restrict__ list) {
     extern __shared__ __align__(16) unsigned char smem[];
     const int w = threadIdx.x >> 5, lane = kcna_lane();
-    uint32_t *kid = reinterpret_cast<uint32_t *>(smem) + w * 2 * range;
+    // STAGED: a warp per block, the rows in front
+    uint32_t *kid = reinterpret_cast<uint32_t *>(smem + (STAGED ? prune_staged_bytes(rows.ld) : 0)) + w * 2 * range;
     float *kd = reinterpret_cast<float *>(kid + range);
-    const uint32_t item = blockIdx.x * PW + w; // node, or the item-th node of `list`
+    const uint32_t item = blockIdx.x * (blockDim.x >> 5) + w; // node, or the item-th node of `list`
     if (item >= n_items) return;
     const uint32_t q = list ? list[item] : item;
     const uint64_t *pr = pool + (uint64_t)q * cap;
@@ -200,7 +349,9 @@ __global__ void __launch_bounds__(PW * 32) prune_kernel(R rows, uint32_t N, cons
         id = kcna_key_id(k);
         dd = kcna_key_dist(k);
     };
-    const int nk = (first < cnt) ? warp_prune(rows, N, rule, first, max(lim, first + 1), range, get, kid, kd, comps) : 0;
+    const int nk = (first < cnt) ? warp_prune<STAGED>(rows, N, rule, first, max(lim, first + 1), range, get, kid, kd,
+                                                      comps, 0, reinterpret_cast<float *>(smem))
+                                 : 0;
     for (int j = lane; j < (int)W; j += 32) {
         g_ids[(uint64_t)q * W + j] = j < nk ? kid[j] : KCNA_NONE;
         g_dist[(uint64_t)q * W + j] = j < nk ? kd[j] : 0.f;
@@ -1400,11 +1551,19 @@ kcna_status kcna_prune_all(kcna_ctx *c, const kcna_params *p, int kind, uint64_t
         c->prune_exact += ex;
     } else if (n_items > 0) {
         if (c->bf16_exact)
-            prune_kernel<<<kcna_div_up(n_items, PW), PW * 32, sm, c->stream>>>(
+            prune_kernel<false><<<kcna_div_up(n_items, PW), PW * 32, sm, c->stream>>>(
                 RowsB16{c->Xh, (int)c->ld}, c->n, c->pool, c->pool_cnt, c->cap, rule, (int)range, maxc, c->g_ids,
                 c->g_dist, c->g_deg, c->W, c->counters + 16, n_items, list);
-        else
-            prune_kernel<<<kcna_div_up(n_items, PW), PW * 32, sm, c->stream>>>(
+        else if ((int)c->ld >= PRUNE_STAGED_MIN && (int)c->ld <= PRUNE_STAGED_MAX) {
+            const size_t ssm = prune_staged_bytes((int)c->ld) + (size_t)2 * range * 4;
+            KCNA_TRY(kcna_cuda_check(c, cudaFuncSetAttribute(prune_kernel<true, RowsF32>,
+                                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ssm),
+                                     "prune smem attr"));
+            prune_kernel<true><<<n_items, 32, ssm, c->stream>>>(
+                RowsF32{c->X, (int)c->ld}, c->n, c->pool, c->pool_cnt, c->cap, rule, (int)range, maxc, c->g_ids,
+                c->g_dist, c->g_deg, c->W, c->counters + 16, n_items, list);
+        } else
+            prune_kernel<false><<<kcna_div_up(n_items, PW), PW * 32, sm, c->stream>>>(
                 RowsF32{c->X, (int)c->ld}, c->n, c->pool, c->pool_cnt, c->cap, rule, (int)range, maxc, c->g_ids,
                 c->g_dist, c->g_deg, c->W, c->counters + 16, n_items, list);
         KCNA_LAUNCHED(c);
