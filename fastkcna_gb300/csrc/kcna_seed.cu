@@ -359,19 +359,17 @@ __global__ void __launch_bounds__(BAND_WARPS * 32) seed_band_kernel(R rows, uint
 // Initial pools, step 2: node i's slots sorted by (distance, id); the same id
 // from several tables gives the same key, so repeats are adjacent and dropped;
 // the nearest `limit` distinct entries become the pool.  Warp per node, the
-// 1024 slots held in registers (32 per lane, slot 32 r + lane in k[r]) and
-// sorted by a bitonic network: strides below 32 exchange across lanes by
-// shuffles, larger strides between a lane's own registers.
+// 1024 slots held in registers (32 per lane) and sorted by a bitonic network;
+// the distinct ones go through shared memory to be written in rows.
+// Instruction issue bounds it.  With the keys the other way round (32 r + lane)
+// 40 stages crossed lanes, 64 shuffles each: 400,003 rows, 16 tables 10.6 ms,
+// 5.8 now.
 static_assert(SEED_CAND == 1024, "the collect sort holds 32 keys per lane");
+constexpr int COLLECT_PITCH = SEED_CAND + SEED_CAND / 32;
 
 __device__ __forceinline__ uint64_t shfl_xor64(uint64_t v, int m) {
     const uint32_t lo = __shfl_xor_sync(KCNA_FULL, (uint32_t)v, m);
     const uint32_t hi = __shfl_xor_sync(KCNA_FULL, (uint32_t)(v >> 32), m);
-    return ((uint64_t)hi << 32) | lo;
-}
-__device__ __forceinline__ uint64_t shfl_idx64(uint64_t v, int src) {
-    const uint32_t lo = __shfl_sync(KCNA_FULL, (uint32_t)v, src);
-    const uint32_t hi = __shfl_sync(KCNA_FULL, (uint32_t)(v >> 32), src);
     return ((uint64_t)hi << 32) | lo;
 }
 __device__ __forceinline__ uint64_t shfl_up64(uint64_t v, int d) {
@@ -380,30 +378,29 @@ __device__ __forceinline__ uint64_t shfl_up64(uint64_t v, int d) {
     return ((uint64_t)hi << 32) | lo;
 }
 
-// Ascending bitonic sort of the 1024 keys k[r] (key index 32 r + lane).
+// Ascending bitonic sort of the 1024 keys k[r] (key index 32 lane + r): 40 of
+// the 55 stages stay in a lane's registers, 15 cross lanes.
 __device__ __forceinline__ void warp_sort1024(uint64_t (&k)[32], int lane) {
 #pragma unroll
     for (int size = 2; size <= 1024; size <<= 1) {
 #pragma unroll
         for (int j = size >> 1; j > 0; j >>= 1) {
-            if (j >= 32) { // partner in this lane's register r ^ (j / 32)
-                const int jr = j >> 5;
+            if (j >= 32) { // partner in lane ^ (j / 32), same register
+                const bool keep_min = ((lane & (j >> 5)) == 0) == ((lane & (size >> 5)) == 0);
 #pragma unroll
                 for (int r = 0; r < 32; ++r) {
-                    if (r & jr) continue;
-                    const bool asc = ((r * 32) & size) == 0;
-                    const uint64_t x = k[r], y = k[r | jr];
-                    const bool sw = asc ? x > y : x < y;
-                    k[r] = sw ? y : x;
-                    k[r | jr] = sw ? x : y;
+                    const uint64_t x = k[r], y = shfl_xor64(x, j >> 5);
+                    k[r] = (x < y) == keep_min ? x : y;
                 }
-            } else { // partner in lane ^ j, same register
+            } else { // partner in this lane's register r ^ j
 #pragma unroll
                 for (int r = 0; r < 32; ++r) {
-                    const bool asc = (((r * 32) | lane) & size) == 0;
-                    const uint64_t x = k[r], y = shfl_xor64(x, j);
-                    const bool keep_min = ((lane & j) == 0) == asc;
-                    k[r] = keep_min ? (y < x ? y : x) : (y > x ? y : x);
+                    if (r & j) continue;
+                    const bool asc = size < 32 ? (r & size) == 0 : (lane & (size >> 5)) == 0;
+                    const uint64_t x = k[r], y = k[r | j];
+                    const bool sw = (x > y) == asc;
+                    k[r] = sw ? y : x;
+                    k[r | j] = sw ? x : y;
                 }
             }
         }
@@ -414,31 +411,42 @@ __global__ void __launch_bounds__(128) seed_collect_kernel(const uint64_t *__res
                                                            uint32_t N, uint32_t cap, uint32_t limit,
                                                            uint64_t *__restrict__ pool,
                                                            uint32_t *__restrict__ pool_cnt) {
+    extern __shared__ __align__(16) uint64_t s_collect[]; // 4 warps x COLLECT_PITCH, entry e at e + e / 32
     const int w = threadIdx.x >> 5, lane = kcna_lane();
     const uint32_t i = blockIdx.x * 4 + w;
     if (i >= N) return;
+    uint64_t *so = s_collect + w * COLLECT_PITCH;
     const uint64_t *src = slots + (uint64_t)i * stride;
     uint64_t k[32];
 #pragma unroll
     for (int r = 0; r < 32; ++r) k[r] = src[32 * r + lane];
     warp_sort1024(k, lane);
-    uint64_t *pr = pool + (uint64_t)i * cap;
-    uint32_t cnt = 0;
-    uint64_t carry = KCNA_EMPTY_KEY;
+    // a lane holds 32 consecutive keys: the distinct ones move up by the number before them
+    unsigned m = 0;
+    uint64_t prev = shfl_up64(k[31], 1);
 #pragma unroll
     for (int r = 0; r < 32; ++r) {
-        const uint64_t v = k[r];
-        uint64_t prev = shfl_up64(v, 1);
-        if (lane == 0) prev = carry;
-        carry = shfl_idx64(v, 31);
-        const bool ok = v != KCNA_EMPTY_KEY && (r + lane == 0 || (prev >> 2) != (v >> 2));
-        const unsigned m = __ballot_sync(KCNA_FULL, ok);
-        const uint32_t pos = cnt + __popc(m & kcna_lanemask_lt());
-        if (ok && pos < limit) pr[pos] = v;
-        cnt += __popc(m);
+        const bool ok = k[r] != KCNA_EMPTY_KEY && ((lane == 0 && r == 0) || (prev >> 2) != (k[r] >> 2));
+        m |= (ok ? 1u : 0u) << r;
+        prev = k[r];
     }
-    const uint32_t keep = min(cnt, limit);
-    for (uint32_t e = keep + lane; e < cap; e += 32) pr[e] = KCNA_EMPTY_KEY;
+    uint32_t incl = __popc(m);
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(KCNA_FULL, incl, o);
+        if (lane >= o) incl += v;
+    }
+    const uint32_t cnt = __shfl_sync(KCNA_FULL, incl, 31), keep = min(cnt, limit);
+    uint32_t pos = incl - __popc(m);
+#pragma unroll
+    for (int r = 0; r < 32; ++r)
+        if ((m >> r) & 1u) {
+            so[pos + (pos >> 5)] = k[r];
+            ++pos;
+        }
+    __syncwarp();
+    uint64_t *pr = pool + (uint64_t)i * cap;
+    for (uint32_t e = lane; e < cap; e += 32) pr[e] = e < keep ? so[e + (e >> 5)] : KCNA_EMPTY_KEY;
     if (lane == 0) pool_cnt[i] = keep;
 }
 
@@ -710,7 +718,7 @@ kcna_status kcna_seed_learned(kcna_ctx *c, const kcna_params *p, kcna_stats *st)
             KCNA_TRY(band(RowsB16{c->Xh, (int)ld}));
         else
             KCNA_TRY(band(RowsF32{c->X, (int)ld}));
-        seed_collect_kernel<<<kcna_div_up(N, 4), 128, 0, s>>>(slots, stride, N, c->cap, limit, c->pool, c->pool_cnt);
+        seed_collect_kernel<<<kcna_div_up(N, 4), 128, 4 * COLLECT_PITCH * sizeof(uint64_t), s>>>(slots, stride, N, c->cap, limit, c->pool, c->pool_cnt);
     } else {
         const size_t srow = (size_t)4 * ld * 4;
         if (c->bf16_exact)
