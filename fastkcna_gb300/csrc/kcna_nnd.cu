@@ -252,8 +252,9 @@ __device__ void join_tiles(const JoinArgs &a, const R &rows, uint32_t node, cons
     }
 }
 
-// Join of the nodes with more rows than join_set_kernel's regions hold: block
-// per node, persistent over the queue (from the end of `list` down).
+// Join of the nodes with more rows than the regions of join_warp_kernel and
+// join_mid_kernel hold: block per node, persistent over the queue (from the end
+// of `list` down).
 template <class R>
 __global__ void __launch_bounds__(JT, 3) join_kernel(JoinArgs a, R rows, const uint32_t *__restrict__ list,
                                                      const uint32_t *__restrict__ cnt) {
