@@ -694,28 +694,31 @@ kcna_status kcna_get_pools(kcna_ctx *c, uint32_t *ids, float *dists, uint32_t *c
     // touched took 2 to 45 ms for the same entries, by how the pages came about,
     // so the host touches each page first, while the kernel runs: 2.3
     // ms fresh and 0.5 touched, always (10.8 and 7.2 to 8.8 with the host loop)
-    const uint64_t total = (uint64_t)c->n * cap;
+    // Nodes are taken in runs of at most 8 M entries, 64 MiB of device memory whatever the pools' size.
+    const uint32_t run = (uint32_t)std::min<uint64_t>(c->n, std::max<uint64_t>(1, (8u << 20) / cap));
     uint32_t *d_ids = nullptr, *d_cnt = nullptr;
     float *d_d = nullptr;
     kcna_status s = KCNA_OK;
-    if (ids) s = kcna_alloc(c, &d_ids, total, "pool ids");
-    if (s == KCNA_OK && dists) s = kcna_alloc(c, &d_d, total, "pool distances");
-    if (s == KCNA_OK && counts) s = kcna_alloc(c, &d_cnt, c->n, "pool counts");
-    if (s == KCNA_OK) {
-        unpack_pools_kernel<<<(unsigned)std::min<uint64_t>(kcna_div_up(c->n, 8), 65535u * 16u), 256, 0, c->stream>>>(
-            c->pool, c->pool_cnt, c->n, c->cap, cap, d_ids, d_d, d_cnt);
+    if (ids) s = kcna_alloc(c, &d_ids, (size_t)run * cap, "pool ids");
+    if (s == KCNA_OK && dists) s = kcna_alloc(c, &d_d, (size_t)run * cap, "pool distances");
+    if (s == KCNA_OK && counts) s = kcna_alloc(c, &d_cnt, run, "pool counts");
+    for (uint32_t i0 = 0; i0 < c->n && s == KCNA_OK; i0 += run) {
+        const uint32_t m = std::min(run, c->n - i0);
+        unpack_pools_kernel<<<kcna_div_up(m, 8), 256, 0, c->stream>>>(c->pool + (uint64_t)i0 * c->cap, c->pool_cnt + i0, m,
+                                                                      c->cap, cap, d_ids, d_d, d_cnt);
         KCNA_LAUNCHED(c);
         s = kcna_cuda_check(c, cudaGetLastError(), "unpack_pools");
+        auto get = [&](auto *dst, const void *src, size_t entries) {
+            if (s != KCNA_OK || !dst) return;
+            const size_t bytes = entries * 4;
+            volatile unsigned char *p = reinterpret_cast<unsigned char *>(dst);
+            for (size_t i = 0; i < bytes; i += 4096 - ((uintptr_t)(p + i) & 4095)) p[i] = 0;
+            s = kcna_cuda_check(c, cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, c->stream), "d2h");
+        };
+        get(ids ? ids + (uint64_t)i0 * cap : nullptr, d_ids, (size_t)m * cap);
+        get(dists ? dists + (uint64_t)i0 * cap : nullptr, d_d, (size_t)m * cap);
+        get(counts ? counts + i0 : nullptr, d_cnt, m);
     }
-    auto get = [&](void *dst, const void *src, size_t bytes) {
-        if (s != KCNA_OK || !dst) return;
-        volatile unsigned char *p = static_cast<unsigned char *>(dst);
-        for (size_t i = 0; i < bytes; i += 4096 - ((uintptr_t)(p + i) & 4095)) p[i] = 0;
-        s = kcna_cuda_check(c, cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, c->stream), "d2h");
-    };
-    get(ids, d_ids, total * 4);
-    get(dists, d_d, total * 4);
-    get(counts, d_cnt, (size_t)c->n * 4);
     if (s == KCNA_OK) s = kcna_cuda_check(c, cudaStreamSynchronize(c->stream), "sync");
     kcna_release(c, d_ids);
     kcna_release(c, d_d);
