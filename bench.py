@@ -316,13 +316,13 @@ def roofline(st, hbm_gbs, ld, n, search_k, tensor_tflops=None):
         "merge": st["cand_merged"] * 8 + st["pool_entries_merged"] * 16,
         "prune": pruned * c * ld * rb,
     }
-    kernels = {"join": "join_tc_kernel" if st["gram_tc"] else "join_kernel", "merge": "merge_warp_kernel",
+    kernels = {"join": "join_tc_kernel" if st["gram_tc"] else "join_warp_kernel", "merge": "merge_set_kernel",
                "prune": "prune_gram_kernel" if st.get("prune_tc") else "prune_kernel"}
     limiters = {
         "join": "scattered 16-byte candidate-slot stores and the TMEM re-read of the write pass (latency, LSU)",
-        "merge": "shared-memory latency: binary search of every candidate in the node's pool (bank conflicts)",
+        "merge": "shared-memory latency: lookup of every candidate in the node's pool and hash table",
         "prune": "issue slots of the mask-building warps; tensor pipe about 30 % busy" if st.get("prune_tc")
-        else "latency of the sequential occlusion scan",
+        else "issue slots of the distance chains",
     }
     name = max(models, key=lambda k: ph.get(k, 0.0))
     ms, nl = ph[name], max(launches[name], 1)
