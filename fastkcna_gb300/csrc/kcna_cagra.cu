@@ -35,7 +35,7 @@
 //                       in closed form.
 // A node's work is small (K = 64: 4,096 look-ups, some 32 reverse keys), so a
 // block of 256 threads per node spent its time at barriers: 2.8 and 2.1 ms for
-// 150,007 nodes at K = 64, 1.6 and 0.3 with a warp per node.
+// 150,007 nodes at K = 64, 1.6 and 0.3 with a warp per node (route: up to K = 64).
 #include <algorithm>
 
 #include "kcna_internal.h"
@@ -53,29 +53,33 @@ __device__ __forceinline__ uint32_t cg_hash(uint32_t id) { return (id * 0x9E3779
 // in-degrees; NT threads per node.  Shared, per node: sort keys[P2], ids[K],
 // route[K], table keys[HS], table ranks[HS] (P2 = K rounded up to a power of
 // two).  The K x K look-ups are what it does, most of them misses, and a warp
-// takes as many steps as its unluckiest lane: HS = 8 P2 slots (an eighth full)
-// for the warp version, where 2 P2 took 3.5 ms for 150,007 nodes at K = 64.
-constexpr uint32_t CG_WARP_K = 128;
-__host__ __device__ constexpr uint32_t cagra_slots(uint32_t K, uint32_t P2) { return K <= CG_WARP_K ? 8 * P2 : 2 * P2; }
-__host__ __device__ constexpr size_t cagra_route_bytes(uint32_t K, uint32_t P2) {
-    return (size_t)P2 * 8 + (((size_t)K * 8 + 15) & ~(size_t)15) + (size_t)cagra_slots(K, P2) * 6;
+// takes as many steps as its unluckiest lane: HS = 8 P2 slots, an eighth full
+// (2 P2: 3.5 ms for 150,007 nodes at K = 64 against 1.6; 28 against 19 ms a
+// call at K = 200, 212 against 121 for 40,000 nodes at K = 1,000).
+// Warp or block per node: whole calls for 150,007 nodes, warp / block, K = 64
+// 2.26 / 2.82 ms, K = 100 8.3 / 6.0, for 11,132 nodes 0.30 / 0.32 and 0.81 /
+// 0.55: from P2 = 128 on the tables of eight warps leave 24 warps an SM.
+constexpr uint32_t CG_WARP_K = 64;
+constexpr uint32_t cagra_slots(uint32_t P2) { return 8 * P2; }
+__host__ __device__ constexpr size_t cagra_route_bytes(uint32_t K, uint32_t P2, uint32_t HS) {
+    return (size_t)P2 * 8 + (((size_t)K * 8 + 15) & ~(size_t)15) + (size_t)HS * 6;
 }
 
 template <int NT>
 __global__ void __launch_bounds__(CG_THREADS) cagra_route_kernel(const uint64_t *__restrict__ pool,
                                                                  const uint32_t *__restrict__ pool_cnt, uint32_t cap,
                                                                  uint32_t N, uint32_t K, uint32_t PK, uint32_t P2,
-                                                                 uint16_t *__restrict__ fwd, uint32_t *__restrict__ indeg,
+                                                                 uint32_t HS, uint16_t *__restrict__ fwd,
+                                                                 uint32_t *__restrict__ indeg,
                                                                  int *err) {
     extern __shared__ __align__(16) unsigned char smem[];
     constexpr int NODES = CG_THREADS / NT, NW = NT / 32; // per block; warps per node
     const int tid = threadIdx.x % NT, warp = tid >> 5, lane = tid & 31;
-    unsigned char *base = smem + (threadIdx.x / NT) * cagra_route_bytes(K, P2);
+    unsigned char *base = smem + (threadIdx.x / NT) * cagra_route_bytes(K, P2, HS);
     uint64_t *skey = reinterpret_cast<uint64_t *>(base);        // P2
     uint32_t *ids = reinterpret_cast<uint32_t *>(skey + P2);    // K
     uint32_t *route = ids + K;                                  // K
-    const uint32_t HS = cagra_slots(K, P2);
-    uint32_t *hkey = reinterpret_cast<uint32_t *>(base + cagra_route_bytes(K, P2) - (size_t)HS * 6); // HS
+    uint32_t *hkey = reinterpret_cast<uint32_t *>(base + cagra_route_bytes(K, P2, HS) - (size_t)HS * 6); // HS
     uint16_t *hval = reinterpret_cast<uint16_t *>(hkey + HS);   // HS
     auto sync = [] {
         if (NT == 32)
@@ -314,7 +318,8 @@ kcna_status kcna_cagra_prune(kcna_ctx *c, const kcna_params *p) {
     cudaMemsetAsync(cursor, 0, (size_t)N * 4, c->stream);
     const uint32_t sms = (uint32_t)std::max(c->num_sms, 1);
     auto route = [&](auto kern, uint32_t nodes) -> kcna_status { // nodes per block
-        const size_t sm = cagra_route_bytes(K, P2) * nodes;
+        const uint32_t HS = cagra_slots(P2);
+        const size_t sm = cagra_route_bytes(K, P2, HS) * nodes;
         int per_sm = 0;
         KCNA_TRY(kcna_cuda_check(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                          (int)std::max<size_t>(sm, 48 * 1024)),
@@ -322,7 +327,7 @@ kcna_status kcna_cagra_prune(kcna_ctx *c, const kcna_params *p) {
         KCNA_TRY(kcna_cuda_check(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, CG_THREADS, sm),
                                  "cagra occupancy"));
         const uint32_t grid = std::min(kcna_div_up(N, nodes), sms * (uint32_t)std::max(per_sm, 1));
-        kern<<<grid, CG_THREADS, sm, c->stream>>>(c->pool, c->pool_cnt, c->cap, N, K, PK, P2, fwd, indeg, c->d_err);
+        kern<<<grid, CG_THREADS, sm, c->stream>>>(c->pool, c->pool_cnt, c->cap, N, K, PK, P2, HS, fwd, indeg, c->d_err);
         KCNA_LAUNCHED(c);
         return kcna_cuda_check(c, cudaGetLastError(), "cagra_route_kernel");
     };
