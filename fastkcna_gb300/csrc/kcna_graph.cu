@@ -875,7 +875,8 @@ __global__ void __launch_bounds__(BW * 32, 5) beam_search_kernel(const float *__
                     }
                     float dist = 0.f;
                     if (fresh) dist = beam_l2(reinterpret_cast<const float4 *>(X + (uint64_t)id * ld), qrow, nv);
-                    fresh = fresh && dist < kcna_key_dist(pool[Lc - 1]);
+                    // as words: a NaN distance is the farthest, so a NaN start entry gives way to any other
+                    fresh = fresh && __float_as_uint(dist) < (uint32_t)(pool[Lc - 1] >> 32);
                     const int c = __popc(__ballot_sync(KCNA_FULL, fresh));
                     if (!c) continue;
                     // nearest first, equal distances in row order
