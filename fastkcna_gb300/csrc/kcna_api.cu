@@ -416,6 +416,7 @@ kcna_status kcna_create(kcna_ctx **out, int device) {
     kcna_status s = bind(c);
     if (s == KCNA_OK) s = kcna_cuda_check(c, cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking), "stream");
     if (s == KCNA_OK) s = kcna_cuda_check(c, cudaDeviceGetAttribute(&c->num_sms, cudaDevAttrMultiProcessorCount, device), "attr");
+    if (s == KCNA_OK) s = kcna_cuda_check(c, cudaDeviceGetAttribute(&c->smem_block, cudaDevAttrMaxSharedMemoryPerBlockOptin, device), "attr");
     if (s == KCNA_OK) s = kcna_alloc(c, &c->d_err, 1, "error word");
     if (s == KCNA_OK) s = kcna_alloc(c, &c->counters, 64, "counters");
     if (s == KCNA_OK) s = kcna_cuda_check(c, cudaMemset(c->d_err, 0, 4), "memset");

@@ -321,9 +321,7 @@ kcna_status kcna_cagra_prune(kcna_ctx *c, const kcna_params *p) {
         const uint32_t HS = cagra_slots(P2);
         const size_t sm = cagra_route_bytes(K, P2, HS) * nodes;
         int per_sm = 0;
-        KCNA_TRY(kcna_cuda_check(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                         (int)std::max<size_t>(sm, 48 * 1024)),
-                                 "cagra smem attr"));
+        KCNA_TRY(kcna_allow_smem(c, kern, sm, "cagra smem attr"));
         KCNA_TRY(kcna_cuda_check(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, CG_THREADS, sm),
                                  "cagra occupancy"));
         const uint32_t grid = std::min(kcna_div_up(N, nodes), sms * (uint32_t)std::max(per_sm, 1));

@@ -1583,9 +1583,7 @@ kcna_status kcna_prune_all(kcna_ctx *c, const kcna_params *p, int kind, uint64_t
                 c->g_dist, c->g_deg, c->W, c->counters + 16, n_items, list);
         else if ((int)c->ld >= PRUNE_STAGED_MIN && (int)c->ld <= PRUNE_STAGED_MAX) {
             const size_t ssm = prune_staged_bytes((int)c->ld) + (size_t)2 * range * 4;
-            KCNA_TRY(kcna_cuda_check(c, cudaFuncSetAttribute(prune_kernel<true, RowsF32>,
-                                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ssm),
-                                     "prune smem attr"));
+            KCNA_TRY(kcna_allow_smem(c, prune_kernel<true, RowsF32>, ssm, "prune smem attr"));
             prune_kernel<true><<<n_items, 32, ssm, c->stream>>>(
                 RowsF32{c->X, (int)c->ld}, c->n, c->pool, c->pool_cnt, c->cap, rule, (int)range, maxc, c->g_ids,
                 c->g_dist, c->g_deg, c->W, c->counters + 16, n_items, list);
@@ -1762,9 +1760,7 @@ kcna_status kcna_search_device(kcna_ctx *c, const float *dQ, uint32_t m, const u
     void *vis = nullptr;
     KCNA_TRY(kcna_scratch2(c, slots * vwords * 4, &vis));
     size_t sm = (size_t)BW * (L + 1) * 8 + (c->ld <= (uint32_t)BEAM_STAGE ? (size_t)BW * c->ld * 4 : 0);
-    KCNA_TRY(kcna_cuda_check(c, cudaFuncSetAttribute(beam_search_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                     (int)std::max<size_t>(sm, 48 * 1024)),
-                             "attr"));
+    KCNA_TRY(kcna_allow_smem(c, beam_search_kernel, sm, "beam search smem attr"));
     beam_search_kernel<<<blocks, BW * 32, sm, c->stream>>>(c->X, (int)c->ld, c->n, c->g_ids, c->g_deg, c->W, dQ, m,
                                                            d_init, (int)L, (int)k, (uint32_t *)vis, vwords, d_out_ids,
                                                            d_out_d);

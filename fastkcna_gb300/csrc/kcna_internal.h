@@ -19,6 +19,7 @@
 struct kcna_ctx {
     int device = 0;
     int num_sms = 0;
+    int smem_block = 0; // shared memory a block may have, in bytes
     cudaStream_t stream = nullptr;
     std::string err;
     // background file writer (kcna_write_nsg_async): one write in flight; its
@@ -175,6 +176,17 @@ kcna_status kcna_alloc(kcna_ctx *c, T **p, size_t count, const char *what) {
         if (_s != KCNA_OK) return _s;                \
     } while (0)
 #define KCNA_LAUNCHED(c) ((c)->launches++)
+// Allows `kern` up to `bytes` of dynamic shared memory a block.  The limit is the
+// kernel's, for every thread of the process, and another thread's context may set
+// it between this call and the launch: so it is always the most the device has,
+// whatever this launch needs.
+template <class Kern> kcna_status kcna_allow_smem(kcna_ctx *c, Kern kern, size_t bytes, const char *what) {
+    cudaFuncAttributes fa;
+    KCNA_TRY(kcna_cuda_check(c, cudaFuncGetAttributes(&fa, kern), what));
+    const size_t most = (size_t)c->smem_block - fa.sharedSizeBytes;
+    if (bytes > most) return kcna_fail(c, KCNA_E_CUDA, std::string(what) + ": more shared memory than a block has");
+    return kcna_cuda_check(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most), what);
+}
 double kcna_now();
 void kcna_log(kcna_ctx *c, const kcna_params *p, const char *fmt, ...);
 

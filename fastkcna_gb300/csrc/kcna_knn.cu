@@ -416,18 +416,10 @@ static kcna_status knn_bounded(kcna_ctx *c, const float *dQ, uint32_t m, const u
     if (st == KCNA_OK) st = kcna_alloc(c, &words, 2 * (size_t)batch + 1, "k-NN bounds");
     const bool cached = s <= SEL_CACHE;
     const size_t fsm = KNN_CAP * 8 + (screened ? (size_t)c->ld * 4 : 0);
-    if (st == KCNA_OK && cached)
-        st = kcna_cuda_check(c, cudaFuncSetAttribute(knn_bound_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                     (int)(SEL_CACHE * 4)),
-                             "knn smem attr");
+    if (st == KCNA_OK && cached) st = kcna_allow_smem(c, knn_bound_kernel<true>, (size_t)s * 4, "knn smem attr");
     if (st == KCNA_OK)
-        st = kcna_cuda_check(c, cudaFuncSetAttribute(knn_final_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                     (int)fsm),
-                             "knn smem attr");
-    if (st == KCNA_OK)
-        st = kcna_cuda_check(c, cudaFuncSetAttribute(knn_final_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                     (int)fsm),
-                             "knn smem attr");
+        st = screened ? kcna_allow_smem(c, knn_final_kernel<true>, fsm, "knn smem attr")
+                      : kcna_allow_smem(c, knn_final_kernel<false>, fsm, "knn smem attr");
     for (uint32_t q0 = 0; q0 < m && st == KCNA_OK; q0 += batch) {
         const uint32_t mb = std::min(batch, m - q0);
         void *buf = nullptr; // asked for each time: knn_all below may move the scratch

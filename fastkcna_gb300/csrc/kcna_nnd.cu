@@ -1581,12 +1581,8 @@ kcna_status kcna_nnd_join(kcna_ctx *c, const kcna_params *p, int iter, uint64_t 
     a.capB = c->fwd_old_cap + std::min(p->R, c->RB);
     a.err = c->d_err;
     size_t sm = join_smem_bytes(a.capA, a.capB);
-    KCNA_TRY(kcna_cuda_check(c, cudaFuncSetAttribute(join_kernel<RowsF32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                     (int)std::max<size_t>(sm, 48 * 1024)),
-                             "join smem attr"));
-    KCNA_TRY(kcna_cuda_check(c, cudaFuncSetAttribute(join_kernel<RowsB16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                     (int)std::max<size_t>(sm, 48 * 1024)),
-                             "join smem attr"));
+    KCNA_TRY(kcna_allow_smem(c, join_kernel<RowsF32>, sm, "join smem attr"));
+    KCNA_TRY(kcna_allow_smem(c, join_kernel<RowsB16>, sm, "join smem attr"));
     KCNA_TRY(kcna_cuda_check(c, cudaMemsetAsync(c->counters, 0, 8 * 8, c->stream), "memset"));
     // found (src/kgraph.cpp:1104,1116): cleared for every node, then set by the
     // merge for the joiners whose candidates it inserts below K
@@ -1604,9 +1600,7 @@ kcna_status kcna_nnd_join(kcna_ctx *c, const kcna_params *p, int iter, uint64_t 
                 ht = 0;
                 rs = (size_t)8 * c->ld * 4;
             }
-            KCNA_TRY(kcna_cuda_check(c, cudaFuncSetAttribute(rescore_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                             (int)std::max<size_t>(rs, 48 * 1024)),
-                                     "rescore smem attr"));
+            KCNA_TRY(kcna_allow_smem(c, rescore_kernel, rs, "rescore smem attr"));
             rescore_kernel<<<kcna_div_up(c->n, 8), 256, rs, c->stream>>>(
                 c->X, (int)c->ld, c->n, c->cand, c->cand_cnt, c->CB, c->radius, c->pool, c->pool_cnt, c->cap, limit,
                 ht, c->counters + 13, c->counters + 14);
@@ -1619,9 +1613,7 @@ kcna_status kcna_nnd_join(kcna_ctx *c, const kcna_params *p, int iter, uint64_t 
             const uint32_t sms = (uint32_t)std::max(c->num_sms, 1);
             auto grid = [&](auto kern, int threads, size_t smem, uint32_t *out) -> kcna_status {
                 int per_sm = 0;
-                KCNA_TRY(kcna_cuda_check(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                                 (int)std::max<size_t>(smem, 48 * 1024)),
-                                         "join smem attr"));
+                KCNA_TRY(kcna_allow_smem(c, kern, smem, "join smem attr"));
                 KCNA_TRY(kcna_cuda_check(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem),
                                          "join occupancy"));
                 *out = std::min(kcna_div_up(c->n, threads == JM_NT ? 1 : threads / 32), sms * (uint32_t)std::max(per_sm, 1));
@@ -1671,13 +1663,9 @@ kcna_status kcna_merge(kcna_ctx *c, uint32_t limit, uint32_t K, uint64_t *overfl
     a.found = c->found;
     a.n_nodes = c->n;
     size_t sm = merge_smem_bytes(c->cap, c->CB);
-    KCNA_TRY(kcna_cuda_check(c, cudaFuncSetAttribute(merge_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                     (int)std::max<size_t>(sm, 48 * 1024)),
-                             "merge smem attr"));
+    KCNA_TRY(kcna_allow_smem(c, merge_kernel, sm, "merge smem attr"));
     auto launch = [&](auto kern, int threads, uint32_t per_block, size_t smem) -> kcna_status {
-        KCNA_TRY(kcna_cuda_check(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                         (int)std::max<size_t>(smem, 48 * 1024)),
-                                 "merge smem attr"));
+        KCNA_TRY(kcna_allow_smem(c, kern, smem, "merge smem attr"));
         int per_sm = 0;
         KCNA_TRY(kcna_cuda_check(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem),
                                  "merge occupancy"));
@@ -1723,9 +1711,7 @@ kcna_status kcna_nnd_sample(kcna_ctx *c, const kcna_params *p, int iter) {
                                                               c->rold, c->rold_cnt, c->RB, c->counters);
     KCNA_LAUNCHED(c);
     const int P = kcna_pow2_ceil((int)c->RB);
-    KCNA_TRY(kcna_cuda_check(c, cudaFuncSetAttribute(select_reverse_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                     SEL_WARPS * P * 8),
-                             "select smem attr"));
+    KCNA_TRY(kcna_allow_smem(c, select_reverse_kernel, (size_t)SEL_WARPS * P * 8, "select smem attr"));
     select_reverse_kernel<<<kcna_div_up(2ull * c->n, SEL_WARPS), SEL_WARPS * 32, (size_t)SEL_WARPS * P * 8, s>>>(
         c->rnew, c->rnew_cnt, c->rold, c->rold_cnt, c->n, c->RB, p->R, p->seed, (uint32_t)iter, P);
     KCNA_LAUNCHED(c);
@@ -1796,10 +1782,7 @@ kcna_status kcna_control_recall(kcna_ctx *c, uint32_t K, float *recall) {
     KCNA_TRY(kcna_phase_begin(c));
     KCNA_TRY(kcna_cuda_check(c, cudaMemsetAsync(c->counters + 8, 0, 8, c->stream), "memset"));
     size_t sm = (size_t)kcna_pow2_ceil((int)K) * 8;
-    KCNA_TRY(kcna_cuda_check(c, cudaFuncSetAttribute(control_recall_kernel,
-                                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                     (int)std::max<size_t>(sm, 48 * 1024)),
-                             "attr"));
+    KCNA_TRY(kcna_allow_smem(c, control_recall_kernel, sm, "control recall smem attr"));
     control_recall_kernel<<<C, 256, sm, c->stream>>>(c->pool, c->pool_cnt, c->cap, c->d_controls, c->d_control_knn,
                                                      c->control_k, K, c->counters + 8);
     KCNA_LAUNCHED(c);

@@ -187,9 +187,7 @@ kcna_status kcna_pool_search_run(kcna_ctx *c, const kcna_params *p, uint32_t max
     if (sm > 200 * 1024) return kcna_fail(c, KCNA_E_ARG, "pool search: MAXL too large for shared memory");
     auto launch = [&](auto rows) -> kcna_status {
         auto kern = pool_search_kernel<decltype(rows)>;
-        KCNA_TRY(kcna_cuda_check(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                         (int)std::max<size_t>(sm, 48 * 1024)),
-                                 "pool search smem attr"));
+        KCNA_TRY(kcna_allow_smem(c, kern, sm, "pool search smem attr"));
         int per_sm = 0;
         KCNA_TRY(kcna_cuda_check(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, PS_WARPS * 32, sm),
                                  "pool search occupancy"));

@@ -706,10 +706,7 @@ kcna_status kcna_seed_learned(kcna_ctx *c, const kcna_params *p, kcna_stats *st)
         KCNA_TRY(kcna_cuda_check(c, cudaMemset2DAsync(slots, (size_t)stride * 8, 0xFF, (size_t)SEED_CAND * 8, N, s),
                                  "memset"));
         auto band = [&](auto rows) -> kcna_status {
-            KCNA_TRY(kcna_cuda_check(c, cudaFuncSetAttribute(seed_band_kernel<decltype(rows)>,
-                                                             cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                             (int)band_smem),
-                                     "seed band smem attr"));
+            KCNA_TRY(kcna_allow_smem(c, seed_band_kernel<decltype(rows)>, band_smem, "seed band smem attr"));
             seed_band_kernel<<<dim3(kcna_div_up(N, 32 * BAND_WARPS), SEED_TABLES), BAND_WARPS * 32, band_smem, s>>>(
                 rows, N, order, slots, stride, c->counters + 30);
             return launch_ok(c, "seed band");
