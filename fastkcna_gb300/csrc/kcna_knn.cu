@@ -18,19 +18,21 @@
 // than computing it (7.3 of 17.7 ms for 1,000 queries against 1,000,000 x 128
 // rows), and the computation itself can be spared for all but a few thousand
 // rows per query:
-//   1. distances to every (n / s)-th row; the max(k, 32)-th smallest of them is
-//      a bound T on the k-th smallest of all;
+//   1. distances to s rows, one drawn from every n / s consecutive ones (not
+//      every (n / s)-th: in rows stored with a period, those can all belong to
+//      a few clusters, and the lists of the other clusters' queries overflow);
+//      the max(k, 32)-th smallest of them is a bound T on the k-th smallest of all;
 //   2. the rows that may lie within T: screened on tensor cores where the work
 //      is large and d <= 128 (kcna_knn_tc.cu), else by the tiled kernel, which
 //      then keeps a pair only if its distance is at most T;
 //   3. per query, canonical distances of the rows handed on (where 2 screened)
 //      and the selection among them.
-// s is chosen so that about 4,096 rows remain; a query whose list of 8,192
-// overflows, or comes up short (NaN), is done again the first way.
+// s is chosen so that about 4,096 rows remain; the queries whose lists of 8,192
+// overflow, or come up short (NaN), are gathered and done again together the
+// first way.
 // The size above: 2.05 ms a call (0.26 sample, 0.08 bounds, 1.07 screen, 0.58
 // selection).
 #include <algorithm>
-#include <vector>
 
 #include "kcna_internal.h"
 #include "kcna_sort.cuh"
@@ -39,9 +41,15 @@ namespace {
 
 constexpr int TQ = 32, TB = 128, KC = 32, KCP = KC + 4;
 
-// FILTER: instead of writing every distance, append (distance, id) to the
-// query's list when the distance is at most thresh[q].
-// Base row b is row b * stride of X.
+// DT_ALL: every distance is written.  DT_FILTER: instead, (distance, id) is
+// appended to the query's list when the distance is at most thresh[q].
+// DT_SAMPLE: as DT_ALL, base row b being row sample_row(b, stride) of X.
+enum { DT_ALL, DT_FILTER, DT_SAMPLE };
+__device__ __forceinline__ uint64_t sample_row(uint64_t b, uint32_t stride) { // one of the rows [b, b + 1) * stride
+    uint32_t h = (uint32_t)b * 0x9E3779B1u;
+    h = (h ^ (h >> 15)) * 0x85EBCA77u;
+    return b * stride + __umulhi(h ^ (h >> 13), stride);
+}
 struct DistOut {
     float *D;
     uint64_t ldD;
@@ -49,7 +57,7 @@ struct DistOut {
     uint64_t *cand;
     uint32_t *cnt, cap;
 };
-template <bool FILTER>
+template <int MODE>
 __global__ void __launch_bounds__(256) dist_tile_kernel(const float *__restrict__ Q, uint32_t m,
                                                         const float *__restrict__ X, uint32_t n, uint32_t stride,
                                                         int ld, const uint32_t *__restrict__ q_self, DistOut o) {
@@ -63,6 +71,10 @@ __global__ void __launch_bounds__(256) dist_tile_kernel(const float *__restrict_
     for (int i = 0; i < 4; ++i)
 #pragma unroll
         for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+    auto row_of = [&](uint64_t b) { return MODE == DT_SAMPLE ? sample_row(b, stride) : b; };
+    uint64_t at[4]; // this thread's rows of a chunk
+#pragma unroll
+    for (int s = 0; s < 4; ++s) at[s] = row_of(b0 + ((tid + s * 256) >> 3));
 
     for (int k0 = 0; k0 < ld; k0 += KC) {
         {   // Q chunk: 32 rows x 32 floats, one float4 per thread
@@ -76,7 +88,7 @@ __global__ void __launch_bounds__(256) dist_tile_kernel(const float *__restrict_
             int idx = tid + s * 256;
             int r = idx >> 3, c = (idx & 7) * 4;
             float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (b0 + r < n && k0 + c < ld) v = __ldg(reinterpret_cast<const float4 *>(X + (b0 + r) * stride * ld + k0 + c));
+            if (b0 + r < n && k0 + c < ld) v = __ldg(reinterpret_cast<const float4 *>(X + at[s] * ld + k0 + c));
             *reinterpret_cast<float4 *>(&Xs[r][c]) = v;
         }
         __syncthreads();
@@ -103,12 +115,13 @@ __global__ void __launch_bounds__(256) dist_tile_kernel(const float *__restrict_
         for (int j = 0; j < 4; ++j) {
             uint64_t b = b0 + tx + 32 * j;
             if (b >= n) continue;
-            const bool own = b * stride == self;
-            if (!FILTER) {
+            const uint64_t row = row_of(b);
+            const bool own = row == self;
+            if (MODE != DT_FILTER) {
                 o.D[(uint64_t)q * o.ldD + b] = own ? __uint_as_float(0x7F800000u) : acc[i][j];
             } else if (!own && __float_as_uint(acc[i][j]) <= o.thresh[q]) {
                 const uint32_t p = atomicAdd(o.cnt + q, 1u);
-                if (p < o.cap) o.cand[(uint64_t)q * o.cap + p] = ((uint64_t)__float_as_uint(acc[i][j]) << 32) | (b * stride);
+                if (p < o.cap) o.cand[(uint64_t)q * o.cap + p] = ((uint64_t)__float_as_uint(acc[i][j]) << 32) | row;
             }
         }
     }
@@ -308,7 +321,7 @@ __global__ void __launch_bounds__(SEL_T) knn_bound_kernel(const float *__restric
 
 // Selection among the rows handed on; SCREENED: they are ids only, and their
 // canonical distances are computed here, a row per thread, sixteen loads in
-// flight.  A query with too many or too few counts in *redo.
+// flight.  A query with too many or too few goes to redo[1 ..], counted in redo[0].
 template <bool SCREENED>
 __global__ void __launch_bounds__(SEL_T) knn_final_kernel(const float *__restrict__ Q, const float *__restrict__ X,
                                                           int ld, const uint32_t *__restrict__ q_self,
@@ -325,7 +338,7 @@ __global__ void __launch_bounds__(SEL_T) knn_final_kernel(const float *__restric
     const uint32_t q = blockIdx.x, n = cnt[q];
     const uint32_t self = q_self ? q_self[q] : KCNA_NONE;
     if (n > KNN_CAP || n < k) {
-        if (threadIdx.x == 0) atomicAdd(redo, 1u);
+        if (threadIdx.x == 0) redo[1 + atomicAdd(redo, 1u)] = q;
         return;
     }
     if (SCREENED) {
@@ -369,6 +382,22 @@ __global__ void gather_rows_kernel(const float *__restrict__ X, int ld, const ui
     reinterpret_cast<float4 *>(dst)[t] = reinterpret_cast<const float4 *>(X + (uint64_t)id * ld)[c];
 }
 
+// Entry i of the queries done again: the query to exclude for it, or its k results to their place.
+__global__ void redo_self_kernel(const uint32_t *__restrict__ list, uint32_t m, const uint32_t *__restrict__ q_self,
+                                 uint32_t *__restrict__ out) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < m) out[i] = q_self[list[i]];
+}
+__global__ void redo_place_kernel(const uint32_t *__restrict__ list, uint64_t entries, uint32_t k,
+                                  const uint32_t *__restrict__ ids, const float *__restrict__ d,
+                                  uint32_t *__restrict__ out_ids, float *__restrict__ out_d) {
+    const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= entries) return;
+    const uint64_t to = (uint64_t)list[t / k] * k + t % k;
+    out_ids[to] = ids[t];
+    out_d[to] = d[t];
+}
+
 } // namespace
 
 kcna_status kcna_gather_rows(kcna_ctx *c, const uint32_t *d_ids, uint32_t m, float *dst) {
@@ -393,7 +422,7 @@ static kcna_status knn_all(kcna_ctx *c, const float *dQ, uint32_t m, const uint3
     for (uint32_t q0 = 0; q0 < m; q0 += batch) {
         uint32_t mb = std::min(batch, m - q0);
         dim3 grid(kcna_div_up(c->n, TB), kcna_div_up(mb, TQ));
-        dist_tile_kernel<false><<<grid, 256, 0, c->stream>>>(dQ + (uint64_t)q0 * c->ld, mb, c->X, c->n, 1, (int)c->ld,
+        dist_tile_kernel<DT_ALL><<<grid, 256, 0, c->stream>>>(dQ + (uint64_t)q0 * c->ld, mb, c->X, c->n, 1, (int)c->ld,
                                                              q_self ? q_self + q0 : nullptr,
                                                              DistOut{D, c->n, nullptr, nullptr, nullptr, 0});
         KCNA_LAUNCHED(c);
@@ -404,6 +433,42 @@ static kcna_status knn_all(kcna_ctx *c, const float *dQ, uint32_t m, const uint3
     return KCNA_OK;
 }
 
+// The m queries of `list` (of n_q) done again the first way, together: one by
+// one, each was a pass over the base with 31 of a tile's 32 query places empty
+// (60 of 1,000 queries, 200,000 x 64 rows: 5.6 ms a call against 2.2 for doing
+// all 1,000 again, 1.2 so).
+static kcna_status knn_redo(kcna_ctx *c, const float *dQ, uint32_t n_q, const uint32_t *q_self, uint32_t k,
+                            const uint32_t *list, uint32_t m, uint32_t *d_out_ids, float *d_out_d) {
+    if (m == n_q) return knn_all(c, dQ, n_q, q_self, k, d_out_ids, d_out_d);
+    float *q = nullptr, *od = nullptr;
+    uint32_t *self = nullptr, *oi = nullptr;
+    kcna_status st = kcna_alloc(c, &q, (size_t)m * c->ld, "queries done again");
+    if (st == KCNA_OK && q_self) st = kcna_alloc(c, &self, m, "queries done again");
+    if (st == KCNA_OK) st = kcna_alloc(c, &oi, (size_t)m * k, "queries done again");
+    if (st == KCNA_OK) st = kcna_alloc(c, &od, (size_t)m * k, "queries done again");
+    if (st == KCNA_OK) {
+        gather_rows_kernel<<<kcna_div_up((uint64_t)m * (c->ld / 4), 256), 256, 0, c->stream>>>(dQ, (int)c->ld, list, m, n_q,
+                                                                                              q, c->d_err);
+        KCNA_LAUNCHED(c);
+        if (self) {
+            redo_self_kernel<<<kcna_div_up(m, 256), 256, 0, c->stream>>>(list, m, q_self, self);
+            KCNA_LAUNCHED(c);
+        }
+        st = knn_all(c, q, m, self, k, oi, od);
+    }
+    if (st == KCNA_OK) {
+        redo_place_kernel<<<kcna_div_up((uint64_t)m * k, 256), 256, 0, c->stream>>>(list, (uint64_t)m * k, k, oi, od,
+                                                                                    d_out_ids, d_out_d);
+        KCNA_LAUNCHED(c);
+        st = kcna_cuda_check(c, cudaGetLastError(), "redo_place_kernel");
+    }
+    kcna_release(c, q); // later users run behind these kernels on the context's stream
+    kcna_release(c, self);
+    kcna_release(c, oi);
+    kcna_release(c, od);
+    return st;
+}
+
 // A bound per query from a sample, the rows that may lie within it, selection among those.
 static kcna_status knn_bounded(kcna_ctx *c, const float *dQ, uint32_t m, const uint32_t *q_self, uint32_t k, uint32_t s,
                                uint32_t *d_out_ids, float *d_out_d) {
@@ -411,9 +476,9 @@ static kcna_status knn_bounded(kcna_ctx *c, const float *dQ, uint32_t m, const u
     // the tensor-core screen pays from about 0.1 ms of FP32 work on
     const bool screened = c->ld <= 128 && (uint64_t)m * c->n * c->ld >= (1ull << 30);
     uint64_t *cand = nullptr;
-    uint32_t *words = nullptr; // bounds, counts, and the number of queries to do again
+    uint32_t *words = nullptr; // bounds, counts, and the queries to do again behind their number
     kcna_status st = kcna_alloc(c, &cand, ((uint64_t)batch * KNN_CAP + (screened ? 1 : 0)) / (screened ? 2 : 1), "k-NN lists");
-    if (st == KCNA_OK) st = kcna_alloc(c, &words, 2 * (size_t)batch + 1, "k-NN bounds");
+    if (st == KCNA_OK) st = kcna_alloc(c, &words, 3 * (size_t)batch + 1, "k-NN bounds");
     const bool cached = s <= SEL_CACHE;
     const size_t fsm = KNN_CAP * 8 + (screened ? (size_t)c->ld * 4 : 0);
     if (st == KCNA_OK && cached) st = kcna_allow_smem(c, knn_bound_kernel<true>, (size_t)s * 4, "knn smem attr");
@@ -429,7 +494,7 @@ static kcna_status knn_bounded(kcna_ctx *c, const float *dQ, uint32_t m, const u
         const uint32_t *self = q_self ? q_self + q0 : nullptr;
         uint32_t *thresh = words, *cnt = words + batch, *redo = words + 2 * (size_t)batch;
         cudaMemsetAsync(redo, 0, 4, c->stream);
-        dist_tile_kernel<false><<<dim3(kcna_div_up(s, TB), kcna_div_up(mb, TQ)), 256, 0, c->stream>>>(
+        dist_tile_kernel<DT_SAMPLE><<<dim3(kcna_div_up(s, TB), kcna_div_up(mb, TQ)), 256, 0, c->stream>>>(
             Q, mb, c->X, s, stride, (int)c->ld, self, DistOut{D, s, nullptr, nullptr, nullptr, 0});
         if (cached)
             knn_bound_kernel<true><<<mb, SEL_T, (size_t)s * 4, c->stream>>>(D, s, rank, thresh, cnt);
@@ -442,7 +507,7 @@ static kcna_status knn_bounded(kcna_ctx *c, const float *dQ, uint32_t m, const u
                                                                   reinterpret_cast<uint32_t *>(cand), cnt, k, q0,
                                                                   d_out_ids, d_out_d, redo, c->d_err);
         } else {
-            dist_tile_kernel<true><<<dim3(kcna_div_up(c->n, TB), kcna_div_up(mb, TQ)), 256, 0, c->stream>>>(
+            dist_tile_kernel<DT_FILTER><<<dim3(kcna_div_up(c->n, TB), kcna_div_up(mb, TQ)), 256, 0, c->stream>>>(
                 Q, mb, c->X, c->n, 1, (int)c->ld, self, DistOut{nullptr, 0, thresh, cand, cnt, KNN_CAP});
             knn_final_kernel<false><<<mb, SEL_T, fsm, c->stream>>>(Q, c->X, (int)c->ld, self, cand, nullptr, cnt, k, q0,
                                                                    d_out_ids, d_out_d, redo, c->d_err);
@@ -453,18 +518,8 @@ static kcna_status knn_bounded(kcna_ctx *c, const float *dQ, uint32_t m, const u
         st = kcna_cuda_check(c, cudaGetLastError(), "knn kernels");
         if (st == KCNA_OK) st = kcna_cuda_check(c, cudaMemcpyAsync(&again, redo, 4, cudaMemcpyDeviceToHost, c->stream), "d2h");
         if (st == KCNA_OK) st = kcna_cuda_check(c, cudaStreamSynchronize(c->stream), "knn sync");
-        if (st != KCNA_OK || again == 0) continue;
-        if (again > 64) { // too many to do one by one
-            st = knn_all(c, Q, mb, self, k, d_out_ids + (uint64_t)q0 * k, d_out_d + (uint64_t)q0 * k);
-            continue;
-        }
-        std::vector<uint32_t> h(mb);
-        st = kcna_cuda_check(c, cudaMemcpyAsync(h.data(), cnt, (size_t)mb * 4, cudaMemcpyDeviceToHost, c->stream), "d2h");
-        if (st == KCNA_OK) st = kcna_cuda_check(c, cudaStreamSynchronize(c->stream), "knn sync");
-        for (uint32_t i = 0; i < mb && st == KCNA_OK; ++i)
-            if (h[i] > KNN_CAP || h[i] < k)
-                st = knn_all(c, Q + (uint64_t)i * c->ld, 1, self ? self + i : nullptr, k, d_out_ids + (uint64_t)(q0 + i) * k,
-                             d_out_d + (uint64_t)(q0 + i) * k);
+        if (st == KCNA_OK && again)
+            st = knn_redo(c, Q, mb, self, k, redo + 1, again, d_out_ids + (uint64_t)q0 * k, d_out_d + (uint64_t)q0 * k);
     }
     kcna_release(c, cand);
     kcna_release(c, words);

@@ -1,0 +1,83 @@
+"""Exact k-NN queries whose lists overflow: few of a batch are done again
+together (same answers, and a call with 60 of them costs less than one with
+1,000), and rows stored with a period do not make the lists overflow."""
+import time
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _best(f, reps=9):
+    f()
+    times = []
+    for _ in range(reps):
+        t0 = time.perf_counter()
+        f()
+        times.append(time.perf_counter() - t0)
+    return min(times)
+
+
+@pytest.fixture(scope="module")
+def crowded():
+    """100,003 rows, 12,000 of them close together; queries, and queries in the crowd."""
+    rng = np.random.default_rng(31)
+    X = rng.standard_normal((100003, 32)).astype(np.float32)
+    X[30000:42000] = X[3] + 1e-3 * rng.standard_normal((12000, 32)).astype(np.float32)
+    Q = rng.standard_normal((1000, 32)).astype(np.float32)
+    return X, Q, X[3] + 1e-3 * rng.standard_normal((1000, 32)).astype(np.float32)
+
+
+@pytest.mark.parametrize("bad", [1, 2, 33, 64, 65, 999, 1000])
+@pytest.mark.parametrize("k", [7, 300])
+def test_done_again_together(index, oracle, crowded, bad, k):
+    X, Q, C = crowded
+    at = np.random.default_rng(bad).choice(1000, bad, replace=False)
+    Q = Q.copy()
+    Q[at] = C[:bad]
+    index.upload(X)
+    gi, gd = index.knn_queries(Q, k)
+    some = np.unique(np.r_[0, 999, at[:12], np.arange(0, 1000, 97)])
+    oi, od = oracle.knn_queries(X, Q[some], k)
+    assert np.array_equal(gi[some], oi) and np.array_equal(gd[some], od)
+
+
+def test_own_rows_done_again(index, oracle, crowded):
+    X, _, _ = crowded
+    index.upload(X)
+    ids = np.r_[np.arange(0, 30000, 60), np.arange(30000, 42000, 500)].astype(np.uint32)
+    gi, gd = index.knn_exact(ids, 20)
+    some = np.r_[0:ids.size:41, ids.size - 24:ids.size]
+    oi, od = oracle.knn(X, ids[some], 20)
+    assert np.array_equal(gi[some], oi) and np.array_equal(gd[some], od)
+    assert not (gi == ids[:, None]).any()
+
+
+def test_few_cost_less_than_all(index):
+    rng = np.random.default_rng(7)
+    X = rng.standard_normal((200000, 64)).astype(np.float32)
+    X[50000:62000] = X[3] + 1e-3 * rng.standard_normal((12000, 64)).astype(np.float32)
+    Q = rng.standard_normal((1000, 64)).astype(np.float32)
+    C = X[3] + 1e-3 * rng.standard_normal((1000, 64)).astype(np.float32)
+    index.upload(X)
+    t_few = _best(lambda: index.knn_queries(np.concatenate([C[:60], Q[60:]]), 10))
+    t_all = _best(lambda: index.knn_queries(C, 10))
+    assert t_few < 1.3 * t_all, (t_few, t_all)
+
+
+def test_rows_with_a_period(index):
+    """Row i of cluster i mod 256, and the same rows in another order."""
+    n, d = 1 << 20, 32
+    rng = np.random.default_rng(9)
+    c = 3.0 * rng.standard_normal((256, d)).astype(np.float32)
+    noise = 0.1 * rng.standard_normal((n, d)).astype(np.float32)
+    X = c[np.arange(n) % 256] + noise
+    Q = c[np.arange(512) % 256] + 0.1 * rng.standard_normal((512, d)).astype(np.float32)
+    perm = rng.permutation(n)
+    t = []
+    for rows in (X, X[perm]):
+        index.upload(rows)
+        t.append((_best(lambda: index.knn_queries(Q, 10)), index.knn_queries(Q, 10)))
+    assert np.array_equal(t[0][1][1], t[1][1][1]) and np.array_equal(t[0][1][0], perm[t[1][1][0]])
+    assert t[0][0] < 2.0 * t[1][0], (t[0][0], t[1][0])
