@@ -9,6 +9,7 @@
 // sequences phases, reads counters and moves data across the boundary.
 #include <stdarg.h>
 #include <stdio.h>
+#include <stdlib.h>
 #include <string.h>
 
 #include <algorithm>
@@ -100,6 +101,30 @@ static void copy_phase_stats(const kcna_ctx *c, kcna_stats *st) {
     st->prune_skipped = c->prune_skipped;
 }
 
+// cudaMalloc, again without the cached blocks where they leave no room
+static cudaError_t device_malloc(kcna_ctx *c, size_t bytes, void **out) {
+    auto get = [&] {
+        if (c->mem_limit && c->mem_held + bytes > c->mem_limit) return cudaErrorMemoryAllocation;
+        const cudaError_t e = cudaMalloc(out, bytes);
+        if (e != cudaSuccess) (void)cudaGetLastError();
+        return e;
+    };
+    cudaError_t e = get();
+    if (e == cudaErrorMemoryAllocation && !c->free_blocks.empty()) {
+        kcna_release_all(c);
+        e = get();
+    }
+    if (e == cudaSuccess)
+        c->mem_held += bytes;
+    else
+        *out = nullptr;
+    return e;
+}
+static void device_free(kcna_ctx *c, void *p, size_t bytes) {
+    cudaFree(p);
+    c->mem_held -= bytes;
+}
+
 kcna_status kcna_dev_malloc(kcna_ctx *c, size_t bytes, void **out, const char *what) {
     *out = nullptr;
     // smallest cached block that holds `bytes` without wasting more than half of it
@@ -109,17 +134,8 @@ kcna_status kcna_dev_malloc(kcna_ctx *c, size_t bytes, void **out, const char *w
         c->free_blocks.erase(it);
         return KCNA_OK;
     }
-    cudaError_t e = cudaMalloc(out, bytes);
-    if (e == cudaErrorMemoryAllocation && !c->free_blocks.empty()) {
-        (void)cudaGetLastError();
-        kcna_release_all(c);
-        e = cudaMalloc(out, bytes);
-    }
-    if (e != cudaSuccess) {
-        *out = nullptr;
-        (void)cudaGetLastError();
+    if (device_malloc(c, bytes, out) != cudaSuccess)
         return kcna_fail(c, KCNA_E_OOM, std::string("cudaMalloc failed for ") + what);
-    }
     c->block_bytes[*out] = bytes;
     return KCNA_OK;
 }
@@ -137,22 +153,17 @@ void kcna_release(kcna_ctx *c, void *p) {
 void kcna_release_all(kcna_ctx *c) {
     for (auto &b : c->free_blocks) {
         c->block_bytes.erase(b.second);
-        cudaFree(b.second);
+        device_free(c, b.second, b.first);
     }
     c->free_blocks.clear();
 }
 
 static kcna_status grow(kcna_ctx *c, void **p, size_t *cur, size_t bytes) {
     if (*cur >= bytes && *p) return KCNA_OK;
-    if (*p) kcna_release(c, *p);
+    if (*p) device_free(c, *p, *cur);
     *p = nullptr;
     *cur = 0;
-    cudaError_t e = cudaMalloc(p, bytes);
-    if (e != cudaSuccess) {
-        (void)cudaGetLastError();
-        *p = nullptr;
-        return kcna_fail(c, KCNA_E_OOM, "scratch allocation failed");
-    }
+    if (device_malloc(c, bytes, p) != cudaSuccess) return kcna_fail(c, KCNA_E_OOM, "scratch allocation failed");
     *cur = bytes;
     return KCNA_OK;
 }
@@ -413,6 +424,7 @@ kcna_status kcna_create(kcna_ctx **out, int device) {
         delete c;
         return KCNA_E_CUDA;
     }
+    if (const char *mb = getenv("KCNA_DEVICE_LIMIT_MB")) c->mem_limit = (size_t)strtoull(mb, nullptr, 10) << 20;
     kcna_status s = bind(c);
     if (s == KCNA_OK) s = kcna_cuda_check(c, cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking), "stream");
     if (s == KCNA_OK) s = kcna_cuda_check(c, cudaDeviceGetAttribute(&c->num_sms, cudaDevAttrMultiProcessorCount, device), "attr");

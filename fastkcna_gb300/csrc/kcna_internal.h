@@ -119,6 +119,9 @@ struct kcna_ctx {
     // when cudaMalloc runs out of memory
     std::multimap<size_t, void *> free_blocks;
     std::unordered_map<void *, size_t> block_bytes;
+    // device memory held, and the most that may be (0: what the device has); KCNA_DEVICE_LIMIT_MB
+    // stands in for a device that others have filled
+    size_t mem_held = 0, mem_limit = 0;
 
     kcna_stats *stats = nullptr;
     double t0 = 0;

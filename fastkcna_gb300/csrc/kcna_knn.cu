@@ -436,7 +436,7 @@ static kcna_status knn_all(kcna_ctx *c, const float *dQ, uint32_t m, const uint3
 // The m queries of `list` (of n_q) done again the first way, together: one by
 // one, each was a pass over the base with 31 of a tile's 32 query places empty
 // (60 of 1,000 queries, 200,000 x 64 rows: 5.6 ms a call against 2.2 for doing
-// all 1,000 again, 1.2 so).
+// all 1,000 again, 0.94 so).
 static kcna_status knn_redo(kcna_ctx *c, const float *dQ, uint32_t n_q, const uint32_t *q_self, uint32_t k,
                             const uint32_t *list, uint32_t m, uint32_t *d_out_ids, float *d_out_d) {
     if (m == n_q) return knn_all(c, dQ, n_q, q_self, k, d_out_ids, d_out_d);
@@ -472,7 +472,9 @@ static kcna_status knn_redo(kcna_ctx *c, const float *dQ, uint32_t n_q, const ui
 // A bound per query from a sample, the rows that may lie within it, selection among those.
 static kcna_status knn_bounded(kcna_ctx *c, const float *dQ, uint32_t m, const uint32_t *q_self, uint32_t k, uint32_t s,
                                uint32_t *d_out_ids, float *d_out_d) {
-    const uint32_t batch = std::min<uint32_t>(m, 2048), rank = std::max<uint32_t>(k, 32), stride = c->n / s;
+    // queries at a time: their sampled distances within 1 GiB, as the distances of knn_all are
+    const uint32_t batch = std::min<uint32_t>(m, std::min<uint32_t>(2048, (uint32_t)((1ull << 30) / (s * 4ull)) & ~31u));
+    const uint32_t rank = std::max<uint32_t>(k, 32), stride = c->n / s;
     // the tensor-core screen pays from about 0.1 ms of FP32 work on
     const bool screened = c->ld <= 128 && (uint64_t)m * c->n * c->ld >= (1ull << 30);
     uint64_t *cand = nullptr;
@@ -485,7 +487,8 @@ static kcna_status knn_bounded(kcna_ctx *c, const float *dQ, uint32_t m, const u
     if (st == KCNA_OK)
         st = screened ? kcna_allow_smem(c, knn_final_kernel<true>, fsm, "knn smem attr")
                       : kcna_allow_smem(c, knn_final_kernel<false>, fsm, "knn smem attr");
-    for (uint32_t q0 = 0; q0 < m && st == KCNA_OK; q0 += batch) {
+    uint32_t q0 = 0;
+    for (; q0 < m && st == KCNA_OK; q0 += batch) {
         const uint32_t mb = std::min(batch, m - q0);
         void *buf = nullptr; // asked for each time: knn_all below may move the scratch
         if ((st = kcna_scratch(c, (uint64_t)batch * s * 4, &buf)) != KCNA_OK) break;
@@ -520,9 +523,15 @@ static kcna_status knn_bounded(kcna_ctx *c, const float *dQ, uint32_t m, const u
         if (st == KCNA_OK) st = kcna_cuda_check(c, cudaStreamSynchronize(c->stream), "knn sync");
         if (st == KCNA_OK && again)
             st = knn_redo(c, Q, mb, self, k, redo + 1, again, d_out_ids + (uint64_t)q0 * k, d_out_d + (uint64_t)q0 * k);
+        if (st != KCNA_OK) break;
     }
     kcna_release(c, cand);
     kcna_release(c, words);
+    if (st == KCNA_E_OOM) { // a nearly full device: the rest the first way
+        c->err.clear();
+        return knn_all(c, dQ + (uint64_t)q0 * c->ld, m - q0, q_self ? q_self + q0 : nullptr, k,
+                       d_out_ids + (uint64_t)q0 * k, d_out_d + (uint64_t)q0 * k);
+    }
     return st;
 }
 
@@ -536,7 +545,7 @@ kcna_status kcna_knn_device(kcna_ctx *c, const float *dQ, uint32_t m, const uint
     // them, the bound pays, unless k is so large that the sample is half the base
     const uint64_t s = std::max<uint64_t>(std::max<uint64_t>(2048, 2 * (uint64_t)k),
                                           (std::max<uint64_t>(k, 32) * c->n + 4095) / 4096);
-    const bool bounded = 2 * s <= c->n && s * 4 * 2048 <= (1ull << 31) &&
+    const bool bounded = 2 * s <= c->n && s <= (1u << 18) &&
                          (c->n > SEL_CACHE || ((uint64_t)m * c->n >= (1ull << 25) && c->n >= 16384));
     if (bounded) return knn_bounded(c, dQ, m, q_self, k, (uint32_t)s, d_out_ids, d_out_d);
     return knn_all(c, dQ, m, q_self, k, d_out_ids, d_out_d);

@@ -1,0 +1,42 @@
+"""Calls on a device that others have nearly filled (KCNA_DEVICE_LIMIT_MB: an
+allocation past the limit fails as cudaMalloc does): what ran in a given room
+runs there still, with the same answers."""
+import numpy as np
+import pytest
+
+from fastkcna_gb300 import kcna
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture
+def limited(monkeypatch):
+    made = []
+
+    def make(mb):
+        monkeypatch.setenv("KCNA_DEVICE_LIMIT_MB", str(mb))
+        ix = kcna.Index(0)
+        monkeypatch.delenv("KCNA_DEVICE_LIMIT_MB")
+        made.append(ix)
+        return ix
+
+    yield make
+    for ix in made:
+        ix.close()
+
+
+# rows, queries and results take 48 MiB; every distance of 268 queries 1,022 MiB,
+# the sampled ones of 1,088 and their lists 1,047
+@pytest.mark.parametrize("mb", [1075, 1300])
+def test_knn_within_a_limit(index, limited, mb):
+    n, d, m, k = 1000000, 4, 2048, 1000
+    rng = np.random.default_rng(2)
+    X = rng.standard_normal((n, d)).astype(np.float32)
+    Q = rng.standard_normal((m, d)).astype(np.float32)
+    index.upload(X)
+    want = index.knn_queries(Q, k)
+    ix = limited(mb)
+    ix.upload(X)
+    for _ in range(2):
+        got = ix.knn_queries(Q, k)
+        assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
