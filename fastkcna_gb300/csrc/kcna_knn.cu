@@ -6,7 +6,7 @@
 // reference scans ids in order and inserts equal distances after existing
 // ones, src/kgraph.cpp:227-260).
 //
-// Small bases: two kernels,
+// Few rows or few queries (knn_bound_pays): two kernels,
 //   1. a tiled distance kernel (32 queries x 128 rows per block, 4x4 register
 //      micro-tiles, dimensions staged through shared memory in chunks of 32)
 //      computing the canonical FMA-chain distance of every pair;
@@ -14,7 +14,7 @@
 //      the distance bits find the k-th smallest distance T, then every row with
 //      distance < T plus the lowest ids among rows with distance == T are kept
 //      and sorted by (distance, id).
-// Larger ones: writing every distance and reading it four times costs more
+// Else: writing every distance and reading it four times costs more
 // than computing it (7.3 of 17.7 ms for 1,000 queries against 1,000,000 x 128
 // rows), and the computation itself can be spared for all but a few thousand
 // rows per query:
@@ -71,10 +71,7 @@ __global__ void __launch_bounds__(256) dist_tile_kernel(const float *__restrict_
     for (int i = 0; i < 4; ++i)
 #pragma unroll
         for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
-    auto row_of = [&](uint64_t b) { return MODE == DT_SAMPLE ? sample_row(b, stride) : b; };
-    uint64_t at[4]; // this thread's rows of a chunk
-#pragma unroll
-    for (int s = 0; s < 4; ++s) at[s] = row_of(b0 + ((tid + s * 256) >> 3));
+    auto row_of = [&](uint64_t b) { return MODE == DT_SAMPLE ? sample_row(b, stride) : b * stride; };
 
     for (int k0 = 0; k0 < ld; k0 += KC) {
         {   // Q chunk: 32 rows x 32 floats, one float4 per thread
@@ -88,7 +85,7 @@ __global__ void __launch_bounds__(256) dist_tile_kernel(const float *__restrict_
             int idx = tid + s * 256;
             int r = idx >> 3, c = (idx & 7) * 4;
             float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (b0 + r < n && k0 + c < ld) v = __ldg(reinterpret_cast<const float4 *>(X + at[s] * ld + k0 + c));
+            if (b0 + r < n && k0 + c < ld) v = __ldg(reinterpret_cast<const float4 *>(X + row_of(b0 + r) * ld + k0 + c));
             *reinterpret_cast<float4 *>(&Xs[r][c]) = v;
         }
         __syncthreads();
@@ -134,7 +131,7 @@ constexpr int SEL_TIES = 1024;
 constexpr int SEL_QUICK = 256;
 
 constexpr uint32_t KNN_CAP = 8192;       // rows handed on per query at most
-constexpr uint32_t SEL_CACHE = 40960;    // a sample up to this length is read once, into shared memory; dispatch below
+constexpr uint32_t SEL_CACHE = 40960;    // a sample up to this length is read once, into shared memory
 
 struct SelectShared {
     uint32_t hist[SEL_BINS];
@@ -469,14 +466,18 @@ static kcna_status knn_redo(kcna_ctx *c, const float *dQ, uint32_t n_q, const ui
     return st;
 }
 
+// Whether the rows within a bound are found on tensor cores: from about 0.1 ms of FP32 work on.
+static bool knn_screened(const kcna_ctx *c, uint32_t m) {
+    return c->ld <= 128 && (uint64_t)m * c->n * c->ld >= (1ull << 30);
+}
+
 // A bound per query from a sample, the rows that may lie within it, selection among those.
 static kcna_status knn_bounded(kcna_ctx *c, const float *dQ, uint32_t m, const uint32_t *q_self, uint32_t k, uint32_t s,
                                uint32_t *d_out_ids, float *d_out_d) {
     // queries at a time: their sampled distances within 1 GiB, as the distances of knn_all are
     const uint32_t batch = std::min<uint32_t>(m, std::min<uint32_t>(2048, (uint32_t)((1ull << 30) / (s * 4ull)) & ~31u));
     const uint32_t rank = std::max<uint32_t>(k, 32), stride = c->n / s;
-    // the tensor-core screen pays from about 0.1 ms of FP32 work on
-    const bool screened = c->ld <= 128 && (uint64_t)m * c->n * c->ld >= (1ull << 30);
+    const bool screened = knn_screened(c, m);
     uint64_t *cand = nullptr;
     uint32_t *words = nullptr; // bounds, counts, and the queries to do again behind their number
     kcna_status st = kcna_alloc(c, &cand, ((uint64_t)batch * KNN_CAP + (screened ? 1 : 0)) / (screened ? 2 : 1), "k-NN lists");
@@ -535,18 +536,42 @@ static kcna_status knn_bounded(kcna_ctx *c, const float *dQ, uint32_t m, const u
     return st;
 }
 
+// Whether the bound pays, by the time of either way; 3,360 calls were timed
+// both ways (8 to 960 dimensions, 16,384 to 2,000,000 rows, 1 to 4,000 queries, k =
+// 10 to 1,000).  This takes the slower way by 0.3 % on average, 29 % at worst; a
+// bound from 40,960 rows on took it by 29 %, at worst at nearly nine times the time
+// (25,000 x 8 rows, 4,000 queries, k = 300: 4.7 ms against 0.54).
+static bool knn_bound_pays(const kcna_ctx *c, uint32_t m, uint32_t k, uint64_t sample) {
+    const double n = c->n, ld = c->ld, q = m, s = (double)sample;
+    const bool passes = k > SEL_QUICK; // selection by histogram passes
+    if (!knn_screened(c, m)) {
+        // Every distance is computed either way; what is saved is writing and
+        // selecting from them, against launches, the sample and the lists' atomics,
+        // which short rows do not hide.  One query, k = 10, both ways: 41,000 x 960
+        // rows 210 us (first way) and 306, 240,000 x 32 115 and 108, 700,000 x 128 415
+        // and 319; 1,000 queries, 130,000 x 8: 430 and 1,147.
+        const double from = passes ? (m <= 4 ? 65536 : 180000) : 262144;
+        return n >= (ld <= 64 && m > (passes ? 16u : 4u) ? 2 * from : from);
+    }
+    // Microseconds, fitted; mean error 8 %.  First way: launches and waits, one
+    // block's selection, and per pair the write, the selection and the FP32 chain.
+    // Bound: the rows once, a pass over them per 128 queries, the sample, and a list
+    // of about `len` rows a query, appended and rescored.
+    const double len = std::max<uint32_t>(k, 32) * n / s;
+    const double first = 57 + n * ((passes ? 7.4e-4 : 1.6e-4) + 1.3e-6 * ld + q * ((passes ? 4.9e-6 : 2e-6) + 7.2e-8 * ld));
+    const double bound = 150 + n * (2.4e-6 * ld + 6.7e-5 * (m / 128 + 1)) + 2.9e-4 * s +
+                         q * (0.08 + s * (5.6e-6 + 3.4e-8 * ld) + len * (8.7e-5 + 8.1e-7 * ld));
+    return bound < first;
+}
+
 kcna_status kcna_knn_device(kcna_ctx *c, const float *dQ, uint32_t m, const uint32_t *q_self, uint32_t k,
                             uint32_t *d_out_ids, float *d_out_d) {
     if (k == 0 || k > SEL_MAXK || k > c->n) return kcna_fail(c, KCNA_E_ARG, "knn: k must be in [1, min(1024, n)]");
     if (q_self && k >= c->n) return kcna_fail(c, KCNA_E_ARG, "knn: k must be < n when self is excluded");
-    // rows sampled for the bound: about 4,096 of n then lie within it.  Bases up
-    // to SEL_CACHE rows take two launches the first way (20,000
-    // rows, one query: 57 us with its copies); above, and where many queries meet
-    // them, the bound pays, unless k is so large that the sample is half the base
+    // rows sampled for the bound: about 4,096 of n then lie within it
     const uint64_t s = std::max<uint64_t>(std::max<uint64_t>(2048, 2 * (uint64_t)k),
                                           (std::max<uint64_t>(k, 32) * c->n + 4095) / 4096);
-    const bool bounded = 2 * s <= c->n && s <= (1u << 18) &&
-                         (c->n > SEL_CACHE || ((uint64_t)m * c->n >= (1ull << 25) && c->n >= 16384));
+    const bool bounded = 2 * s <= c->n && s <= (1u << 18) && knn_bound_pays(c, m, k, s);
     if (bounded) return knn_bounded(c, dQ, m, q_self, k, (uint32_t)s, d_out_ids, d_out_d);
     return knn_all(c, dQ, m, q_self, k, d_out_ids, d_out_d);
 }

@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 
 
 def _knn(ix, rng, d, size):
-    ix.upload(rng.standard_normal((50000, d)).astype(np.float32))
+    ix.upload(rng.standard_normal((300000, d), dtype=np.float32))
     Q = rng.standard_normal((200, d)).astype(np.float32)
     return lambda: ix.knn_queries(Q, size)
 

@@ -21,12 +21,12 @@ def _best(f, reps=9):
 
 @pytest.fixture(scope="module")
 def crowded():
-    """100,003 rows, 12,000 of them close together; queries, and queries in the crowd."""
+    """200,003 rows, 12,000 of them close together; queries, and queries in the crowd."""
     rng = np.random.default_rng(31)
-    X = rng.standard_normal((100003, 32)).astype(np.float32)
-    X[30000:42000] = X[3] + 1e-3 * rng.standard_normal((12000, 32)).astype(np.float32)
-    Q = rng.standard_normal((1000, 32)).astype(np.float32)
-    return X, Q, X[3] + 1e-3 * rng.standard_normal((1000, 32)).astype(np.float32)
+    X = rng.standard_normal((200003, 64)).astype(np.float32)
+    X[30000:42000] = X[3] + 1e-3 * rng.standard_normal((12000, 64)).astype(np.float32)
+    Q = rng.standard_normal((1000, 64)).astype(np.float32)
+    return X, Q, X[3] + 1e-3 * rng.standard_normal((1000, 64)).astype(np.float32)
 
 
 @pytest.mark.parametrize("bad", [1, 2, 33, 64, 65, 999, 1000])
