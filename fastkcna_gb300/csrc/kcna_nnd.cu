@@ -892,7 +892,10 @@ __global__ void __launch_bounds__(MS_NT, 9) merge_set_kernel(MergeArgs a, uint32
             for (int u = 0; u < CG; ++u) {
                 h[u] = __umulhi(id[u] * 0x9E3779B1u, (uint32_t)MS_H);
                 seen[u] = s_sv[h[u]];
-                // entries at the candidate's distance: by id; its own twin drops it
+                // entries at the candidate's distance: by id; its own twin drops it.  Mostly
+                // one or two; in a longer run (few-valued rows: a hundred and more) the
+                // place is sought by growing steps, then by halving ones
+                int walked = 0;
                 while (b[u] < (int)np && s_pd[b[u]] == d[u]) {
                     const uint32_t e = s_pi[b[u]] >> 2;
                     if (e >= id[u]) {
@@ -900,6 +903,13 @@ __global__ void __launch_bounds__(MS_NT, 9) merge_set_kernel(MergeArgs a, uint32
                         break;
                     }
                     ++b[u];
+                    if (++walked == 3) {
+                        auto below = [&](int t) { return t < (int)np && s_pd[t] == d[u] && (s_pi[t] >> 2) < id[u]; };
+                        int step = 1;
+                        for (; below(b[u] + step - 1); step <<= 1) b[u] += step;
+                        while (step >>= 1)
+                            if (below(b[u] + step - 1)) b[u] += step;
+                    }
                 }
                 if ((uint32_t)b[u] >= a.limit) surv[u] = false;
             }
