@@ -777,9 +777,9 @@ __global__ void __launch_bounds__(CB_T) centroid_final_kernel(const double *__re
 // an insert lands at is the nearest neighbour's.  So a batch of up to 32 is
 // sorted in registers and the pool's tail moves once.
 // A query is a chain of dependent loads (graph row, visited word, rows), so
-// what counts is their number and how many queries run beside it: eight blocks
-// an SM, a graph row together with its degree, sixteen 16-byte loads of a
-// neighbour's row in flight.  10,000 queries, beam 100, 100,003 x 128 rows:
+// what counts is their number and how many queries run beside it: five blocks
+// an SM (96 registers), a graph row together with its degree, sixteen 16-byte
+// loads of a neighbour's row in flight.  10,000 queries, beam 100, 100,003 x 128 rows:
 // 6.0 ms a call with one lane inserting and sorting the start entries, 2.9 ms
 // now; one query, beam 40, 20,000 x 32 rows: 0.29 and 0.14 ms.
 constexpr int BW = 4;
@@ -1753,12 +1753,18 @@ kcna_status kcna_search_device(kcna_ctx *c, const float *dQ, uint32_t m, const u
     if (!c->has_graph) return kcna_fail(c, KCNA_E_STATE, "search: no graph");
     if (L == 0 || L > 2048 || k == 0 || k > L) return kcna_fail(c, KCNA_E_ARG, "search: need 0 < k <= L <= 2048");
     const uint32_t vwords = (c->n + 31) / 32;
-    // eight blocks an SM, four where that many bitmaps would take more than 1 GiB
+    // Eight blocks an SM, where five run at once: the others start as the first
+    // finish, which evens out queries of unequal length (1,000,000 x 96 rows, 4,000 queries
+    // at beam 400: 5.6 ms against 6.1 with five; 20,000 at beam 100 7.0 against 6.7; even
+    // for most).  Four where that many bitmaps would take more than 1 GiB, and fewer
+    // on a nearly full device.
     const uint32_t per_sm = (uint64_t)c->num_sms * 8 * BW * vwords * 4 > (1ull << 30) ? 4 : 8;
     uint32_t blocks = std::max<uint32_t>(1, std::min<uint32_t>(kcna_div_up(m, BW), (uint32_t)c->num_sms * per_sm));
-    uint64_t slots = (uint64_t)blocks * BW;
     void *vis = nullptr;
-    KCNA_TRY(kcna_scratch2(c, slots * vwords * 4, &vis));
+    kcna_status vs;
+    while ((vs = kcna_scratch2(c, (uint64_t)blocks * BW * vwords * 4, &vis)) == KCNA_E_OOM && blocks > 1) blocks /= 2;
+    if (vs != KCNA_OK) return vs;
+    c->err.clear();
     size_t sm = (size_t)BW * (L + 1) * 8 + (c->ld <= (uint32_t)BEAM_STAGE ? (size_t)BW * c->ld * 4 : 0);
     KCNA_TRY(kcna_allow_smem(c, beam_search_kernel, sm, "beam search smem attr"));
     beam_search_kernel<<<blocks, BW * 32, sm, c->stream>>>(c->X, (int)c->ld, c->n, c->g_ids, c->g_deg, c->W, dQ, m,

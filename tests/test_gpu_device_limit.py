@@ -40,3 +40,21 @@ def test_knn_within_a_limit(index, limited, mb):
     for _ in range(2):
         got = ix.knn_queries(Q, k)
         assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
+
+
+# rows 15 MiB, the graph and its copies about 100; bitmaps of four blocks an SM 290 MiB, of eight 580
+@pytest.mark.parametrize("mb", [200, 480])
+def test_search_within_a_limit(index, limited, mb):
+    n, d, W, m, L = 1000000, 4, 8, 6000, 12
+    rng = np.random.default_rng(3)
+    X = rng.standard_normal((n, d)).astype(np.float32)
+    g = rng.integers(0, n, (n, W)).astype(np.uint32)
+    deg = np.full(n, W, np.uint32)
+    Q = rng.standard_normal((m, d)).astype(np.float32)
+    init = rng.integers(0, n, (m, L)).astype(np.uint32)
+    out = []
+    for ix in (index, limited(mb)):
+        ix.upload(X)
+        ix.set_graph(g, deg, 0)
+        out.append(ix.search(Q, L, 5, init))
+    assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
