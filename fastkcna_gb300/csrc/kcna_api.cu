@@ -707,7 +707,8 @@ kcna_status kcna_get_pools(kcna_ctx *c, uint32_t *ids, float *dists, uint32_t *c
     // touched took 2 to 45 ms for the same entries, by how the pages came about,
     // so the host touches each page first, while the kernel runs: 2.3
     // ms fresh and 0.5 touched, always (10.8 and 7.2 to 8.8 with the host loop)
-    // Nodes are taken in runs of at most 8 M entries, 64 MiB of device memory whatever the pools' size.
+    // Nodes are taken in runs of at most 8 M entries, 64 MiB of device memory whatever the pools'
+    // size; a device without that much left gets them taken apart on the host.
     const uint32_t run = (uint32_t)std::min<uint64_t>(c->n, std::max<uint64_t>(1, (8u << 20) / cap));
     uint32_t *d_ids = nullptr, *d_cnt = nullptr;
     float *d_d = nullptr;
@@ -715,8 +716,36 @@ kcna_status kcna_get_pools(kcna_ctx *c, uint32_t *ids, float *dists, uint32_t *c
     if (ids) s = kcna_alloc(c, &d_ids, (size_t)run * cap, "pool ids");
     if (s == KCNA_OK && dists) s = kcna_alloc(c, &d_d, (size_t)run * cap, "pool distances");
     if (s == KCNA_OK && counts) s = kcna_alloc(c, &d_cnt, run, "pool counts");
+    const bool on_host = s == KCNA_E_OOM;
+    std::vector<uint64_t> keys;
+    std::vector<uint32_t> cnt;
+    if (on_host) {
+        s = KCNA_OK;
+        c->err.clear();
+        keys.resize((size_t)run * c->cap);
+        cnt.resize(run);
+    }
     for (uint32_t i0 = 0; i0 < c->n && s == KCNA_OK; i0 += run) {
         const uint32_t m = std::min(run, c->n - i0);
+        if (on_host) {
+            s = kcna_cuda_check(c, cudaMemcpyAsync(keys.data(), c->pool + (uint64_t)i0 * c->cap, (size_t)m * c->cap * 8,
+                                                   cudaMemcpyDeviceToHost, c->stream), "d2h");
+            if (s == KCNA_OK)
+                s = kcna_cuda_check(c, cudaMemcpyAsync(cnt.data(), c->pool_cnt + i0, (size_t)m * 4, cudaMemcpyDeviceToHost,
+                                                       c->stream), "d2h");
+            if (s == KCNA_OK) s = kcna_cuda_check(c, cudaStreamSynchronize(c->stream), "sync");
+            for (uint32_t i = 0; i < m && s == KCNA_OK; ++i) {
+                const uint32_t k = std::min(cnt[i], c->cap);
+                if (counts) counts[i0 + i] = k;
+                for (uint32_t j = 0; j < cap; ++j) {
+                    const uint64_t key = j < k ? keys[(size_t)i * c->cap + j] : 0, at = (uint64_t)(i0 + i) * cap + j;
+                    const uint32_t bits = j < k ? (uint32_t)(key >> 32) : 0x7F800000u;
+                    if (ids) ids[at] = j < k ? (uint32_t)key >> 2 : KCNA_NONE;
+                    if (dists) memcpy(dists + at, &bits, 4);
+                }
+            }
+            continue;
+        }
         unpack_pools_kernel<<<kcna_div_up(m, 8), 256, 0, c->stream>>>(c->pool + (uint64_t)i0 * c->cap, c->pool_cnt + i0, m,
                                                                       c->cap, cap, d_ids, d_d, d_cnt);
         KCNA_LAUNCHED(c);

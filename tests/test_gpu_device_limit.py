@@ -58,3 +58,21 @@ def test_search_within_a_limit(index, limited, mb):
         ix.set_graph(g, deg, 0)
         out.append(ix.search(Q, L, 5, init))
     assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
+
+
+# the pools take 45 MiB, the outputs taken apart 44 more
+@pytest.mark.parametrize("mb", [50, 75, 400])
+def test_pools_within_a_limit(limited, mb):
+    n, cap = 60001, 97
+    rng = np.random.default_rng(4)
+    ids = rng.integers(0, n, (n, cap)).astype(np.uint32)
+    dist = np.sort(rng.random((n, cap)).astype(np.float32), 1)
+    cnt = rng.integers(0, cap + 1, n).astype(np.uint32)
+    ix = limited(mb)
+    ix.upload(rng.standard_normal((n, 4)).astype(np.float32))
+    ix.set_pools(ids, dist, cnt, kcna.params(K=cap, L=cap, search_K=cap, search_L=cap))
+    gi, gd, gc = ix.pools()
+    assert np.array_equal(gc, cnt)
+    there = np.arange(gi.shape[1])[None, :] < cnt[:, None]
+    assert np.array_equal(gi, np.where(there, ids, np.uint32(0xFFFFFFFF)))
+    assert np.array_equal(gd, np.where(there, dist, np.float32(np.inf)))
