@@ -1196,7 +1196,7 @@ __global__ void count_new_edges_kernel(const uint8_t *__restrict__ g_isnew, cons
 // 150,001 x 128 rows (1.1 ms here).  What is left is the latency of a node's
 // loads, so its ids come while the node before it is computed, and the radii
 // while its rows do.  13.7 KB a warp: sixteen warps an SM.
-constexpr int PJ_WARPS = 16, PJ_ROWS = 80, PJ_COLS = 64, PJ_U = 24;
+constexpr int PJ_WARPS = 16, PJ_ROWS = 80, PJ_COLS = 64, PJ_U = 24, PJ_NODE = 4, PJ_EMPTY = 128;
 struct P2kWarp {
     float x[pairs_region(PJ_ROWS)]; // rows, then the distance matrix: pusher i at i * (PJ_COLS + 1)
     uint32_t id[PJ_ROWS];           // neighbours, then pushers
@@ -1275,56 +1275,81 @@ __global__ void __launch_bounds__(PJ_WARPS * 32, 1) p2k_warp_kernel(RowsT rows, 
     const int lane = kcna_lane();
     P2kWarp &S = reinterpret_cast<P2kWarp *>(smem)[threadIdx.x >> 5];
     unsigned long long cc = 0;
-    // this warp's share of the pushes, [p0, p1): equal shares, so that a hub's
-    // pushers are split among warps (with nodes dealt out instead, the warps with
-    // the hubs ran four times as long as the rest on 40,009 x 960 rows)
-    const uint64_t total = off[N], G = (uint64_t)gridDim.x * PJ_WARPS, gw = blockIdx.x * PJ_WARPS + (threadIdx.x >> 5);
-    const uint64_t share = (total + G - 1) / G, p0 = min(total, gw * share), p1 = min(total, p0 + share);
-    if (p0 == p1) return;
-    // the last node whose pushers begin at or before p0
-    uint32_t q0 = 0;
-    for (uint32_t hi = N; hi - q0 > 1;) {
-        const uint32_t mid = q0 + (hi - q0) / 2;
-        if (off[mid] <= p0)
-            q0 = mid;
-        else
-            hi = mid;
-    }
-    // pushers' range and degree of 32 nodes from `at`, one per lane
-    uint64_t m0 = 0, m1 = 0;
-    int md = 0;
-    // the walk: node `at` (its place j among the 32), its pushers [t0, r1) and neighbours [c0, deg) to come
-    uint64_t at = q0, r0 = 0, r1 = 0, t0 = 0;
-    int j = -1, deg = 0, c0 = 0;
-    auto next = [&](P2kUnit &u) -> bool { // loads only: nothing is waited for
+    // this warp's share of the work, [p0, p1) of pushes and nodes laid end to end,
+    // node q at off[q] + PJ_NODE q: so that a hub's pushers are split among warps (with
+    // nodes dealt out instead, the warps with the hubs ran four times as long as the
+    // rest on 40,009 x 960 rows), and a warp with many nodes of one pusher, each a unit
+    // by itself, gets fewer pushes.  P2K of a build, 20,000 x 400 rows sorted by
+    // norm: pushes alone 18.7 ms (10.0 with a block per node before), PJ_NODE = 4 7.6,
+    // 8 7.4; the same rows shuffled 5.7, 5.3, 6.4; 40,009 x 960: 40.8, 38.8, 41.6.
+    const uint64_t G = (uint64_t)gridDim.x * PJ_WARPS, all = off[N] + (uint64_t)PJ_NODE * N;
+    const uint64_t p0 = (all + G - 1) / G * (blockIdx.x * PJ_WARPS + (threadIdx.x >> 5)), p1 = p0 + (all + G - 1) / G;
+    if (p0 >= all) return;
+    // of 32 nodes from `base`, one per lane: their pushers in this share, and their
+    // degrees; `some`: those with both; `end`: the first pusher behind the 32
+    uint64_t m0 = 0, m1 = 0, end = 0;
+    uint32_t base = 0;
+    int md = 0, empty = 0;
+    unsigned some = 0;
+    auto load = [&](uint32_t from) {
+        base = from;
+        const uint32_t q = base + lane;
+        m0 = off[min(q, N)];
+        m1 = off[min(q + 1, N)];
+        md = q < N ? (int)min(g_deg[q], W) : 0;
+        end = __shfl_sync(KCNA_FULL, m1, 31);
+        const int64_t s0 = (int64_t)(p0 - (uint64_t)PJ_NODE * q), s1 = s0 + (int64_t)(p1 - p0); // the share's pushes, were they all of q
+        m0 = (uint64_t)max((int64_t)m0, s0);
+        m1 = (uint64_t)min((int64_t)m1, s1);
+        some = __ballot_sync(KCNA_FULL, (int64_t)m0 < (int64_t)m1 && md > 0);
+    };
+    // the 32 nodes from the last whose place, a node counting as `per` pushes, is at or before p
+    auto load_at = [&](uint64_t p, uint32_t per) {
+        uint32_t q = 0, hi = N;
+        while (hi - q > 1) {
+            const uint32_t step = (hi - q + 31) / 32, x = q + step * (lane + 1);
+            q += step * __popc(__ballot_sync(KCNA_FULL, x < hi && off[x] + (uint64_t)per * x <= p));
+            hi = min(hi, q + step);
+        }
+        empty = 0;
+        load(q);
+    };
+    load_at(p0, PJ_NODE);
+    // the walk: node `at`, its pushers [t0, r1) and neighbours [c0, deg) to come.  Nodes
+    // without pushers cost their 32's load, and past PJ_EMPTY of them the next
+    // push's node is searched for
+    uint64_t r0 = 0, r1 = 0, t0 = 0;
+    uint32_t at = 0;
+    int deg = 0, c0 = 0;
+    auto next = [&](P2kUnit &u) -> bool {
         while (c0 >= deg || t0 >= r1) {
             if (c0 < deg && (c0 += PJ_COLS) < deg) { // the next neighbours, all pushers again
                 t0 = r0;
                 break;
             }
-            if (j >= 0) ++at;
-            if (at >= N) return false;
-            j = (j + 1) & 31;
-            if (j == 0) {
-                const uint64_t q = at + lane;
-                m0 = q < N ? max(off[q], p0) : p1;
-                m1 = q < N ? min(off[q + 1], p1) : p1;
-                md = q < N ? (int)min(g_deg[q], W) : 0;
+            while (!some) {
+                if (N - base <= 32 || end + (uint64_t)PJ_NODE * (base + 32) >= p1) return false;
+                if ((empty += 32) >= PJ_EMPTY)
+                    load_at(end, 0);
+                else
+                    load(base + 32);
             }
+            const int j = __ffs(some) - 1;
+            some &= some - 1;
+            empty = 0;
+            at = base + j;
             r0 = t0 = __shfl_sync(KCNA_FULL, m0, j);
             r1 = __shfl_sync(KCNA_FULL, m1, j);
             deg = __shfl_sync(KCNA_FULL, md, j);
             c0 = 0;
-            if (t0 >= p1) return false; // the next warp's
-            if (t0 >= r1) c0 = deg;     // no pushers: the next node
         }
-        u.q = (uint32_t)at;
+        u.q = at;
         u.nw = min(PJ_COLS, deg - c0);
         u.cap = min(PJ_U, PJ_ROWS - u.nw);
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const int k = lane + 32 * h;
-            const uint64_t e = at * W + c0 + k;
+            const uint64_t e = (uint64_t)at * W + c0 + k;
             u.w[h] = k < u.nw ? __ldg(g_ids + e) : KCNA_NONE;
             u.f[h] = k < u.nw && __ldg(g_isnew + e);
         }
