@@ -17,7 +17,8 @@
 // With Ki = min(K, pool count), entries past a pool's count are absent.
 //
 // GPU form, four steps on the context's stream:
-//   cagra_route_kernel  warp per node up to K = 128, else block per node: the node's first Ki pool ids in a
+//   cagra_route_kernel  warp per node up to K = 64 (cagra_route_warps), else
+//                       block per node: the node's first Ki pool ids in a
 //                       shared-memory hash table (id -> rank), the K x K
 //                       two-hop entries looked up in it (warp per one-hop
 //                       node, lanes over its pool: coalesced 8-byte keys),
@@ -28,14 +29,15 @@
 //   cagra_rev_fill_kernel  thread per kept edge: (rank << 32 | source) into
 //                       the target's segment;
 //   cagra_merge_warp_kernel / cagra_merge_kernel  warp per node with up to 256
-//                       reverse entries, else block per node: the smallest
+//                       reverse entries, else (and for every node below
+//                       CG_MERGE_WARPS of them) block per node: the smallest
 //                       reverse keys (the segment sorted in shared memory, or
 //                       streamed through a 1024-key best set for hubs), then
 //                       the interleaved row with every slot's position computed
 //                       in closed form.
 // A node's work is small (K = 64: 4,096 look-ups, some 32 reverse keys), so a
 // block of 256 threads per node spent its time at barriers: 2.8 and 2.1 ms for
-// 150,007 nodes at K = 64, 1.6 and 0.3 with a warp per node (route: up to K = 64).
+// 150,007 nodes at K = 64, 1.6 and 0.3 with a warp per node.
 #include <algorithm>
 
 #include "kcna_internal.h"
@@ -58,8 +60,16 @@ __device__ __forceinline__ uint32_t cg_hash(uint32_t id) { return (id * 0x9E3779
 // call at K = 200, 212 against 121 for 40,000 nodes at K = 1,000).
 // Warp or block per node: whole calls for 150,007 nodes, warp / block, K = 64
 // 2.26 / 2.82 ms, K = 100 8.3 / 6.0, for 11,132 nodes 0.30 / 0.32 and 0.81 /
-// 0.55: from P2 = 128 on the tables of eight warps leave 24 warps an SM.
+// 0.55: from P2 = 128 on the tables of eight warps leave 24 warps an SM.  Few
+// nodes leave SMs idle with a warp each: 600 nodes, K = 64 0.133 / 0.098 ms, 4,500
+// 0.180 / 0.167, 9,000 0.231 / 0.240; K = 33, 2,000 0.121 / 0.114, 4,500 0.128 / 0.138;
+// K = 16, 1,000 equal, 3,000 0.096 / 0.106.
 constexpr uint32_t CG_WARP_K = 64;
+constexpr bool cagra_route_warps(uint32_t N, uint32_t K) { return K <= CG_WARP_K && N >= 96 * K; }
+// Merge: one launch with a block for every node below this many nodes, a warp a
+// node and a second launch for the hubs from there on (600 nodes 0.092 / 0.098 ms a
+// call, 1,000 equal, 2,000 0.139 / 0.129).
+constexpr uint32_t CG_MERGE_WARPS = 1024;
 constexpr uint32_t cagra_slots(uint32_t P2) { return 8 * P2; }
 __host__ __device__ constexpr size_t cagra_route_bytes(uint32_t K, uint32_t P2, uint32_t HS) {
     return (size_t)P2 * 8 + (((size_t)K * 8 + 15) & ~(size_t)15) + (size_t)HS * 6;
@@ -257,14 +267,15 @@ __global__ void __launch_bounds__(CG_MW * 32) cagra_merge_warp_kernel(CagraRow<R
     }
 }
 
+// the nodes of `list`, or all (null)
 template <class R>
 __global__ void __launch_bounds__(CG_THREADS) cagra_merge_kernel(CagraRow<R> a, const uint32_t *__restrict__ list,
                                                                  const uint32_t *__restrict__ list_cnt) {
     __shared__ uint64_t s[2 * CG_BEST];
     const int tid = threadIdx.x;
-    const uint32_t n_list = *list_cnt;
+    const uint32_t n_list = list ? *list_cnt : a.N;
     for (uint32_t li = blockIdx.x; li < n_list; li += gridDim.x) {
-        const uint32_t i = list[li];
+        const uint32_t i = list ? list[li] : li;
         const uint32_t nk = min(a.PK, min(a.K, a.pool_cnt[i]));
         const uint64_t b = a.off[i];
         const uint32_t m = (uint32_t)(a.off[i + 1] - b);
@@ -329,7 +340,7 @@ kcna_status kcna_cagra_prune(kcna_ctx *c, const kcna_params *p) {
         KCNA_LAUNCHED(c);
         return kcna_cuda_check(c, cudaGetLastError(), "cagra_route_kernel");
     };
-    s = K <= CG_WARP_K ? route(cagra_route_kernel<32>, CG_THREADS / 32) : route(cagra_route_kernel<CG_THREADS>, 1);
+    s = cagra_route_warps(N, K) ? route(cagra_route_kernel<32>, CG_THREADS / 32) : route(cagra_route_kernel<CG_THREADS>, 1);
     if (s != KCNA_OK) return cleanup(), s;
     uint64_t E = 0;
     if ((s = kcna_exclusive_scan_u32(c, indeg, N, off, &E)) != KCNA_OK) return cleanup(), s;
@@ -343,6 +354,11 @@ kcna_status kcna_cagra_prune(kcna_ctx *c, const kcna_params *p) {
     auto merge = [&](auto rows) {
         const CagraRow<decltype(rows)> a{rows, c->pool, c->pool_cnt, c->cap,  N,        K,        PK,   fwd,
                                          off,  rev,     c->g_ids,    c->g_dist, c->g_deg, c->W, c->d_err};
+        if (N < CG_MERGE_WARPS) {
+            cagra_merge_kernel<<<N, CG_THREADS, 0, c->stream>>>(a, nullptr, nullptr);
+            KCNA_LAUNCHED(c);
+            return;
+        }
         cagra_merge_warp_kernel<<<std::min(kcna_div_up(N, CG_MW), sms * 12), CG_MW * 32, 0, c->stream>>>(a, indeg,
                                                                                                          list_cnt);
         cagra_merge_kernel<<<std::min(N, sms * 4), CG_THREADS, 0, c->stream>>>(a, indeg, list_cnt);

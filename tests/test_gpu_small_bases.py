@@ -1,0 +1,58 @@
+"""The rank prune on both sides of the node counts from which a warp per node pays,
+against the oracle.  And the rank
+prune of few nodes at a small K costs no more than at a larger one."""
+import time
+
+import numpy as np
+import oracle_py
+import pytest
+
+from fastkcna_gb300 import kcna
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n,K", [(1023, 8), (1024, 8), (767, 8), (1535, 16), (1536, 16), (6143, 64), (6144, 64), (6300, 62), (6400, 66)])
+def test_rank_prune_equals_oracle(index, oracle, n, K):
+    d = 12
+    rng = np.random.default_rng(n + K)
+    X = rng.integers(-200, 201, (n, d)).astype(np.float32)
+    X[:5] //= 8  # in many pools: long reverse segments
+    index.upload(X)
+    ids, dist = index.knn_exact(np.arange(n, dtype=np.uint32), K)
+    cnt = np.full(n, K, np.uint32)
+    cnt[::9] = max(K // 2 + 1, 2)
+    kw = dict(K=K, L=K, S=10, R=100, iterations=1, search_L=min(K, 40), nsg_R=min(K, 32), search_K=K)
+    p = kcna.params(**kw)
+    index.set_pools(ids, dist, cnt, p)
+    index.prune("cagra", p)
+    g, deg, _ = index.graph()
+    oi, _, odeg = oracle.prune(oracle_py.KCNA_CAGRA, X, oracle_py.params(**kw), ids, dist, cnt, K // 2 + 1)
+    assert np.array_equal(deg, odeg)
+    live = np.arange(K // 2 + 1) < deg[:, None]
+    assert np.array_equal(g[:, : K // 2 + 1][live], oi[live])
+
+
+def _time(f, reps=60):
+    f()
+    t = []
+    for _ in range(reps):
+        t0 = time.perf_counter()
+        f()
+        t.append(time.perf_counter() - t0)
+    return sorted(t)[reps // 6]
+
+
+def test_rank_prune_of_few_nodes(index):
+    """K = 64 (a warp per node on large bases) against the four times as many
+    look-ups of K = 128 (a block per node)."""
+    n = 600
+    X = np.random.default_rng(1).standard_normal((n, 32)).astype(np.float32)
+    index.upload(X)
+    ids, dist = index.knn_exact(np.arange(n, dtype=np.uint32), 128)
+    t = []
+    for K in (64, 128):
+        p = kcna.params(K=K, L=128, search_K=K, search_L=128)
+        index.set_pools(ids, dist, np.full(n, 128, np.uint32), p)
+        t.append(_time(lambda: index.prune("cagra", p)))
+    assert t[0] < 1.02 * t[1], t
