@@ -44,8 +44,12 @@ __device__ __forceinline__ bool occludes(const PruneRule &r, float td, float djk
 // Row lengths whose batches are staged: three prunes of 60,000 unit rows, 40
 // kept, pools of 260, straight against staged: d = 8 2.0 / 2.2 ms, 32 5.1 / 4.0,
 // 96 16.2 / 12.3, 128 21.9 / 17.2, 160 27.7 / 23.2, 192 33.5 / 31.7, 256 45.4 /
-// 45.0 (the batches of ever fewer warps fit an SM).
+// 45.0 (the batches of ever fewer warps fit an SM).  Few nodes leave an SM few
+// warps either way, and a batch's copies are then waited for: 600 nodes, staged
+// against straight, d = 32 to 192 1.13 to 1.3 times as long; 1,500 at d = 64 to
+// 192 0.85 to 1.04; at d = 32 3,000 1.04 to 1.17, 4,500 0.82 to 0.89.
 constexpr int PRUNE_STAGED_MIN = 32, PRUNE_STAGED_MAX = 192;
+constexpr uint32_t prune_staged_from(int ld) { return ld < 64 ? 4096 : 1536; }
 // pitch in floats of a staged row: an odd number of 16-byte pieces, so that the lanes' rows lie in distinct banks
 __host__ __device__ constexpr int prune_pitch(int ld) { return ((ld >> 2) | 1) * 4; }
 __host__ __device__ constexpr size_t prune_staged_bytes(int ld) { return (size_t)(32 * prune_pitch(ld) + 4 * ld) * 4; }
@@ -1606,7 +1610,8 @@ kcna_status kcna_prune_all(kcna_ctx *c, const kcna_params *p, int kind, uint64_t
             prune_kernel<false><<<kcna_div_up(n_items, PW), PW * 32, sm, c->stream>>>(
                 RowsB16{c->Xh, (int)c->ld}, c->n, c->pool, c->pool_cnt, c->cap, rule, (int)range, maxc, c->g_ids,
                 c->g_dist, c->g_deg, c->W, c->counters + 16, n_items, list);
-        else if ((int)c->ld >= PRUNE_STAGED_MIN && (int)c->ld <= PRUNE_STAGED_MAX) {
+        else if ((int)c->ld >= PRUNE_STAGED_MIN && (int)c->ld <= PRUNE_STAGED_MAX &&
+                 n_items >= prune_staged_from((int)c->ld)) {
             const size_t ssm = prune_staged_bytes((int)c->ld) + (size_t)2 * range * 4;
             KCNA_TRY(kcna_allow_smem(c, prune_kernel<true, RowsF32>, ssm, "prune smem attr"));
             prune_kernel<true><<<n_items, 32, ssm, c->stream>>>(

@@ -1,5 +1,5 @@
-"""The rank prune on both sides of the node counts from which a warp per node pays,
-against the oracle.  And the rank
+"""The rank prune and the FP32 prune on both sides of the node counts from which a
+warp per node, and batches in shared memory, pay; against the oracle.  And the rank
 prune of few nodes at a small K costs no more than at a larger one."""
 import time
 
@@ -31,6 +31,30 @@ def test_rank_prune_equals_oracle(index, oracle, n, K):
     assert np.array_equal(deg, odeg)
     live = np.arange(K // 2 + 1) < deg[:, None]
     assert np.array_equal(g[:, : K // 2 + 1][live], oi[live])
+
+
+@pytest.mark.parametrize("kind", [1, 3, 4])
+@pytest.mark.parametrize("n,d,k,R", [(4096, 32, 33, 4), (4095, 61, 60, 32), (4100, 61, 200, 5), (1536, 96, 260, 128), (1535, 96, 100, 40),
+                                     (1600, 189, 70, 36), (1600, 192, 100, 40), (1600, 96, 2, 1), (1600, 64, 90, 37)])
+def test_warp_prune_equals_oracle(index, oracle, kind, n, d, k, R):
+    rng = np.random.default_rng(d + k)
+    X = rng.standard_normal((n, d)).astype(np.float32)
+    X /= np.linalg.norm(X, axis=1, keepdims=True)
+    X[50:90] = X[7]
+    X[90:130] *= np.float32(0.25)
+    index.upload(X)
+    ids, dist = index.knn_exact(np.arange(n, dtype=np.uint32), k)
+    cnt = np.full(n, k, np.uint32)
+    cnt[::7] = 1
+    cnt[3::7] = max(1, k // 3)
+    kw = dict(K=k, L=k, S=10, R=100, iterations=1, search_L=40, nsg_R=R, search_K=k, tau=0.02, angle=60.0)
+    kp = kcna.params(**kw)
+    index.set_pools(ids, dist, cnt, kp)
+    index.prune({1: "nsg", 3: "taumng", 4: "alphapg"}[kind], kp)
+    g, deg, _ = index.graph()
+    oi, _, odeg = oracle.prune(kind, X, oracle_py.params(**kw), ids, dist, cnt, g.shape[1])
+    assert np.array_equal(deg, odeg)
+    assert np.array_equal(g, oi)
 
 
 def _time(f, reps=60):
