@@ -895,21 +895,22 @@ __global__ void __launch_bounds__(MS_NT, 9) merge_set_kernel(MergeArgs a, uint32
                 // entries at the candidate's distance: by id; its own twin drops it.  Mostly
                 // one or two; in a longer run (few-valued rows: a hundred and more) the
                 // place is sought by growing steps, then by halving ones
-                int walked = 0;
-                while (b[u] < (int)np && s_pd[b[u]] == d[u]) {
+                const int stop = min((int)np, b[u] + 3);
+                while (b[u] < stop && s_pd[b[u]] == d[u]) {
                     const uint32_t e = s_pi[b[u]] >> 2;
                     if (e >= id[u]) {
                         if (e == id[u]) surv[u] = false;
                         break;
                     }
                     ++b[u];
-                    if (++walked == 3) {
-                        auto below = [&](int t) { return t < (int)np && s_pd[t] == d[u] && (s_pi[t] >> 2) < id[u]; };
-                        int step = 1;
-                        for (; below(b[u] + step - 1); step <<= 1) b[u] += step;
-                        while (step >>= 1)
-                            if (below(b[u] + step - 1)) b[u] += step;
-                    }
+                }
+                if (b[u] == stop && stop < (int)np) {
+                    auto below = [&](int t) { return t < (int)np && s_pd[t] == d[u] && (s_pi[t] >> 2) < id[u]; };
+                    int step = 1;
+                    for (; below(b[u] + step - 1); step <<= 1) b[u] += step;
+                    while (step >>= 1)
+                        if (below(b[u] + step - 1)) b[u] += step;
+                    if (b[u] < (int)np && s_pd[b[u]] == d[u] && (s_pi[b[u]] >> 2) == id[u]) surv[u] = false;
                 }
                 if ((uint32_t)b[u] >= a.limit) surv[u] = false;
             }
