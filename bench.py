@@ -319,10 +319,11 @@ def roofline(st, hbm_gbs, ld, n, search_k, tensor_tflops=None):
     kernels = {"join": "join_tc_kernel" if st["gram_tc"] else "join_warp_kernel", "merge": "merge_set_kernel",
                "prune": "prune_gram_kernel" if st.get("prune_tc") else "prune_kernel"}
     limiters = {
-        "join": "scattered 16-byte candidate-slot stores and the TMEM re-read of the write pass (latency, LSU)",
-        "merge": "shared-memory latency: lookup of every candidate in the node's pool and hash table",
+        "join": "scattered 16-byte candidate-slot stores and the TMEM re-read of the write pass (latency, LSU)" if st["gram_tc"]
+        else "issue slots (two thirds), FMA pipe 40 %",
+        "merge": "issue slots and shared memory (70 to 80 % each): lookup of every candidate in the node's pool and hash table",
         "prune": "issue slots of the mask-building warps; tensor pipe about 30 % busy" if st.get("prune_tc")
-        else "issue slots of the distance chains",
+        else "shared memory: the staged rows' reads (84 % of the L1's cycles)",
     }
     name = max(models, key=lambda k: ph.get(k, 0.0))
     ms, nl = ph[name], max(launches[name], 1)

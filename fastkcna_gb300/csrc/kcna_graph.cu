@@ -86,9 +86,10 @@ __device__ __forceinline__ int nth_bit(unsigned m, int n) {
 // kept[4..nk), the (survivor, kept row) pairs dealt to the lanes; finally the
 // batch is resolved in candidate order (the first unoccluded lane is kept and
 // tests the later lanes; the last eight or fewer test all their pairs at once).
-// Instruction issue bounds it: with one survivor at a time against a lane per
-// kept row, and a round per kept candidate, half of the lanes had no pair (30,000
-// x 96, 40 kept: 16.5 of 32 lanes, 43 instructions a pair and warp).  Prune
+// With one survivor at a time against a lane per kept row, and a round per kept
+// candidate, half of the lanes had no pair (30,000 x 96, 40 kept: 16.5 of 32
+// lanes, 43 instructions a pair and warp); now 27 have.  What bounds the staged
+// form is shared memory (60,000 x 96: 84 % of the L1's cycles, issue 0.45).  Prune
 // of the 150,007 x 96 layer build 35.3 -> 23.9 ms, of 150,001 x 128 NSG 28 ->
 // 20.3 (staging alone 33.1 and 21.9), of the 40,009 x 960 tau-MNG 65 -> 54.
 // Rows are read through R (FP32 or exact BF16 copy).
@@ -785,7 +786,9 @@ __global__ void __launch_bounds__(CB_T) centroid_final_kernel(const double *__re
 // an SM (96 registers), a graph row together with its degree, sixteen 16-byte
 // loads of a neighbour's row in flight.  10,000 queries, beam 100, 100,003 x 128 rows:
 // 6.0 ms a call with one lane inserting and sorting the start entries, 2.9 ms
-// now; one query, beam 40, 20,000 x 32 rows: 0.29 and 0.14 ms.
+// now; one query, beam 40, 20,000 x 32 rows: 0.29 and 0.14 ms.  A full batch ends
+// at the L1's data path (95 % busy; a lane per row, 16 bytes at a time), one query
+// at its chain.
 constexpr int BW = 4;
 constexpr int BEAM_STAGE = 2048; // floats of a query row kept in shared memory at most
 
@@ -1197,9 +1200,10 @@ __global__ void count_new_edges_kernel(const uint8_t *__restrict__ g_isnew, cons
 // Survivors within u's radius become candidates of u, one run per (q, u) after
 // one atomicAdd.  A node has about 10 pushers and 26 neighbours (C2): a block
 // per node with a 32 x 64 tile for those 260 pairs took 2.6 ms a round on
-// 150,001 x 128 rows (1.1 ms here).  What is left is the latency of a node's
-// loads, so its ids come while the node before it is computed, and the radii
-// while its rows do.  13.7 KB a warp: sixteen warps an SM.
+// 150,001 x 128 rows (1.1 ms here).  A node's ids come while the node before it is
+// computed, and the radii while its rows do.  13.7 KB a warp: sixteen warps an SM.
+// What is left is issue (60,000 x 128: 0.55 a cycle, FMA pipe 37 %, 20 of 32 lanes),
+// and the code's size (instruction fetch, two cycles of an issue's six).
 constexpr int PJ_WARPS = 16, PJ_ROWS = 80, PJ_COLS = 64, PJ_U = 24, PJ_NODE = 4, PJ_EMPTY = 128;
 struct P2kWarp {
     float x[pairs_region(PJ_ROWS)]; // rows, then the distance matrix: pusher i at i * (PJ_COLS + 1)

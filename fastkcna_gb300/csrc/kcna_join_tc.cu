@@ -1,8 +1,8 @@
 // kcna_join_tc.cu - NN-descent local join on tcgen05 Gram tiles, several
 // nodes per tile.
 //
-// Same work as join_kernel (kcna_nnd.cu; reference join src/kgraph.cpp:1097-1117
-// with Nhood::join :970-987): for node n, every pair of its new list A
+// Same work as the FP32 join (join_warp_kernel and its two versions for more rows,
+// kcna_nnd.cu; reference join src/kgraph.cpp:1097-1117 with Nhood::join :970-987): for node n, every pair of its new list A
 // (i < j) and of A x old list B, each pair emitted to both endpoints'
 // candidate buffers when within that endpoint's radius.  Here the distances
 // come from Gram tiles: d(i, j) = (|x_i|^2 + |x_j|^2) - 2 <x_i, x_j>, with the

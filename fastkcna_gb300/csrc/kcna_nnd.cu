@@ -6,16 +6,20 @@
 // statistics / stop rule (:1365-1426).
 //
 // GPU form of one iteration:
-//   join    one warp per node n (a block for a node of more than 64 rows): gather the node's new list A and old list B, compute every
-//           pair of A x A (i < j) and A x B with the canonical FMA-chain
-//           distance in register tiles (rows staged through shared memory),
-//           and emit each pair to both endpoints' candidate buffers when it is
-//           within that endpoint's radius.  Candidates of one target from one
-//           node are written as one contiguous run after a single atomicAdd.
-//   merge   one block per node: sort the candidate buffer, drop duplicates,
-//           merge with the sorted pool by rank, keep the best `limit`; new
-//           entries carry flag=new (the reference's InsertIntoPool
-//           :261-298 semantics applied to a batch).
+//   join    one warp per node n (a block for a node of more than 64 rows):
+//           gather the node's new list A and old list B, compute every pair
+//           of A x A (i < j) and A x B with the canonical FMA-chain distance
+//           in register tiles (rows staged through shared memory), and emit
+//           each pair to both endpoints' candidate buffers when it is within
+//           that endpoint's radius.  Candidates of one target from one node
+//           are written as one contiguous run after a single atomicAdd.
+//   merge   the candidates a node's pool lacks, each once, put in by rank, the
+//           best `limit` kept; new entries carry flag=new (the reference's
+//           InsertIntoPool :261-298 semantics applied to a batch).
+//           merge_set_kernel: four warps per node, the distinct ones in a
+//           hash table, ranks from counts, no sort; merge_kernel: a block for
+//           a node of more than 892; merge_warp_kernel: the few of a
+//           refinement round, sorted by a warp.
 //   sample  the update step: M (prefix holding S new entries), radiusM, the
 //           forward new/old lists and reverse lists (atomics, capped buffers,
 //           random subset of R chosen in the join).
@@ -314,7 +318,8 @@ __global__ void __launch_bounds__(JT, 3) join_kernel(JoinArgs a, R rows, const u
 // those for the block version from the front (cnt[0]), those for join_kernel
 // from the end (cnt[1]).  150,001 x 128 rows (28 rows a node): 20 ms a
 // build against 47 for a block of 256 threads per node.
-// 11.5 KB a warp: sixteen warps an SM, as many as the registers allow.
+// 11.5 KB a warp: sixteen warps an SM, as many as the registers allow.  Instruction
+// issue bounds it (60,000 x 128: 0.66 a cycle, FMA pipe 40 %, 18 to 19 of 32 lanes).
 template <int NT, int ROWS>
 struct JoinSet {
     float x[pairs_region(ROWS)]; // rows, then the distance matrix: row i at i * (n | 1)
@@ -800,7 +805,8 @@ __device__ uint32_t block_exclusive_scan(uint32_t *data, int n, uint32_t *s_warp
 // only, and equal distances are told apart by the id once at the end.
 // 400,003 rows, the four merges of a learned build: 58 ms with a warp per node
 // and a sort of all survivors with their repeats, 26 ms now (9 nodes of each
-// SM in flight; the table alone, with a warp per node, gave 50).
+// SM in flight; the table alone, with a warp per node, gave 50).  Now issue (0.65 to
+// 0.74 a cycle) and shared memory (66 to 79 % of its cycles) are what is left.
 // MS_H: table slots (a prime, for the double hashing).  A node with more than
 // MS_CAP distinct survivors is queued for the block merge; the count is read
 // before each warp's batch of 32, and the four warps' batches fit beside it.

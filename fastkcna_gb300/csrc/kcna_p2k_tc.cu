@@ -1,6 +1,6 @@
 // kcna_p2k_tc.cu - P2K (BridgeView) join on tcgen05 Gram tiles.
 //
-// Same work as p2k_join_kernel (kcna_graph.cu; reference BridgeView_join,
+// Same work as p2k_warp_kernel (kcna_graph.cu; reference BridgeView_join,
 // src/kgraph.cpp:2634-2648): for every node q, every pusher u of q (the
 // entries of rnn(q), with u's isnew flag) meets every graph neighbour w of q;
 // the pair is skipped when u == w or both are old, counted otherwise, and w

@@ -35,9 +35,11 @@
 // (prune_resume_kernel, kcna_graph.cu), which continues from the kept list.
 //
 // The screen pays where the rule's margin is wide against the FP8 error: on
-// the 960-dimensional C4 rows with tau = 10, every pair of the first 50
-// candidates is decided "not occluded" by a wide margin, so the prune reads
-// 128 one-byte rows per node and computes no FP32 distance at all.
+// the 960-dimensional C4 rows with tau = 10, nearly every pair of the first 50
+// candidates is decided "not occluded", so the prune reads 128 one-byte rows
+// per node and a build of 1M rows recomputes 1,280 pairs in FP32.  Where
+// clusters are smaller it leaves more: 288 pairs a node for 40,009 rows in 512
+// clusters.
 //
 // Block layout: persistent, one block per SM, warp-specialised, mbarrier
 // hand-offs, every wait bounded (a wait that gives up sets the error word,
@@ -491,7 +493,8 @@ __global__ void __launch_bounds__(F8_THREADS, 1) prune_fp8_kernel(F8Args a) {
 // that turns out dropped is never read).  40,009 rows of 960 (512 clusters,
 // tau = 10: 288 undecided pairs a node): 213 ms a prune when the tile kernel's
 // scan warp resolved them, one kept neighbour at a time and one warp per SM;
-// 21 ms now, 16 of them here (5.8 TB/s of rows from L2).  Two blocks an SM:
+// 21 ms now, 16 of them here (5.8 TB/s of rows from L2, 16 bytes a lane from 32
+// rows at a time: the L1's data path is busy 95 % of the time).  Two blocks an SM:
 // three (80 registers) take 17 ms, four (64) 26, with fewer loads in flight.
 constexpr int RW_WARPS = 8;
 struct ResolveShared {

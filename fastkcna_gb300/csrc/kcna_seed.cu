@@ -361,9 +361,9 @@ __global__ void __launch_bounds__(BAND_WARPS * 32) seed_band_kernel(R rows, uint
 // the nearest `limit` distinct entries become the pool.  Warp per node, the
 // 1024 slots held in registers (32 per lane) and sorted by a bitonic network;
 // the distinct ones go through shared memory to be written in rows.
-// Instruction issue bounds it.  With the keys the other way round (32 r + lane)
-// 40 stages crossed lanes, 64 shuffles each: 400,003 rows, 16 tables 10.6 ms,
-// 5.8 now.
+// The integer pipe (74 %) and the fetch of the unrolled network's code bound it.
+// With the keys the other way round (32 r + lane) 40 stages crossed lanes, 64
+// shuffles each: 400,003 rows, 16 tables 10.6 ms, 5.8 now.
 static_assert(SEED_CAND == 1024, "the collect sort holds 32 keys per lane");
 constexpr int COLLECT_PITCH = SEED_CAND + SEED_CAND / 32;
 
