@@ -77,8 +77,10 @@ __device__ void warp_gen_random(uint64_t seed, uint64_t stream, uint32_t size, u
     __syncwarp();
 }
 
+// keep: entries a pool starts with, min(S, L).
 __global__ void __launch_bounds__(128) init_kernel(const float *__restrict__ X, int ld, uint32_t N, uint32_t S,
-                                                   uint32_t cap, uint64_t seed, uint64_t *__restrict__ pool,
+                                                   uint32_t keep, uint32_t cap, uint64_t seed,
+                                                   uint64_t *__restrict__ pool,
                                                    uint32_t *__restrict__ pool_cnt,
                                                    uint32_t *__restrict__ fwd_new, uint32_t fwd_new_cap,
                                                    uint32_t *__restrict__ fwd_new_cnt) {
@@ -92,23 +94,23 @@ __global__ void __launch_bounds__(128) init_kernel(const float *__restrict__ X, 
     for (uint32_t i = lane; i < 2 * S; i += 32) fwd_new[(uint64_t)n * fwd_new_cap + i] = s_ids[w][i];
     if (lane == 0) fwd_new_cnt[n] = 2 * S;
     __syncwarp();
-    // pool: S+1 random ids, n dropped, first S kept
+    // pool: S+1 random ids, n dropped, of the first S the nearest `keep`
     warp_gen_random(seed, (uint64_t)n * 4 + 1, S + 1, N, s_ids[w], s_tmp[w]);
     uint64_t key = KCNA_EMPTY_KEY;
     {
         uint32_t r = lane <= (int)S ? s_ids[w][lane] : n;
-        bool keep = lane <= (int)S && r != n;
-        unsigned mk = __ballot_sync(KCNA_FULL, keep);
+        bool other = lane <= (int)S && r != n;
+        unsigned mk = __ballot_sync(KCNA_FULL, other);
         int pos = __popc(mk & kcna_lanemask_lt());
-        if (keep && pos < (int)S) {
+        if (other && pos < (int)S) {
             float dd = kcna_l2_ldg(X + (uint64_t)r * ld, X + (uint64_t)n * ld, ld);
             key = kcna_key(dd, r, (uint32_t)(KCNA_FLAG_NEW | KCNA_FLAG_ISNEW));
         }
     }
     key = kcna_warp_sort32(key);
     uint64_t *pr = pool + (uint64_t)n * cap;
-    for (uint32_t i = lane; i < cap; i += 32) pr[i] = (i == (uint32_t)lane && i < S) ? key : KCNA_EMPTY_KEY;
-    if (lane == 0) pool_cnt[n] = S;
+    for (uint32_t i = lane; i < cap; i += 32) pr[i] = (i == (uint32_t)lane && i < keep) ? key : KCNA_EMPTY_KEY;
+    if (lane == 0) pool_cnt[n] = keep;
 }
 
 // ---------------------------------------------------------------------------
@@ -1555,13 +1557,16 @@ kcna_status kcna_cand_alloc(kcna_ctx *c, const kcna_params *p) {
 kcna_status kcna_nnd_init(kcna_ctx *c, const kcna_params *p) {
     if (p->S == 0 || p->S > 31) return kcna_fail(c, KCNA_E_ARG, "S must be in [1, 31]");
     KCNA_TRY(kcna_phase_begin(c));
-    init_kernel<<<kcna_div_up(c->n, 4), 128, 0, c->stream>>>(c->X, (int)c->ld, c->n, p->S, c->cap, p->seed, c->pool,
-                                                           c->pool_cnt, c->fwd_new, c->fwd_new_cap, c->fwd_new_cnt);
+    // the pools hold L entries, and M (how many the next lists come from) stays within a pool's count
+    const uint32_t keep = std::min(p->S, p->L);
+    init_kernel<<<kcna_div_up(c->n, 4), 128, 0, c->stream>>>(c->X, (int)c->ld, c->n, p->S, keep, c->cap, p->seed,
+                                                           c->pool, c->pool_cnt, c->fwd_new, c->fwd_new_cap,
+                                                           c->fwd_new_cnt);
     KCNA_LAUNCHED(c);
     KCNA_TRY(kcna_cuda_check(c, cudaGetLastError(), "init_kernel"));
     KCNA_TRY(kcna_pools_set_radius(c, p->L));
     // M = S (src/kgraph.cpp:1030)
-    std::vector<uint32_t> Ms(c->n, p->S);
+    std::vector<uint32_t> Ms(c->n, keep);
     KCNA_TRY(kcna_cuda_check(c, cudaMemcpyAsync(c->M, Ms.data(), (size_t)c->n * 4, cudaMemcpyHostToDevice, c->stream),
                              "M init"));
     KCNA_TRY(kcna_phase_end(c, KCNA_PHASE_INIT));
@@ -1832,6 +1837,7 @@ kcna_status kcna_nndescent_run(kcna_ctx *c, const kcna_params *pin, kcna_stats *
     }
     const uint32_t maxl = std::max(std::max(P.L, P.K), std::max(P.search_L, P.search_K));
     if (maxl > 1024) return kcna_fail(c, KCNA_E_ARG, "max(L, K, search_L, search_K) must be <= 1024");
+    if (P.L == 0) return kcna_fail(c, KCNA_E_ARG, "L must be at least 1");
     st->maxl = maxl;
     KCNA_TRY(kcna_nnd_alloc(c, &P, maxl));
     KCNA_TRY(kcna_controls_setup(c, &P, maxl));
