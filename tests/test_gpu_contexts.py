@@ -40,7 +40,20 @@ def _rank_prune(ix, rng, d, size):
     return run
 
 
-@pytest.mark.parametrize("make,forms", [(_knn, [(128, 10), (96, 10), (200, 10)]), (_search, [(128, 1500), (1024, 1000), (32, 40)]),
+def _build(ix, rng, d, size):
+    ix.upload(rng.standard_normal((2500, d)).astype(np.float32))
+    p = kcna.params(K=size, L=size, S=10, R=100, iterations=3, search_L=20, search_K=size, nsg_R=20, screen=1, tau=0.1)
+
+    def run():  # no two builds of these are alike
+        ix.build("taumng" if d >= 256 else "nsg", p)
+        ids, dist, cnt = ix.pools()
+        assert (cnt > 0).all() and (ids[:, 0] < 2500).all() and (np.diff(dist[:, :10]) >= 0).all()
+        return ()
+
+    return run
+
+
+@pytest.mark.parametrize("make,forms", [(_build, [(24, 60), (300, 40), (64, 600), (130, 200)]), (_knn, [(128, 10), (96, 10), (200, 10)]), (_search, [(128, 1500), (1024, 1000), (32, 40)]),
                                         (_rank_prune, [(8, 1000), (8, 64), (8, 300)])])
 def test_calls_of_several_threads(make, forms):
     errors = []
